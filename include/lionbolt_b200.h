@@ -203,10 +203,11 @@ int lb_synchronize(lb_handle* h);
  * synchronisation reports, LB_ERR_TIMEOUT (message in lb_last_error), and clears the flag, so the
  * handle stays usable. */
 int lb_probe_pipeline_timeout(lb_handle* h, long long polls);
-/* Sweep launch shape picked by the autotuner: cfg[0] schedule (0 levels, 1 dataflow, 2 levels with
+/* Sweep launch shape (the tile schedule on meshes of hexes split along their main diagonal, elsewhere the
+ * autotuner's pick): cfg[0] schedule (0 levels, 1 dataflow, 2 levels with
  * next-level prefetch, 3 element flags, 4 grouped directions, 5 blocks of 6 elements swept as
- * units, 6 the same with per-type element tables), cfg[1] threads per CTA, cfg[2] directions per CTA
- * (minimum CTAs per SM for 5 and 6), cfg[3] updates in flight per thread.  Returns
+ * units, 6 the same with per-type element tables, 7 the same blocks moved through shared-memory tiles),
+ * cfg[1] threads per CTA, cfg[2] directions per CTA (minimum CTAs per SM for 5, 6 and 7), cfg[3] updates in flight per thread.  Returns
  * LB_ERR_STATE while candidates are still being timed (the first sweeps of a handle). */
 int lb_get_sweep_config(lb_handle* h, int* cfg);
 
@@ -231,7 +232,7 @@ int lb_givens(double x, double y, double* c, double* s, double* r);
  *     (optional) = block members (-1: empty), *max_records = largest record count of a direction.
  *   lb_get_cluster_schedule: rec[rec_base[NI]][4] records in execution order (x = block index; y, z, w =
  *     two 16-bit slots each in execution order: member position in the block (3 b, 7 = empty),
- *     upstream-face mask << 3, outflow-face mask << 7), starts[NI][max_records + 1] block-level
+ *     upstream-face mask << 3, outflow-face mask << 7, tile type << 11), starts[NI][max_records + 1] block-level
  *     starts (relative to rec_base[i]), nlevels[NI].
  * Diagnostics for tests; no counterpart in the reference. */
 int lb_cluster_info(lb_handle* h, int* nblocks, int* max_levels);
@@ -307,8 +308,8 @@ int lb_batch_add_problem(lb_batch* b, int NE, int NN, const double* rg, const in
 int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int* iters);
 /* flux[G][NENK], dose[NENK] of problem id (either may be NULL). */
 int lb_batch_get_results(lb_batch* b, int id, double* flux, double* dose);
-/* Problem count, largest group count, device time of the last solve (ms), sweep threads picked by
- * the tuner, graph replays and batched sweep launches so far.  Any pointer may be NULL. */
+/* Problem count, largest group count, device time of the last solve (ms), threads per CTA of the batched
+ * sweep, graph replays and batched sweep launches so far.  Any pointer may be NULL. */
 int lb_batch_info(lb_batch* b, int* nproblems, int* max_groups, double* last_ms, int* sweep_threads,
                   long long* graph_launches, long long* sweep_launches);
 

@@ -204,12 +204,15 @@ class Handle:
         if st != LB_OK:
             return None
         names = ("levels", "dataflow", "levels+prefetch", "element flags", "grouped directions", "cluster levels",
-                 "cluster levels+type tables")
+                 "cluster levels+type tables", "block tiles")
         kind = int(cfg[0])
         d = dict(schedule=names[kind] if 0 <= kind < len(names) else str(kind), threads=int(cfg[1]),
                  dirs_per_cta=int(cfg[2]), ilp=int(cfg[3]))
-        if kind in (5, 6):
+        if kind >= 5:
             d["min_ctas_per_sm"] = d.pop("dirs_per_cta")
+            if kind == 7:
+                d["tile_mode"] = d.pop("ilp")
+                return d
             if d["ilp"] >= 2:
                 d["schedule"] += "+element prefetch"
             if d["ilp"] == 3:

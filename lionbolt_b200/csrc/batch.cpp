@@ -12,7 +12,7 @@
 //     captured once per group step as a CUDA graph and replayed for every Arnoldi step, on fixed
 //     per-problem ping-pong buffers;
 //   * the Gram-Schmidt dots, axpys and norms are segmented kernels: one launch for all problems.
-// The sweep launch shape (threads per CTA) is chosen by timing the candidates on the batch.
+// The threads that take a direction are chosen from the sizes of its groups (choose_team).
 #include "lb_internal.h"
 #include "gmres_host.h"
 #include <algorithm>
@@ -39,8 +39,7 @@ struct lb_batch {
     int work_cap = 0;
     int nwork = 0;
     int* d_counter = nullptr;
-    int sweep_threads = 0;                     // chosen by timing (0: not yet)
-    float tune_ms[2] = {0.f, 0.f};
+    int sweep_team = 0;                        // threads of a CTA that take a direction (choose_team)
     cudaGraphExec_t gx[3] = {nullptr, nullptr, nullptr};   // residual, a->b, b->a
     cudaEvent_t ev[2] = {nullptr, nullptr};
     double last_ms = 0.0;
@@ -106,6 +105,11 @@ int build_work(lb_batch* b, const std::vector<int>& ids, int threads) {
                     x.gtab = h->d_gtab;
                     x.tmat = h->d_tmat;
                 }
+                if (h->tiles_ok) {
+                    x.nxtype = h->nxtype;
+                    x.xtab = h->d_xtab;
+                    x.xmat = h->d_xmat;
+                }
                 const int* st = &h->cl_start_h[h->cl_base_h[i]];
                 for (int L = 0; L < x.ncl; ++L) c += 1.0 + kClusterSize * std::ceil((double)(st[L + 1] - st[L]) / threads);
             } else {
@@ -141,40 +145,33 @@ int build_work(lb_batch* b, const std::vector<int>& ids, int threads) {
 
 int sweep_all(lb_batch* b) {
     ++b->sweep_launches;
-    int rc = launch_sweep_batch(bstream(b), b->d_work, b->nwork, b->d_counter, b->d_active, b->sweep_threads,
+    int rc = launch_sweep_batch(bstream(b), b->d_work, b->nwork, b->d_counter, b->d_active, b->sweep_team,
                                 b->aux->sm_count);
     return rc ? bfail(b, rc, "batched sweep launch failed") : LB_OK;
 }
 
-// Times the sweep launch shapes on the current work list (contents of psi are overwritten later).
-int tune_sweep(lb_batch* b, const std::vector<int>& ids) {
-    const int cand[2] = {1024, 512};
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    for (int c = 0; c < 2; ++c) {
-        b->sweep_threads = cand[c];
-        int rc = build_work(b, ids, cand[c]);
-        if (!rc) rc = sweep_all(b);   // first launch loads the module
-        cudaEventRecord(e0, bstream(b));
-        if (!rc) rc = sweep_all(b);
-        cudaEventRecord(e1, bstream(b));
-        cudaError_t e = cudaEventSynchronize(e1);
-        if (rc || e != cudaSuccess) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            return rc ? rc : bcuda(b, e, "sweep tuning");
+// Threads that take a direction in the batched sweep of the problems `ids`: small teams where the groups are
+// small (a wider team's threads would idle in most passes), as long as every SM still gets a CTA of 512 / team
+// teams.  Measured: 8 problems of 8 to 20 hexes per axis (about 70 units a group) 0.655, 0.418 and 0.358 ms per
+// sweep with teams of 512, 256 and 128; a batch of 64 problems of 8 to 32 hexes (about 140 units a group in its
+// first group steps) 779, 703 and 715 ms per solve.
+int choose_team(lb_batch* b, const std::vector<int>& ids) {
+    double units = 0.0, groups = 0.0, dirs = 0.0;
+    for (int p : ids) {
+        const lb_handle* h = b->probs[p];
+        dirs += h->NI;
+        if (h->nclusters > 0) {
+            units += (double)h->crec_base_h[h->NI];
+            groups += (double)h->cluster_levels_total;
+        } else {
+            units += (double)h->NE * h->NI;
+            groups += (double)h->total_levels;
         }
-        cudaEventElapsedTime(&b->tune_ms[c], e0, e1);
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    b->sweep_threads = b->tune_ms[1] < b->tune_ms[0] ? 512 : 1024;
-    if (const char* v = std::getenv("LB_SWEEP_VERBOSE"))
-        if (*v == '1')
-            std::fprintf(stderr, "batched sweep: 1024 threads %.3f ms, 512 threads %.3f ms -> %d\n", b->tune_ms[0],
-                         b->tune_ms[1], b->sweep_threads);
-    return build_work(b, ids, b->sweep_threads);
+    const double mean = units / std::max(groups, 1.0);
+    for (int team : {128, 256})
+        if (mean <= team && dirs >= (double)b->aux->sm_count * kBatchThreads / team) return team;
+    return kBatchThreads;
 }
 
 // y_p = A x_p for every problem in ids (direct launches).  mode 0: y = x - D T^-1 M Sigma x
@@ -638,13 +635,8 @@ int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int*
             if (b->probs[p]->G > g) ids.push_back(p);
         for (int p : ids)
             if ((rc = mg_group_sources(b->probs[p], g))) return prop_error(b, b->probs[p], rc, p);
-        if (b->sweep_threads == 0) {
-            std::fill(b->h_active, b->h_active + P, 1);
-            cudaMemcpyAsync(b->d_active, b->h_active, sizeof(int) * P, cudaMemcpyHostToDevice, s);
-            if ((rc = tune_sweep(b, ids))) return rc;
-        } else if ((rc = build_work(b, ids, b->sweep_threads))) {
-            return rc;
-        }
+        b->sweep_team = choose_team(b, ids);
+        if ((rc = build_work(b, ids, b->sweep_team))) return rc;
         // b = D T^{-1} M src for every problem of the step, then x = b
         cudaStreamSynchronize(s);
         std::fill(b->h_active, b->h_active + P, 0);
@@ -700,7 +692,7 @@ int lb_batch_info(lb_batch* b, int* nproblems, int* max_groups, double* last_ms,
     if (nproblems) *nproblems = (int)b->probs.size();
     if (max_groups) *max_groups = Gmax;
     if (last_ms) *last_ms = b->last_ms;
-    if (sweep_threads) *sweep_threads = b->sweep_threads;
+    if (sweep_threads) *sweep_threads = kBatchThreads;
     if (graph_launches) *graph_launches = b->graph_launches;
     if (sweep_launches) *sweep_launches = b->sweep_launches;
     return LB_OK;

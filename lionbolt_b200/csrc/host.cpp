@@ -125,7 +125,7 @@ static int dev_upload(Handle* h, T** p, const T* src, size_t count, const char* 
 
 static void free_all(Handle* h) {
     void* ptrs[] = {h->d_geom, h->d_rec, h->d_crec, h->d_crec_base, h->d_blk_elem, h->d_beam_plane, h->d_beam_xyz,
-                    h->d_beam_node, h->d_beam_nbr, h->d_cl_start, h->d_cl_base, h->d_ncl, h->d_gtab, h->d_tmat, h->d_mat, h->d_items, h->d_groups, h->d_pitems, h->d_pbase, h->d_chunks, h->d_lvl_start, h->d_lvl_base, h->d_nlev, h->d_done, h->d_status, h->d_tc_err, h->d_dirs, h->d_sigt,
+                    h->d_beam_node, h->d_beam_nbr, h->d_cl_start, h->d_cl_base, h->d_ncl, h->d_gtab, h->d_tmat, h->d_xtab, h->d_xmat, h->d_mat, h->d_items, h->d_groups, h->d_pitems, h->d_pbase, h->d_chunks, h->d_lvl_start, h->d_lvl_base, h->d_nlev, h->d_done, h->d_status, h->d_tc_err, h->d_dirs, h->d_sigt,
                     h->d_psi, h->d_qext, h->d_Ym2d, h->d_Yd2m, h->d_sigl, h->d_lofj, h->d_V, h->d_Z, h->d_x,
                     h->d_b, h->d_t, h->d_red, h->d_unc, h->d_phi_all, h->d_src, h->d_dose, h->d_flux,
                     h->d_sigl_mg, h->d_yb, h->d_dd};
@@ -305,6 +305,37 @@ int lb_sn_quadrature(int Ng, int Nc, double* k, double* w) {
     return LB_OK;
 }
 
+// Neighbour words of a tile type for the tile sweep, from the type's place in its block and, per face, the
+// neighbour's id offset * 64 + its node indices (kAnyWord: no neighbour).  The tile sweep's element update is
+// written for hexes split into 6 tets along their main diagonal, where every tet has
+//   faces 1 and 2 inside the hex, with node indices (0, 2, 3) and (0, 1, 3) in the neighbour, and
+//   faces 0 and 3 on the hex's surface, with (1, 2, 3) and (0, 1, 2), or (2, 3, 1) and (2, 0, 1) in the
+//   tets whose two middle nodes are swapped for a positive orientation.
+// False when the type is not of that form.  Words: x, z = byte offset, from the block's first element, of the
+// elements across faces 0 and 3; y = (byte offset in the block row of the elements across faces 1 and 2,
+// swapped) << (8, 16, 24).
+static constexpr int kAnyWord = INT32_MIN;
+static bool tile_word(int pos, const int* w, int4* out) {
+    constexpr int kIn[2] = {0 | 2 << 2 | 3 << 4, 0 | 1 << 2 | 3 << 4};
+    constexpr int kOut[2][2] = {{1 | 2 << 2 | 3 << 4, 0 | 1 << 2 | 2 << 4}, {2 | 3 << 2 | 1 << 4, 2 | 0 << 2 | 1 << 4}};
+    int in[2], far[2] = {0, 0}, swapped = -1;
+    for (int k = 0; k < 2; ++k) {
+        const int wi = w[1 + k];
+        if (wi == kAnyWord || (wi & 63) != kIn[k]) return false;
+        in[k] = pos + (wi >> 6);
+        if (in[k] < 0 || in[k] >= kClusterSize) return false;
+        const int wo = w[3 * k];
+        if (wo == kAnyWord) continue;
+        const int s = (wo & 63) == kOut[0][k] ? 0 : (wo & 63) == kOut[1][k] ? 1 : -1;
+        const int np = pos + (wo >> 6);
+        if (s < 0 || (swapped >= 0 && s != swapped) || (np >= 0 && np < kClusterSize)) return false;
+        swapped = s;
+        far[k] = 16 * np;
+    }
+    *out = make_int4(far[0], in[0] * 16 << 8 | in[1] * 16 << 16 | (swapped == 1 ? 1 : 0) << 24, far[1], 0);
+    return true;
+}
+
 int lb_set_mesh(lb_handle* h, int NE, int NN, const double* rg, const int* node, const int* neighbors, const int* mat,
                 int Nm) {
     if (!h) return LB_ERR_ARG;
@@ -449,6 +480,58 @@ int lb_set_mesh(lb_handle* h, int NE, int NN, const double* rg, const int* node,
             if ((rc = dev_upload(h, &h->d_tmat, tmat.data(), tmat.size(), "upload type materials"))) return rc;
             h->ngeom = (int)types.size();
         }
+        h->xtype.clear();
+        h->nxtype = 0;
+        if (ok) {
+            // tile types: elements of one type and one place in their block of kClusterSize ids whose existing
+            // neighbours sit at equal id offsets with equal node indices; a boundary face takes whatever the
+            // type's other elements have there
+            struct Tile {
+                int geom, mat, pos, w[4];
+            };
+            std::vector<Tile> tiles;
+            std::vector<uint8_t> xt(NE);
+            bool fits = NE % kClusterSize == 0;
+            for (int e = 0; e < NE && fits; ++e) {
+                int w[4];
+                for (int f = 0; f < 4; ++f) {
+                    const int ep = h->nbr[(size_t)e * 4 + f];
+                    w[f] = ep < 0 ? kAnyWord : (ep - e) * 64 + (int)((h->nbrpack[(size_t)e * 4 + f] >> 24) & 63u);
+                }
+                const int pos = e % kClusterSize;
+                size_t t = 0;
+                for (; t < tiles.size(); ++t) {
+                    bool same = tiles[t].geom == idx[e] && tiles[t].pos == pos;
+                    for (int f = 0; f < 4 && same; ++f)
+                        same = w[f] == kAnyWord || tiles[t].w[f] == kAnyWord || w[f] == tiles[t].w[f];
+                    if (same) break;
+                }
+                if (t == tiles.size()) {
+                    if ((int)t >= kMaxTileTypes) { fits = false; break; }
+                    tiles.push_back(Tile{idx[e], h->mat[e], pos, {kAnyWord, kAnyWord, kAnyWord, kAnyWord}});
+                }
+                for (int f = 0; f < 4; ++f)
+                    if (w[f] != kAnyWord) tiles[t].w[f] = w[f];
+                xt[e] = (uint8_t)t;
+            }
+            std::vector<float4> xtab;
+            std::vector<int> xmat;
+            for (const Tile& t : tiles) {
+                int4 w;
+                fits = fits && tile_word(t.pos, t.w, &w);
+                for (int d = 0; d < 3; ++d) xtab.push_back(tab[(size_t)t.geom * 3 + d]);
+                float4 v;
+                std::memcpy(&v, &w, sizeof v);
+                xtab.push_back(v);
+                xmat.push_back(t.mat);
+            }
+            if (fits) {
+                if ((rc = dev_upload(h, &h->d_xtab, xtab.data(), xtab.size(), "upload tile types"))) return rc;
+                if ((rc = dev_upload(h, &h->d_xmat, xmat.data(), xmat.size(), "upload tile materials"))) return rc;
+                h->xtype.swap(xt);
+                h->nxtype = (int)tiles.size();
+            }
+        }
     }
     rc = dev_upload(h, &h->d_mat, h->mat.data(), h->mat.size(), "upload materials");
     if (rc) return rc;
@@ -466,7 +549,8 @@ int lb_set_mesh(lb_handle* h, int NE, int NN, const double* rg, const int* node,
 // has an upstream neighbour in A) must be acyclic; its longest-path levels order the blocks, and
 // blocks with the same element order and face masks are adjacent inside a level.  Record of a block:
 //   x: block index;  y, z, w: two 16-bit slots each, in execution order: element offset in the
-//   block (3 b, 7 = empty) | upstream-face mask << 3 | outflow-face mask << 7.
+//   block (3 b, 7 = empty) | upstream-face mask << 3 | outflow-face mask << 7 | tile type << 11 (0 without
+//   tile types).
 // Built on device handles; when some direction's block graph has a cycle no cluster schedule is
 // kept and the sweep uses the element schedules.
 // Blocks of the cluster schedule.  Box meshes number the 6 tets of a hex consecutively, so blocks of
@@ -584,6 +668,7 @@ static int cluster_group_cap() {
 static int build_cluster_schedule(Handle* h) {
     constexpr int K = kClusterSize;
     h->nclusters = 0;
+    h->tiles_ok = false;
     h->max_cluster_levels = 0;
     h->max_cluster_records = 0;
     h->cl_start_h.clear();
@@ -689,6 +774,7 @@ static int build_cluster_schedule(Handle* h) {
             for (int es = 0; es < NE; ++es) {
                 const int e = it[es] & 0xFFFFFF;
                 fld[e] = (uint16_t)(blk_pos[e] | (((it[es] >> 24) & 0xF) << 3) | (((it[es] >> 28) & 0xF) << 7));
+                if (h->nxtype > 0) fld[e] |= (uint16_t)(h->xtype[e] << 11);
             }
             // element edges y -> x (y upstream of x), as downstream lists
             std::fill(dstart.begin(), dstart.end(), 0);
@@ -836,6 +922,8 @@ static int build_cluster_schedule(Handle* h) {
     h->nclusters = NC;
     h->max_cluster_levels = maxl;
     h->max_cluster_records = maxr;
+    // the tile sweep moves whole blocks: every unit must be one (no block split on a cycle, no short last block)
+    h->tiles_ok = h->nxtype > 0 && blk_elem.empty() && NE % K == 0 && base[NI] == (long long)NC * NI;
     h->cluster_levels_total = 0;
     for (int i = 0; i < NI; ++i) h->cluster_levels_total += ncl[i];
     h->cl_start_h = cl_start;

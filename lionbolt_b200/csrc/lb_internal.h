@@ -13,6 +13,9 @@ namespace lb {
 // elements per block of the cluster sweep schedule (a hex of a box mesh split into 6 tets)
 constexpr int kClusterSize = 6;
 
+// tile types a slot of a block record can name (5 bits)
+constexpr int kMaxTileTypes = 32;
+
 // Packed schedule item (one per element-direction, in sweep order):
 //   bits 0-23 element id, bits 24-27 upstream-face mask, bits 28-31 outflow-face mask.
 constexpr int kElemBits = 24;
@@ -96,6 +99,15 @@ struct Handle {
     float4* d_gtab = nullptr;      // [ngeom][3] (snx, sny, snz)
     int* d_tmat = nullptr;         // [ngeom] material of each type
     int ngeom = 0;                 // number of types; 0: no table (use d_geom)
+    // tile types of the tile sweep (sweep_tile_kernel): elements of one type that also share their place in
+    // the block and the id offset of every neighbour (boundary faces match any offset: they are never
+    // upstream), so that an element needs no record of its own.  Only for meshes of hexes split along their
+    // main diagonal (tile_word in host.cpp); a box has one per tet of a hex and material.
+    std::vector<uint8_t> xtype;    // [NE] tile type of each element (empty: none)
+    float4* d_xtab = nullptr;      // [nxtype][4] face vectors and the neighbour words
+    int* d_xmat = nullptr;         // [nxtype] material of each tile type
+    int nxtype = 0;
+    bool tiles_ok = false;         // every direction's units are whole blocks of kClusterSize consecutive ids
     // cluster schedule: blocks of up to kClusterSize face-connected elements swept as units (0 blocks:
     // none).  Blocks are kClusterSize consecutive ids when those are face-connected (box meshes: one hex
     // each); otherwise they are grown greedily from face neighbours and listed in blk_elem.  A direction
@@ -286,12 +298,16 @@ struct BatchWork {
     const float4* gtab;     // [ngeom][3] face vectors of the types
     const int* tmat;        // [ngeom] material of the types
     int ncl;
-    int pad[3];
+    int nxtype;             // tile types of the problem when the tile sweep takes its directions, else 0
+    int pad[2];
+    const float4* xtab;     // [nxtype][4] the problem's tile types
+    const int* xmat;        // [nxtype] material of the tile types
 };
 // Sweeps every work item whose problem has active[problem] != 0, CTAs claiming items in order from
-// *counter (reset before the launch).  threads: 1024 or 512.
-int launch_sweep_batch(cudaStream_t s, const BatchWork* work, int nwork, int* counter, const int* active,
-                       int threads, int sm_count);
+// *counter (reset before the launch).  team: threads of a CTA that take an item (512, 256 or 128).
+constexpr int kBatchThreads = 512;   // threads per CTA, two CTAs per SM
+int launch_sweep_batch(cudaStream_t s, const BatchWork* work, int nwork, int* counter, const int* active, int team,
+                       int sm_count);
 
 // Segmented (per-problem) FP64 vector operations of a batch: one launch for all problems.
 struct SegVec {

@@ -19,15 +19,17 @@
 //  * cluster levels: blocks of 6 consecutive elements (a hex of a box mesh split into 6 tets) are
 //    swept as units over each direction's block-level graph, one thread per block, a CTA barrier
 //    between block levels; optionally with the element matrices of every element type computed once
-//    per direction.  The fastest at the 768k-tet configuration.
+//    per direction.
+//  * block tiles: the cluster schedule's blocks moved through shared memory by their warp, without element
+//    records; for meshes of hexes split along their main diagonal, and the fastest there.
 //  * levels: one CTA owns whole directions and walks their element wavefront levels in order with a
 //    CTA barrier between levels; upstream values written by the same SM are re-read through its L1.
 //  * levels with next-level prefetch, element flags in shared memory, grouped same-schedule
 //    directions, and dataflow (warps claim 32-element chunks from a global counter and wait, with a
 //    bounded spin, on the completion counter of the previous level): candidates for other meshes.
-// Launch shape (schedule, threads per CTA, directions or CTAs per SM, updates in flight per thread)
-// is picked by timing the first sweeps of a handle (the three fastest twice); every candidate
-// computes bit-identical results.
+// Box-like meshes (hexes split along their main diagonal) take the tile schedule; elsewhere the launch shape
+// (schedule, threads per CTA, directions or CTAs per SM, updates in flight per thread) is picked by timing the
+// first sweeps of a handle (the three fastest twice).  Every candidate computes bit-identical results.
 #include "lb_internal.h"
 #include <algorithm>
 #include <cstdio>
@@ -76,6 +78,9 @@ struct SweepArgs {
     const int* __restrict__ cl_base;
     const int* __restrict__ ncl;
     int nclusters;                    // 0: no cluster schedule
+    const float4* __restrict__ xtab;  // [nxtype][4] tile types: face vectors, neighbour words
+    const int* __restrict__ xmat;     // [nxtype] material of the tile types
+    int nxtype;
 };
 
 __device__ __forceinline__ float pick(const float4& v, int idx) {
@@ -185,41 +190,25 @@ __device__ __forceinline__ void assemble(const SweepArgs& a, const float* base, 
     assemble_g<kCG, kHaveQ>(base, dir, item, G, s_sigt, u, qpre);
 }
 
-// kPrev >= 1: the solution of element prev_e (the thread's previous update) is passed in registers and used
-// instead of a load when it is an upstream neighbour; kPrev = 2 also the one before it (prev2_e).
-template <bool kCG, bool kHaveQ, int kPrev>
-__device__ __forceinline__ void assemble_g(const float* base, float4 dir, int item, const Geom& G, const float* s_sigt,
-                                           Update& u, float4 qpre, int prev_e, float4 prev_v, int prev2_e,
-                                           float4 prev2_v) {
+// The element system from the source q, the face masks, the face vectors and sigma; up(f, u0, u1, u2) gives
+// the upstream neighbour's values at the nodes of inflow face f.
+template <class Up>
+__device__ __forceinline__ void assemble_sys(float4 q, float4 dir, int upm, int outm, float4 gx, float4 gy, float4 gz,
+                                             float sig, Up&& up, Update& u) {
     // gmsh face -> local nodes; the vertex opposite face f is 3 - f
     constexpr int F[4][3] = {{0, 1, 2}, {0, 1, 3}, {0, 2, 3}, {1, 2, 3}};
-    const int e = item & 0xFFFFFF;
-    const int upm = (item >> 24) & 0xF;
-    const int outm = (item >> 28) & 0xF;
-    const float4 gx = G.gx, gy = G.gy, gz = G.gz;
-    const int4 gn = G.gn;
-    const float4 q = kHaveQ ? qpre : ld4<kCG>(base + 4 * (size_t)e);
     float c[4];
     c[0] = fmaf(dir.x, gx.x, fmaf(dir.y, gy.x, dir.z * gz.x));
     c[1] = fmaf(dir.x, gx.y, fmaf(dir.y, gy.y, dir.z * gz.y));
     c[2] = fmaf(dir.x, gx.z, fmaf(dir.y, gy.z, dir.z * gz.z));
     c[3] = fmaf(dir.x, gx.w, fmaf(dir.y, gy.w, dir.z * gz.w));
-    const unsigned nw[4] = {(unsigned)gn.x, (unsigned)gn.y, (unsigned)gn.z, (unsigned)gn.w};
-    const int matid = (int)((nw[0] >> 30) | ((nw[1] >> 30) << 2) | ((nw[2] >> 30) << 4) | ((nw[3] >> 30) << 6));
-    const float sig = s_sigt[matid];
     u.r[0] = q.x; u.r[1] = q.y; u.r[2] = q.z; u.r[3] = q.w;
     // upstream coupling: r -= (k.n_f) IIM_f psi_up over the inflow faces
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
         if ((upm >> f) & 1) {
-            const unsigned wd = nw[f];
-            const int ep = (int)(wd & 0xFFFFFFu);
-            const float4 u4 = (kPrev >= 1 && ep == prev_e)   ? prev_v
-                              : (kPrev >= 2 && ep == prev2_e) ? prev2_v
-                                                              : ld4<kCG>(base + 4 * (size_t)ep);
-            const float u0 = pick(u4, (wd >> 24) & 3);
-            const float u1 = pick(u4, (wd >> 26) & 3);
-            const float u2 = pick(u4, (wd >> 28) & 3);
+            float u0, u1, u2;
+            up(f, u0, u1, u2);
             const float U = u0 + u1 + u2;
             const float cf = c[f];
             const float t3 = U * kThird;
@@ -239,6 +228,30 @@ __device__ __forceinline__ void assemble_g(const float* base, float4 dir, int it
         u.a[k] = kFiveThirds * (c[3 - k] - co[3 - k]);
         u.b[k] = (Ct - co[3 - k]) * kThird;
     }
+}
+
+// kPrev >= 1: the solution of element prev_e (the thread's previous update) is passed in registers and used
+// instead of a load when it is an upstream neighbour; kPrev = 2 also the one before it (prev2_e).
+template <bool kCG, bool kHaveQ, int kPrev>
+__device__ __forceinline__ void assemble_g(const float* base, float4 dir, int item, const Geom& G, const float* s_sigt,
+                                           Update& u, float4 qpre, int prev_e, float4 prev_v, int prev2_e,
+                                           float4 prev2_v) {
+    const int e = item & 0xFFFFFF;
+    const int4 gn = G.gn;
+    const float4 q = kHaveQ ? qpre : ld4<kCG>(base + 4 * (size_t)e);
+    const unsigned nw[4] = {(unsigned)gn.x, (unsigned)gn.y, (unsigned)gn.z, (unsigned)gn.w};
+    const int matid = (int)((nw[0] >> 30) | ((nw[1] >> 30) << 2) | ((nw[2] >> 30) << 4) | ((nw[3] >> 30) << 6));
+    assemble_sys(q, dir, (item >> 24) & 0xF, (item >> 28) & 0xF, G.gx, G.gy, G.gz, s_sigt[matid],
+                 [&](int f, float& u0, float& u1, float& u2) {
+                     const unsigned wd = nw[f];
+                     const int ep = (int)(wd & 0xFFFFFFu);
+                     const float4 u4 = (kPrev >= 1 && ep == prev_e)   ? prev_v
+                                       : (kPrev >= 2 && ep == prev2_e) ? prev2_v
+                                                                       : ld4<kCG>(base + 4 * (size_t)ep);
+                     u0 = pick(u4, (wd >> 24) & 3);
+                     u1 = pick(u4, (wd >> 26) & 3);
+                     u2 = pick(u4, (wd >> 28) & 3);
+                 }, u);
 }
 
 // Solve (d I + a 1^T + 1 b^T) x = r through the 2x2 capacitance system
@@ -281,13 +294,16 @@ struct ElemTab {
     float4 a;    // a_k
     float4 b;    // b_k
     float4 s0;   // e00, e11, b.a, 1 / det
-    float4 s1;   // 1 / d, outflow mask (int bits), -, -
+    float4 s1;   // 1 / d, outflow mask (int bits), -, - (tile types: the neighbour words)
 };
 
+// kTile: the types are tile types, [4] float4 each, whose neighbour words (tile_word in host.cpp) go into s1.
+template <bool kTile = false>
 __device__ __forceinline__ void build_tab(const float4* s_gtab, const float* s_sigt, int ngeom, float4 dir,
-                                          ElemTab* s_tab) {
-    for (int t = threadIdx.x; t < ngeom; t += blockDim.x) {
-        const float4 gx = s_gtab[3 * t + 0], gy = s_gtab[3 * t + 1], gz = s_gtab[3 * t + 2];
+                                          ElemTab* s_tab, int t0, int tstep) {
+    for (int t = t0; t < ngeom; t += tstep) {
+        constexpr int S = kTile ? 4 : 3;
+        const float4 gx = s_gtab[S * t + 0], gy = s_gtab[S * t + 1], gz = s_gtab[S * t + 2];
         float c[4];
         c[0] = fmaf(dir.x, gx.x, fmaf(dir.y, gy.x, dir.z * gz.x));
         c[1] = fmaf(dir.x, gx.y, fmaf(dir.y, gy.y, dir.z * gz.y));
@@ -318,6 +334,10 @@ __device__ __forceinline__ void build_tab(const float4* s_gtab, const float* s_s
         T.b = make_float4(u.b[0], u.b[1], u.b[2], u.b[3]);
         T.s0 = make_float4(e00, e11, ba, __fdividef(1.0f, det));
         T.s1 = make_float4(__fdividef(1.0f, u.d), __int_as_float(outm), 0.f, 0.f);
+        if (kTile) {
+            const float4 w = s_gtab[S * t + 3];
+            T.s1 = make_float4(T.s1.x, __int_as_float(outm | __float_as_int(w.y)), w.x, w.z);
+        }
         s_tab[t] = T;
     }
 }
@@ -557,7 +577,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_cluster_kernel(SweepArgs a) {
         const float4 dir = __ldg(&a.dirs[i]);
         if (TAB) {
             __syncthreads();   // the previous direction's updates have read the table
-            build_tab(s_gtab, s_sigt, a.ngeom, dir, s_tab);
+            build_tab(s_gtab, s_sigt, a.ngeom, dir, s_tab, threadIdx.x, blockDim.x);
             __syncthreads();
         }
         const int4* rec = a.crec + __ldg(&a.crec_base[i]);
@@ -648,6 +668,201 @@ __global__ void __launch_bounds__(NT, MINB) sweep_cluster_kernel(SweepArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Tile schedule: the cluster schedule's blocks and groups, with a block's data moved by its warp.
+//
+// What bounds the cluster kernel is the L1 data pipe: a lane's 16-byte access of its own block touches a line
+// of its own, so every element record, source and solution access of a warp costs 32 tag lookups (about 115 of
+// the 140 cycles per warp and element step at 768,000 tets, 288 directions).  Here
+//  * the 96 contiguous bytes of a block's sources enter shared memory by six 16-byte cp.async per lane whose
+//    lanes walk the warp's blocks in address order (about 8 lines per instruction), and the solutions leave
+//    the same way; the row pitch of 7 lines of 16 bytes keeps every shared access free of bank conflicts;
+//  * elements have no record: a slot names its tile type, whose per-direction table (the same for a whole warp
+//    as a rule) is read from shared memory by broadcast, the neighbour offsets with it;
+//  * upstream values from the block itself are read from its row;
+//  * the update is written for hexes split along their main diagonal (tile_word in host.cpp), where the node
+//    indices of a face are the same in every tet up to one swap: no selection by index.
+// The next pass's record and sources are requested before the barrier that ends a group: no other thread
+// writes them.  Element arithmetic as in the other schedules (bit-identical results).
+// Measured per sweep, cluster kernel -> this one: 768,000 tets x 288 directions 4.15 -> 3.03 ms, 96,000 x 288
+// 0.647 -> 0.424, 57,456 x 288 0.489 -> 0.301, 24,480 x 168 0.246 -> 0.174, 6,000 x 80 0.105 -> 0.089 (144 instead of 270
+// warp instructions per warp and element step).  What is left is the L1 pipe (61 % busy) and the gathers of
+// upstream values from other blocks (27 % of the time); neither the sources' latency nor the barriers show.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTileRow = kClusterSize + 1;   // 16-byte lines per block row
+
+__device__ __forceinline__ void cp_async16(const void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// One element of a block: row = the block's tile row, bb = its 96 bytes in global memory, f = slot.
+__device__ __forceinline__ void tile_update(char* row, const char* bb, unsigned f, float4 dir, const float4* s_x,
+                                            const float* s_sig, const ElemTab* s_tab) {
+    const int pos = (int)(f & 7u), t = (int)(f >> 11);
+    const ElemTab* T = s_tab + t;
+    const float4 s1 = T->s1;
+    const int word = __float_as_int(s1.y);
+    float4* mine = reinterpret_cast<float4*>(row + 16 * pos);
+    const float4 q = *mine;
+    float r[4] = {q.x, q.y, q.z, q.w};
+    const float4 c = T->c;
+    const bool swapped = (word >> 24) != 0;
+    // r -= (k.n_f) IIM_f psi_up over the inflow faces, faces in order (as assemble_sys)
+    if (f & 0x08u) {   // face 0: nodes 0 1 2, the vertex opposite is 3
+        const float4 v = *reinterpret_cast<const float4*>(bb + __float_as_int(s1.z));
+        const float u0 = swapped ? v.z : v.y, u1 = swapped ? v.w : v.z, u2 = swapped ? v.y : v.w;
+        const float U = u0 + u1 + u2, t3 = U * kThird;
+        r[0] = fmaf(-c.x, fmaf(kFiveThirds, u0, t3), r[0]);
+        r[1] = fmaf(-c.x, fmaf(kFiveThirds, u1, t3), r[1]);
+        r[2] = fmaf(-c.x, fmaf(kFiveThirds, u2, t3), r[2]);
+        r[3] = fmaf(c.x * kFourThirds, U, r[3]);
+    }
+    if (f & 0x10u) {   // face 1: nodes 0 1 3
+        const float4 v = *reinterpret_cast<const float4*>(row + ((word >> 8) & 0xFF));
+        const float U = v.x + v.z + v.w, t3 = U * kThird;
+        r[0] = fmaf(-c.y, fmaf(kFiveThirds, v.x, t3), r[0]);
+        r[1] = fmaf(-c.y, fmaf(kFiveThirds, v.z, t3), r[1]);
+        r[3] = fmaf(-c.y, fmaf(kFiveThirds, v.w, t3), r[3]);
+        r[2] = fmaf(c.y * kFourThirds, U, r[2]);
+    }
+    if (f & 0x20u) {   // face 2: nodes 0 2 3
+        const float4 v = *reinterpret_cast<const float4*>(row + ((word >> 16) & 0xFF));
+        const float U = v.x + v.y + v.w, t3 = U * kThird;
+        r[0] = fmaf(-c.z, fmaf(kFiveThirds, v.x, t3), r[0]);
+        r[2] = fmaf(-c.z, fmaf(kFiveThirds, v.y, t3), r[2]);
+        r[3] = fmaf(-c.z, fmaf(kFiveThirds, v.w, t3), r[3]);
+        r[1] = fmaf(c.z * kFourThirds, U, r[1]);
+    }
+    if (f & 0x40u) {   // face 3: nodes 1 2 3
+        const float4 v = *reinterpret_cast<const float4*>(bb + __float_as_int(s1.w));
+        const float u0 = swapped ? v.z : v.x, u1 = swapped ? v.x : v.y, u2 = swapped ? v.y : v.z;
+        const float U = u0 + u1 + u2, t3 = U * kThird;
+        r[1] = fmaf(-c.w, fmaf(kFiveThirds, u0, t3), r[1]);
+        r[2] = fmaf(-c.w, fmaf(kFiveThirds, u1, t3), r[2]);
+        r[3] = fmaf(-c.w, fmaf(kFiveThirds, u2, t3), r[3]);
+        r[0] = fmaf(c.w * kFourThirds, U, r[0]);
+    }
+    if (((word ^ (int)(f >> 7)) & 0xF) != 0) {
+        // a face nearly parallel to the direction: the schedule's outflow mask differs from the table's
+        Update u;
+        auto no_face = [](int, float&, float&, float&) {};
+        assemble_sys(make_float4(r[0], r[1], r[2], r[3]), dir, 0, (int)((f >> 7) & 0xFu), s_x[4 * t], s_x[4 * t + 1],
+                     s_x[4 * t + 2], s_sig[t], no_face, u);
+        solve_rank2(u);
+        *mine = make_float4(u.r[0], u.r[1], u.r[2], u.r[3]);
+        return;
+    }
+    const float4 A = T->a, B = T->b, S0 = T->s0;
+    const float v0 = (r[0] + r[1]) + (r[2] + r[3]);
+    const float v1 = fmaf(B.x, r[0], fmaf(B.y, r[1], fmaf(B.z, r[2], B.w * r[3])));
+    const float z0 = fmaf(S0.y, v0, -4.0f * v1) * S0.w;
+    const float z1 = fmaf(S0.x, v1, -S0.z * v0) * S0.w;
+    *mine = make_float4((r[0] - fmaf(A.x, z0, z1)) * s1.x, (r[1] - fmaf(A.y, z0, z1)) * s1.x,
+                        (r[2] - fmaf(A.z, z0, z1)) * s1.x, (r[3] - fmaf(A.w, z0, z1)) * s1.x);
+}
+
+// Barrier of the `threads` threads of team `team` of a CTA (0 of 1: the whole CTA).
+template <int NT, int TEAM>
+__device__ __forceinline__ void team_sync(int team) {
+    if (NT == TEAM) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(TEAM) : "memory");
+}
+
+// All groups of one direction, walked by the TEAM threads of team `team` of an NT-thread CTA: rec = its block
+// records, ls[nl + 1] = group starts, base = its angular block, s_tile = the team's rows.
+template <int NT, int TEAM>
+__device__ __forceinline__ void walk_tiles(const int4* __restrict__ rec, const int* __restrict__ ls, int nl, float* base,
+                                           float4 dir, const float4* s_x, const float* s_sig, const ElemTab* s_tab,
+                                           float4* s_tile, int team) {
+    const int tid = threadIdx.x % TEAM, lane = tid & 31;
+    char* wt = reinterpret_cast<char*>(s_tile + (tid - lane) * kTileRow);   // the warp's rows
+    char* row = wt + lane * (16 * kTileRow);
+    char* gb = reinterpret_cast<char*>(base);
+    // a lane moves line lane % 6 of blocks lane / 6, + 5, ... of the warp (lanes 30 and 31 none): all its
+    // shared-memory offsets are constants from mt, a global address is one multiply-add
+    const int mb = lane / kClusterSize;
+    const unsigned ml = 16u * (lane % kClusterSize);
+    char* mt = wt + mb * (16 * kTileRow) + ml;
+    char* mg = gb + ml;
+    const bool mover = lane < 5 * kClusterSize;
+    auto fill = [&](int blk) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            const int b = __shfl_sync(0xffffffffu, blk, mb + 5 * j);
+            if (b >= 0 && mover && (j < 6 || mb < 2)) cp_async16(mt + j * (5 * 16 * kTileRow), mg + (size_t)(unsigned)b * 96u);
+        }
+    };
+    int L = 0, s = __ldg(&ls[0]), s1 = __ldg(&ls[1]);
+    const int4 none = make_int4(-1, 0, 0, 0);
+    int4 r = s + tid < s1 ? __ldcs(rec + s + tid) : none;
+    fill(r.x);
+    while (true) {
+        int ns = s + TEAM, ns1 = s1;
+        const bool last = ns >= s1;   // last pass of the group
+        if (last) {
+            ++L;
+            ns = s1;
+            if (L < nl) ns1 = __ldg(&ls[L + 1]);
+        }
+        const int4 rn = ns + tid < ns1 ? __ldcs(rec + ns + tid) : none;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (r.x >= 0) {
+            const char* bb = gb + (size_t)(unsigned)r.x * 96u;
+            unsigned w0 = (unsigned)r.y, w1 = (unsigned)r.z, w2 = (unsigned)r.w;
+#pragma unroll 1
+            for (int k = 0; k < kClusterSize; k += 2) {
+                tile_update(row, bb, w0 & 0xFFFFu, dir, s_x, s_sig, s_tab);
+                tile_update(row, bb, w0 >> 16, dir, s_x, s_sig, s_tab);
+                w0 = w1;
+                w1 = w2;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            const int b = __shfl_sync(0xffffffffu, r.x, mb + 5 * j);
+            if (b >= 0 && mover && (j < 6 || mb < 2))
+                *reinterpret_cast<float4*>(mg + (size_t)(unsigned)b * 96u) =
+                    *reinterpret_cast<const float4*>(mt + j * (5 * 16 * kTileRow));
+        }
+        __syncwarp();
+        fill(rn.x);
+        if (last) {
+            team_sync<NT, TEAM>(team);
+            if (L >= nl) break;
+        }
+        s = ns;
+        s1 = ns1;
+        r = rn;
+    }
+}
+
+// Shared memory of the tile sweep: types (4 lines each), cross sections, per-direction tables, tile rows.
+constexpr size_t tile_smem(int nt, int nx) {
+    return 64 * (size_t)nx + 16 * (((size_t)nx + 3) / 4) + sizeof(ElemTab) * (size_t)nx + 16 * (size_t)kTileRow * nt;
+}
+
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) sweep_tile_kernel(SweepArgs a) {
+    extern __shared__ float4 s_dyn[];
+    float4* s_x = s_dyn;
+    float* s_sig = reinterpret_cast<float*>(s_x + 4 * a.nxtype);
+    ElemTab* s_tab = reinterpret_cast<ElemTab*>(s_x + 4 * a.nxtype + (a.nxtype + 3) / 4);
+    float4* s_tile = reinterpret_cast<float4*>(s_tab + a.nxtype);
+    for (int k = threadIdx.x; k < 4 * a.nxtype; k += NT) s_x[k] = __ldg(&a.xtab[k]);
+    for (int k = threadIdx.x; k < a.nxtype; k += NT) s_sig[k] = a.sigt[__ldg(&a.xmat[k])];
+    __syncthreads();
+    for (int i = blockIdx.x; i < a.NI; i += gridDim.x) {
+        const float4 dir = __ldg(&a.dirs[i]);
+        build_tab<true>(s_x, s_sig, a.nxtype, dir, s_tab, threadIdx.x, NT);
+        __syncthreads();
+        walk_tiles<NT, NT>(a.crec + __ldg(&a.crec_base[i]), a.cl_start + __ldg(&a.cl_base[i]), __ldg(&a.ncl[i]),
+                           a.psi + (size_t)i * (size_t)a.NENK, dir, s_x, s_sig, s_tab, s_tile, 0);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Batched level schedule: one persistent launch over the directions of many independent problems
 // (meshes, quadratures and cross sections differ).  A direction whose problem has a block schedule is
 // walked block level by block level, as the cluster kernel does, with the problem's element types
@@ -655,43 +870,71 @@ __global__ void __launch_bounds__(NT, MINB) sweep_cluster_kernel(SweepArgs a) {
 // counter, so items sorted by decreasing cost give a longest-first list schedule; each item is a
 // whole direction walked level by level with a CTA barrier between levels, exactly like the
 // single-problem level kernel (same element update, bit-identical results).
+//
+// The TEAM threads that take an item are the whole CTA, or a quarter or half of it: the block levels of a batch's
+// small meshes (8 to 20 hexes per axis: at most a few hundred blocks) leave most of 512 threads idle, and a batch
+// has far more directions than the chip has CTAs, so smaller teams keep more directions in flight per SM.
 // ---------------------------------------------------------------------------------------------
-template <int NT>
-__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) sweep_batch_kernel(const BatchWork* __restrict__ work, int nwork, int* counter,
-                                                        const int* __restrict__ active) {
-    __shared__ float s_sigt[256];
-    __shared__ float4 s_gt[3 * 256];   // the item's element types (face vectors), when it has a type table
-    __shared__ int s_w;
+// Shared memory of a team: tile rows (or the face vectors of up to 256 element types), tile types and their
+// tables, cross sections.
+constexpr int batch_rows(int team) { return kTileRow * team > 3 * 256 ? kTileRow * team : 3 * 256; }
+constexpr size_t batch_team_smem(int team) {
+    return 16 * ((size_t)batch_rows(team) + 4 * kMaxTileTypes + 64) + sizeof(ElemTab) * kMaxTileTypes;
+}
+
+template <int TEAM>
+__global__ void __launch_bounds__(kBatchThreads, 2) sweep_batch_kernel(const BatchWork* __restrict__ work, int nwork,
+                                                                       int* counter, const int* __restrict__ active) {
+    constexpr int NT = kBatchThreads;
+    extern __shared__ float4 s_dyn[];
+    __shared__ int s_work[NT / TEAM];
+    const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
+    float4* s_gt = s_dyn + team * (batch_team_smem(TEAM) / 16);   // tile rows or element types
+    float4* s_x = s_gt + batch_rows(TEAM);
+    ElemTab* s_tab = reinterpret_cast<ElemTab*>(s_x + 4 * kMaxTileTypes);
+    float* s_sigt = reinterpret_cast<float*>(s_tab + kMaxTileTypes);   // [256]
     for (;;) {
-        if (threadIdx.x == 0) s_w = atomicAdd(counter, 1);
-        __syncthreads();
-        const int w = s_w;
+        if (tt == 0) s_work[team] = atomicAdd(counter, 1);
+        team_sync<NT, TEAM>(team);
+        const int w = s_work[team];
         if (w >= nwork) return;
         const BatchWork* W = work + w;
         const int prob = __ldg(&W->problem);
         if (active && __ldg(&active[prob]) == 0) {
-            __syncthreads();
+            team_sync<NT, TEAM>(team);
             continue;
         }
         const int Nm = __ldg(&W->Nm);
         const float* sg = W->sigt;
         const int ngeom = __ldg(&W->ngeom);
+        const int nx = __ldg(&W->nxtype);
         const int4* crec = W->crec;
+        if (nx > 0) {
+            // block tiles, as sweep_tile_kernel
+            for (int k = tt; k < 4 * nx; k += TEAM) s_x[k] = __ldg(&W->xtab[k]);
+            for (int k = tt; k < nx; k += TEAM) s_sigt[k] = __ldg(&sg[__ldg(&W->xmat[k])]);
+            team_sync<NT, TEAM>(team);
+            const float4 d = __ldg(&W->dir);
+            build_tab<true>(s_x, s_sigt, nx, d, s_tab, tt, TEAM);
+            team_sync<NT, TEAM>(team);
+            walk_tiles<NT, TEAM>(crec, W->cl_start, __ldg(&W->ncl), W->psi, d, s_x, s_sigt, s_tab, s_gt, team);
+            continue;
+        }
         // cross sections by material, or by element type when the problem has a type table
-        for (int m = threadIdx.x; m < 256; m += NT) {
+        for (int m = tt; m < 256; m += TEAM) {
             float v = 0.f;
             if (ngeom > 0) v = (m < ngeom) ? __ldg(&sg[__ldg(&W->tmat[m])]) : 0.f;
             else v = (m < Nm) ? __ldg(&sg[m]) : 0.f;
             s_sigt[m] = v;
         }
-        for (int k = threadIdx.x; k < 3 * ngeom; k += NT) s_gt[k] = __ldg(&W->gtab[k]);
+        for (int k = tt; k < 3 * ngeom; k += TEAM) s_gt[k] = __ldg(&W->gtab[k]);
         const int nl = __ldg(&W->nlev);
         const int* ls = W->lvl_start;
         const int* it = W->items;
         const float4* geom = W->geom;
         float* base = W->psi;
         const float4 dir = __ldg(&W->dir);
-        __syncthreads();
+        team_sync<NT, TEAM>(team);
         if (crec) {
             // block schedule, as sweep_cluster_kernel
             const int ncl = __ldg(&W->ncl);
@@ -699,7 +942,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) sweep_batch_kernel(con
             const int4* rec = W->rec;
             for (int L = 0; L < ncl; ++L) {
                 const int s0 = __ldg(&cls[L]), s1 = __ldg(&cls[L + 1]);
-                for (int cs = s0 + threadIdx.x; cs < s1; cs += NT) {
+                for (int cs = s0 + tt; cs < s1; cs += TEAM) {
                     const int4 r = __ldcs(crec + cs);
                     const int e0 = r.x * kClusterSize;
                     const int* mem = W->blk_elem ? W->blk_elem + e0 : nullptr;
@@ -760,20 +1003,20 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) sweep_batch_kernel(con
                         finish<false>(base, item, up);
                     }
                 }
-                __syncthreads();
+                team_sync<NT, TEAM>(team);
             }
             continue;
         }
         for (int L = 0; L < nl; ++L) {
             const int s0 = __ldg(&ls[L]), s1 = __ldg(&ls[L + 1]);
-            for (int es = s0 + threadIdx.x; es < s1; es += NT) {
+            for (int es = s0 + tt; es < s1; es += TEAM) {
                 const int item = __ldcs(&it[es]);
                 const Geom g = load_geom(geom, item & 0xFFFFFF);
                 Update up;
                 assemble_g<false>(base, dir, item, g, s_sigt, up, make_float4(0.f, 0.f, 0.f, 0.f));
                 finish<false>(base, item, up);
             }
-            __syncthreads();
+            team_sync<NT, TEAM>(team);
         }
     }
 }
@@ -1032,9 +1275,10 @@ __global__ void __launch_bounds__(256) sweep_dataflow_kernel(SweepArgs a) {
 
 struct Config {
     int kind;      // 0 levels, 1 dataflow, 2 levels with next-level prefetch, 3 element flags, 4 grouped levels,
-                   // 5 blocks of elements (cluster records), 6 the same with per-type element tables
+                   // 5 blocks of elements (cluster records), 6 the same with per-type element tables,
+                   // 7 blocks moved through shared-memory tiles
     int threads;
-    int dpc;       // directions per CTA (kind 0); minimum CTAs per SM (kinds 2, 5)
+    int dpc;       // directions per CTA (kind 0); minimum CTAs per SM (kinds 2, 5 to 7)
     int ilp;       // updates in flight per thread (kind 0); kinds 5, 6: 2 = next element's record and source
                    // prefetched, 3 = the same and the previous element's solution kept in registers, 4 = the
                    // same with the two previous elements' solutions
@@ -1045,8 +1289,17 @@ const Config kConfigs[] = {
     {0, 1024, 1, 1}, {0, 512, 1, 1}, {2, 1024, 1, 1}, {3, 512, 0, 1}, {1, 256, 0, 0},
     {4, 768, 2, 1}, {0, 1024, 1, 2}, {0, 1024, 1, 3}, {0, 768, 1, 3}, {5, 1024, 1, 1}, {5, 512, 2, 1}, {5, 768, 2, 1}, {5, 1024, 2, 1},
     {6, 512, 2, 1}, {6, 768, 2, 1}, {5, 512, 2, 2}, {6, 512, 2, 2}, {5, 512, 2, 3}, {5, 512, 2, 4},
+    {7, 512, 2, 1},
 };
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
+// Where the tile schedule applies it is taken without trials: it was the fastest on every box tried, from 6,000
+// tets and 80 directions (0.089 ms against 0.099 for the best other) to 768,000 and 288 (3.03 against 4.15).
+constexpr int kTileConfig = 24;
+// The candidates timed on other meshes: element levels (512 and 1024 threads, with prefetch, two updates in
+// flight) and the block walks with the next element prefetched.  The others never came first on any mesh
+// measured (1.05 to 35 times the best); LB_SWEEP_CONFIG still runs them.
+const int kTrials[] = {5, 6, 7, 11, 20, 22, 23};
+constexpr int kNumTrials = sizeof(kTrials) / sizeof(kTrials[0]);
 constexpr int kFinalists = 3;   // candidates timed a second time before one is kept
 
 template <int DPC, int ILP>
@@ -1130,6 +1383,21 @@ cudaError_t launch_cluster(const SweepArgs& a, int sm_count, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <int NT, int MINB>
+cudaError_t launch_tile(const SweepArgs& a, int sm_count, cudaStream_t s) {
+    const size_t smem = tile_smem(NT, a.nxtype);
+    static PerDevice attr;
+    attr.get([&] {
+        allow_max_dynamic_smem(sweep_tile_kernel<NT, MINB>);
+        return 1;
+    });
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_tile_kernel<NT, MINB>, NT, smem);
+    if (per_sm < 1) per_sm = 1;
+    sweep_tile_kernel<NT, MINB><<<std::min(a.NI, sm_count * per_sm), NT, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
 template <int MINB>
 cudaError_t launch_levels_pf(const SweepArgs& a, int threads, int sm_count, cudaStream_t s) {
     const size_t smem = sizeof(float4) * 3 * (size_t)a.ngeom;
@@ -1143,27 +1411,27 @@ cudaError_t launch_levels_pf(const SweepArgs& a, int threads, int sm_count, cuda
 
 }  // namespace
 
-int launch_sweep_batch(cudaStream_t st, const BatchWork* work, int nwork, int* counter, const int* active, int threads,
+int launch_sweep_batch(cudaStream_t st, const BatchWork* work, int nwork, int* counter, const int* active, int team,
                        int sm_count) {
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return LB_ERR_CUDA;
-    if (threads == 512) {
-        static PerDevice per_sm_cache;
-        const int per_sm = per_sm_cache.get([&] {
+    auto run = [&](auto kernel, PerDevice& cache) {
+        const int teams = kBatchThreads / team;
+        const size_t smem = batch_team_smem(team) * teams;
+        const int per_sm = cache.get([&] {
             int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_batch_kernel<512>, 512, 0);
+            allow_max_dynamic_smem(kernel);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBatchThreads, smem);
             return n < 1 ? 1 : n;
         });
-        sweep_batch_kernel<512><<<std::min(nwork, sm_count * per_sm), 512, 0, st>>>(work, nwork, counter, active);
-    } else {
-        static PerDevice per_sm_cache;
-        const int per_sm = per_sm_cache.get([&] {
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_batch_kernel<1024>, 1024, 0);
-            return n < 1 ? 1 : n;
-        });
-        sweep_batch_kernel<1024><<<std::min(nwork, sm_count * per_sm), 1024, 0, st>>>(work, nwork, counter, active);
-    }
+        kernel<<<std::min((nwork + teams - 1) / teams, sm_count * per_sm), kBatchThreads, smem, st>>>(work, nwork, counter,
+                                                                                                  active);
+    };
+    static PerDevice cache[3];
+    if (team == 512) run(sweep_batch_kernel<512>, cache[0]);
+    else if (team == 256) run(sweep_batch_kernel<256>, cache[1]);
+    else if (team == 128) run(sweep_batch_kernel<128>, cache[2]);
+    else return LB_ERR_ARG;
     return cudaGetLastError() == cudaSuccess ? LB_OK : LB_ERR_CUDA;
 }
 
@@ -1200,6 +1468,9 @@ int launch_sweep(Handle* h, float* psi) {
     a.cl_base = h->d_cl_base;
     a.ncl = h->d_ncl;
     a.nclusters = h->nclusters;
+    a.xtab = h->d_xtab;
+    a.xmat = h->d_xmat;
+    a.nxtype = h->tiles_ok ? h->nxtype : 0;
 
     if (h->sweep_cfg_forced < 0) {
         const char* env = std::getenv("LB_SWEEP_CONFIG");
@@ -1210,39 +1481,19 @@ int launch_sweep(Handle* h, float* psi) {
     bool tuning = false;
     if (h->sweep_cfg_forced < kNumConfigs) cfg_idx = h->sweep_cfg_forced;
     else if (h->sweep_cfg >= 0) cfg_idx = h->sweep_cfg;
+    else if (h->tiles_ok) cfg_idx = h->sweep_cfg = kTileConfig;
     else {
         // a first pass times every candidate once; a second pass times the kFinalists fastest once more
-        cfg_idx = h->sweep_trial < kNumConfigs ? h->sweep_trial : h->sweep_finalists[h->sweep_trial - kNumConfigs];
+        cfg_idx = kTrials[h->sweep_trial < kNumTrials ? h->sweep_trial : h->sweep_finalists[h->sweep_trial - kNumTrials]];
         tuning = true;
     }
     if (tuning && h->sweep_trial == 0) {
         // load every candidate's module before timing, so the first trial does not pay for it
         cudaFuncAttributes fa;
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<2, 1024>);
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<2, 512>);
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<3, 1024>);
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<3, 512>);
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<6, 512>);
-        cudaFuncGetAttributes(&fa, sweep_flags_kernel<256>);
-        cudaFuncGetAttributes(&fa, sweep_flags_kernel<512>);
-        cudaFuncGetAttributes(&fa, sweep_flags_kernel<1024>);
         cudaFuncGetAttributes(&fa, sweep_levels_pf_kernel<1>);
-        cudaFuncGetAttributes(&fa, sweep_levels_pf_kernel<2>);
         cudaFuncGetAttributes(&fa, sweep_levels_kernel<1, 1>);
         cudaFuncGetAttributes(&fa, sweep_levels_kernel<1, 2>);
-        cudaFuncGetAttributes(&fa, sweep_levels_kernel<1, 3>);
-        cudaFuncGetAttributes(&fa, sweep_levels_kernel<2, 1>);
-        cudaFuncGetAttributes(&fa, sweep_levels_kernel<2, 2>);
-        cudaFuncGetAttributes(&fa, sweep_dataflow_kernel);
-        cudaFuncGetAttributes(&fa, sweep_group_kernel<2, 768>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<1024, 1, false, 0>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<1024, 2, false, 0>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<768, 2, false, 0>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 0>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, true, 0>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<768, 2, true, 0>);
         cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 1>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, true, 1>);
         cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 2>);
         cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 3>);
     }
@@ -1250,9 +1501,10 @@ int launch_sweep(Handle* h, float* psi) {
     // the autotuner skips the block schedule where it has more barrier levels than the element schedule
     // (unstructured meshes, whose blocks are split on cycles): it cannot win there; a forced
     // configuration still runs it
-    if ((cfg.kind == 5 || cfg.kind == 6) && h->sweep_cfg_forced >= kNumConfigs &&
-        h->cluster_levels_total > (long long)h->total_levels)
+    if (cfg.kind >= 5 && h->sweep_cfg_forced >= kNumConfigs && h->cluster_levels_total > (long long)h->total_levels)
         cfg = Config{0, 1024, 1, 2};
+    // the tile schedule needs whole blocks of elements with tile types
+    if (cfg.kind >= 7 && !h->tiles_ok) cfg = h->nclusters > 0 ? Config{5, 512, 2, 4} : Config{0, 1024, 1, 2};
     // the element-flag schedule keeps one bit per element in shared memory
     if (cfg.kind == 3 && (size_t)((h->NE + 31) / 32) * 4 > 200 * 1024) cfg = Config{0, 1024, 1, 1};
     // the cluster schedule needs block records (built when every direction's block graph is acyclic)
@@ -1287,6 +1539,8 @@ int launch_sweep(Handle* h, float* psi) {
         e = (cfg.threads == 256) ? launch_flags<256>(a, h->sm_count, h->stream)
           : (cfg.threads == 1024) ? launch_flags<1024>(a, h->sm_count, h->stream)
                                   : launch_flags<512>(a, h->sm_count, h->stream);
+    } else if (cfg.kind == 7) {
+        e = launch_tile<512, 2>(a, h->sm_count, h->stream);
     } else if ((cfg.kind == 5 || cfg.kind == 6) && cfg.ilp >= 2) {
         e = cfg.kind == 6   ? launch_cluster<512, 2, true, 1>(a, h->sm_count, h->stream)
             : cfg.ilp == 4 ? launch_cluster<512, 2, false, 3>(a, h->sm_count, h->stream)
@@ -1343,32 +1597,33 @@ int launch_sweep(Handle* h, float* psi) {
         cudaEventElapsedTime(&ms, t.a, t.b);
         h->sweep_trial_ms.push_back(ms);
         ++h->sweep_trial;
-        if (h->sweep_trial == kNumConfigs) {
-            std::vector<int> order(kNumConfigs);
-            for (int c = 0; c < kNumConfigs; ++c) order[c] = c;
+        if (h->sweep_trial == kNumTrials) {
+            std::vector<int> order(kNumTrials);
+            for (int c = 0; c < kNumTrials; ++c) order[c] = c;
             std::stable_sort(order.begin(), order.end(),
                              [&](int x, int y) { return h->sweep_trial_ms[x] < h->sweep_trial_ms[y]; });
-            h->sweep_finalists.assign(order.begin(), order.begin() + std::min(kFinalists, kNumConfigs));
+            h->sweep_finalists.assign(order.begin(), order.begin() + std::min(kFinalists, kNumTrials));
         }
         const int nfin = (int)h->sweep_finalists.size();
-        if (h->sweep_trial == kNumConfigs + nfin) {
+        if (h->sweep_trial == kNumTrials + nfin) {
             // the finalist with the smallest sum of its two times (one noisy sweep decides nothing)
             int best = -1;
             float best_ms = 0.f;
             for (int q = 0; q < nfin; ++q) {
                 const int c = h->sweep_finalists[q];
-                const float tot = h->sweep_trial_ms[c] + h->sweep_trial_ms[kNumConfigs + q];
+                const float tot = h->sweep_trial_ms[c] + h->sweep_trial_ms[kNumTrials + q];
                 if (best < 0 || tot < best_ms) { best = c; best_ms = tot; }
             }
-            h->sweep_cfg = best;
+            h->sweep_cfg = kTrials[best];
             const char* verbose = std::getenv("LB_SWEEP_VERBOSE");
             if (verbose && *verbose == '1')
-                for (int c = 0; c < kNumConfigs; ++c) {
+                for (int c = 0; c < kNumTrials; ++c) {
                     float again = -1.f;
                     for (int q = 0; q < nfin; ++q)
-                        if (h->sweep_finalists[q] == c) again = h->sweep_trial_ms[kNumConfigs + q];
-                    std::fprintf(stderr, "sweep config %d (kind %d threads %d dpc %d ilp %d): %.3f ms", c, kConfigs[c].kind,
-                                 kConfigs[c].threads, kConfigs[c].dpc, kConfigs[c].ilp, h->sweep_trial_ms[c]);
+                        if (h->sweep_finalists[q] == c) again = h->sweep_trial_ms[kNumTrials + q];
+                    const Config& k = kConfigs[kTrials[c]];
+                    std::fprintf(stderr, "sweep config %d (kind %d threads %d dpc %d ilp %d): %.3f ms", kTrials[c], k.kind,
+                                 k.threads, k.dpc, k.ilp, h->sweep_trial_ms[c]);
                     if (again >= 0.f) std::fprintf(stderr, ", again %.3f ms", again);
                     std::fprintf(stderr, "%s\n", c == best ? "  <- chosen" : "");
                 }
@@ -1379,14 +1634,16 @@ int launch_sweep(Handle* h, float* psi) {
 
 int sweep_config(Handle* h, int* kind, int* threads, int* dpc, int* ilp) {
     int c = h->sweep_cfg_forced >= 0 && h->sweep_cfg_forced < kNumConfigs ? h->sweep_cfg_forced : h->sweep_cfg;
+    if (c < 0 && h->tiles_ok && h->sweep_cfg_forced != -1) c = kTileConfig;
     if (c < 0) return -1;
     Config cfg = kConfigs[c];
-    if ((cfg.kind == 5 || cfg.kind == 6) && h->sweep_cfg_forced >= kNumConfigs &&
+    if (cfg.kind >= 5 && h->sweep_cfg_forced >= kNumConfigs &&
         h->cluster_levels_total > (long long)h->total_levels)
         cfg = Config{0, 1024, 1, 2};   // what the launcher runs instead
     if (cfg.kind == 5 && h->nclusters <= 0) cfg = Config{0, 1024, 1, 2};   // what the launcher runs instead
     if (cfg.kind == 6 && (h->nclusters <= 0 || h->ngeom <= 0))
         cfg = h->nclusters > 0 ? Config{5, 512, 2, 1} : Config{0, 1024, 1, 2};
+    if (cfg.kind >= 7 && !h->tiles_ok) cfg = h->nclusters > 0 ? Config{5, 512, 2, 4} : Config{0, 1024, 1, 2};
     *kind = cfg.kind; *threads = cfg.threads; *dpc = cfg.dpc; *ilp = cfg.ilp;
     return c;
 }

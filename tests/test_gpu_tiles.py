@@ -1,0 +1,80 @@
+"""The tile sweep (whole blocks moved through shared memory) on the GPU: the same numbers as the level
+schedule, bit for bit, and the oracle's T^-1, at the sizes where its passes and rows change."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import rel_l2
+from lionbolt_b200 import AngularClass, TransportOp, XSType
+from lionbolt_b200 import mesh as M
+from lionbolt_b200 import problems as P
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5                       # FP32 sweep against the FP64 oracle, as in the other sweep tests
+LEVELS = 6                       # launch candidate: element levels, 512 threads
+TILES = {24: "block tiles"}
+
+
+def _two(c):
+    return (c[:, 0] > 1.0).astype(np.int32)
+
+
+# hexes per axis: one block; fewer blocks than a warp; a level just over one CTA pass of 128, 256 or 512
+# threads (the widest block level of an n^3 box has about 3 n^2 / 4 blocks)
+BOXES = [(1, 1, 1), (2, 1, 3), (5, 4, 3), (14, 14, 14), (19, 20, 18), (27, 28, 26)]
+
+
+def _sweep(monkeypatch, cfg, m, k, w, sigt, q):
+    monkeypatch.setenv("LB_SWEEP_CONFIG", str(cfg))
+    T = TransportOp().Build(m, AngularClass(k=k, w=w), XSType(sigt, np.zeros((sigt.size, 1))))
+    v = q.copy()
+    T.MatInv(v)
+    T.MatInv(v)                  # the second sweep reads what the first one wrote
+    return T, v
+
+
+@pytest.mark.parametrize("n", BOXES)
+@pytest.mark.parametrize("cfg", sorted(TILES))
+def test_tile_sweep_is_bit_identical_to_element_levels(cfg, n, monkeypatch):
+    m = M.box_mesh(*n, (0, 0, 0), (2.0, 1.5, 2.5), material=_two, Nm=2)
+    k, w = P.quadrature(2, 6)
+    sigt = np.array([0.3, 1.7])
+    q = np.random.default_rng(cfg).uniform(size=m.NENK * len(w))
+    T, v = _sweep(monkeypatch, cfg, m, k, w, sigt, q)
+    assert T._h.sweep_config()["schedule"] == TILES[cfg]
+    _, ref = _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)
+    assert np.array_equal(v, ref)
+    if m.NE < 5000:
+        o = O.Oracle(m)
+        assert o.set_angular(k, w, 0) == 0
+        o.set_xs(sigt, np.zeros((2, 1)))
+        assert rel_l2(v, o.transport_inv(o.transport_inv(q))) < TOL
+
+
+def test_more_tile_types_than_a_slot_names_take_the_cluster_schedule(monkeypatch):
+    """11 materials of 6 shapes give more than 32 tile types: the tile candidates run the cluster schedule instead."""
+    m = M.box_mesh(11, 3, 3, (0, 0, 0), (11, 3, 3), material=lambda c: c[:, 0].astype(np.int32), Nm=11)
+    k, w = P.quadrature(2, 4)
+    sigt = np.linspace(0.1, 2.0, 11)
+    q = np.random.default_rng(0).uniform(size=m.NENK * len(w))
+    T, v = _sweep(monkeypatch, 24, m, k, w, sigt, q)
+    assert T._h.sweep_config()["schedule"].startswith("cluster levels")
+    assert np.array_equal(v, _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)[1])
+
+
+@pytest.mark.parametrize("n,quad,count", [((27, 26, 28), (2, 4), 1), ((19, 20, 18), (4, 8), 10), ((5, 4, 6), (8, 10), 8)])
+def test_batched_tile_sweep_matches_single_solves(n, quad, count):
+    """Batches whose groups suit teams of 512, 256 and 128 threads per direction (few wide directions, many
+    middling ones, many small ones), against the single-problem solver (reduction order inside GMRES: 1e-6)."""
+    from lionbolt_b200 import BatchSolver, MultigroupSolver
+    probs = [P.multigroup_box(n=n, size=tuple(0.5 * v for v in n), Ng=quad[0], Nc=quad[1], G=1, Ls=2, seed=s,
+                              slab=(0.5, 1.5)) for s in range(count)]
+    bs = BatchSolver()
+    for p in probs:
+        bs.add_problem(p)
+    bs.solve(m=20, rtol=1e-8)
+    for i in {0, count - 1}:
+        mg = MultigroupSolver().set_problem(probs[i])
+        mg.solve("GMRES", m=20, rtol=1e-8)
+        assert rel_l2(bs.results(i)[1], mg.results()[1]) < 1e-6
