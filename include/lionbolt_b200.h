@@ -111,14 +111,12 @@ int lb_transport_inv(lb_handle* h, double* s);
  * aligned (LB_ERR_ARG otherwise, before anything is launched).  No
  * counterpart in the reference: it exists for callers that cannot allocate device memory at solve
  * time (a host framework that owns the allocator, a Fortran runtime that only passes pre-allocated
- * device arrays, a loop that must not hit cudaMalloc's implicit synchronisation).  Its dependency
- * counters live in a fixed 1 MiB file-scope device array (at most 262,144 direction-level pairs;
- * larger schedules return LB_ERR_ARG) that every GPU loading the library keeps until exit.  The
- * first call on a device looks up the array's device address.  The call runs the dataflow sweep
- * schedule (not the autotuned one of lb_transport_inv) on the handle's stream and waits for it, so
- * it cannot be stream-captured; writes to psi queued on other streams must be finished first (an
- * event wait or a host synchronisation).  All calls on a device share the array: calls that
- * overlap on the GPU race. */
+ * device arrays, a loop that must not hit cudaMalloc's implicit synchronisation).  It uses no scratch: it runs
+ * the handle's sweep schedule where that is known (tiles, or the autotuner's pick once made), element
+ * levels before, with bit-identical results.  Schedules of more than 262,144 direction-level pairs return
+ * LB_ERR_ARG.  The call runs on the handle's stream and waits for it, so it cannot be stream-captured;
+ * writes to psi queued on other streams must be finished first (an event wait or a host
+ * synchronisation). */
 int lb_transport_inv_noalloc(lb_handle* h, float* psi);
 
 /* The two halves of K on caller-owned device arrays of the handle's GPU, asynchronous on the

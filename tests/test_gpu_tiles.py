@@ -78,3 +78,31 @@ def test_batched_tile_sweep_matches_single_solves(n, quad, count):
         mg = MultigroupSolver().set_problem(probs[i])
         mg.solve("GMRES", m=20, rtol=1e-8)
         assert rel_l2(bs.results(i)[1], mg.results()[1]) < 1e-6
+
+
+@pytest.mark.parametrize("amount", [0.0, 0.07])
+def test_noalloc_sweep_runs_the_handles_schedule(amount):
+    """lb_transport_inv_noalloc on a box (tiles) and on a jittered box (element levels before the autotuner's
+    pick, the pick after it): the bits of TransportOp.MatInv, sources in FP32."""
+    import ctypes
+    import torch
+    from helpers import jittered
+    m = M.box_mesh(6, 5, 7, (0, 0, 0), (3.0, 2.5, 3.5), material=_two, Nm=2)
+    if amount:
+        m = jittered(m, amount)
+    k, w = P.quadrature(4, 6)
+    T = TransportOp().Build(m, AngularClass(k=k, w=w), XSType(np.array([0.3, 1.7]), np.zeros((2, 1))))
+    q = np.random.default_rng(3).uniform(size=m.NENK * len(w)).astype(np.float32)
+
+    def noalloc():
+        d = torch.from_numpy(q).to("cuda:0")
+        torch.cuda.synchronize()
+        T._h.call("lb_transport_inv_noalloc", ctypes.c_void_p(d.data_ptr()))
+        return d.cpu().numpy().astype(np.float64)
+
+    first = noalloc()
+    for _ in range(12):
+        ref = q.astype(np.float64)
+        T.MatInv(ref)
+    assert T._h.sweep_config() is not None
+    assert np.array_equal(first, ref) and np.array_equal(noalloc(), ref)
