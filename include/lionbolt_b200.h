@@ -112,8 +112,8 @@ int lb_transport_inv(lb_handle* h, double* s);
  * counterpart in the reference: it exists for callers that cannot allocate device memory at solve
  * time (a host framework that owns the allocator, a Fortran runtime that only passes pre-allocated
  * device arrays, a loop that must not hit cudaMalloc's implicit synchronisation).  It uses no scratch: it runs
- * the handle's sweep schedule where that is known (tiles, or the autotuner's pick once made), element
- * levels before, with bit-identical results.  Schedules of more than 262,144 direction-level pairs return
+ * the handle's sweep schedule where that is known (tiles, or the autotuner's pick once made), the level
+ * relay before, with bit-identical results.  Schedules of more than 262,144 direction-level pairs return
  * LB_ERR_ARG.  The call runs on the handle's stream and waits for it, so it cannot be stream-captured;
  * writes to psi queued on other streams must be finished first (an event wait or a host
  * synchronisation). */
@@ -201,11 +201,12 @@ int lb_synchronize(lb_handle* h);
  * synchronisation reports, LB_ERR_TIMEOUT (message in lb_last_error), and clears the flag, so the
  * handle stays usable. */
 int lb_probe_pipeline_timeout(lb_handle* h, long long polls);
-/* Sweep launch shape (the tile schedule on meshes of hexes split along their main diagonal, elsewhere the
- * autotuner's pick): cfg[0] schedule (0 levels, 1 dataflow, 2 levels with
+/* Sweep launch shape (tiles or the resident relay on meshes of hexes split along their main diagonal, elsewhere
+ * the autotuner's pick): cfg[0] schedule (0 levels, 1 dataflow, 2 levels with
  * next-level prefetch, 3 element flags, 4 grouped directions, 5 blocks of 6 elements swept as
- * units, 6 the same with per-type element tables, 7 the same blocks moved through shared-memory tiles),
- * cfg[1] threads per CTA, cfg[2] directions per CTA (minimum CTAs per SM for 5, 6 and 7), cfg[3] updates in flight per thread.  Returns
+ * units, 6 the same with per-type element tables, 7 the same blocks moved through shared-memory tiles, 8
+ * element levels in relay, 9 the same with the direction in shared memory), cfg[1] threads per CTA, cfg[2] directions per CTA (minimum
+ * CTAs per SM for 5 to 9), cfg[3] updates in flight per thread.  Returns
  * LB_ERR_STATE while candidates are still being timed (the first sweeps of a handle). */
 int lb_get_sweep_config(lb_handle* h, int* cfg);
 

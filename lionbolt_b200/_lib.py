@@ -204,14 +204,14 @@ class Handle:
         if st != LB_OK:
             return None
         names = ("levels", "dataflow", "levels+prefetch", "element flags", "grouped directions", "cluster levels",
-                 "cluster levels+type tables", "block tiles")
+                 "cluster levels+type tables", "block tiles", "level relay", "resident level relay")
         kind = int(cfg[0])
         d = dict(schedule=names[kind] if 0 <= kind < len(names) else str(kind), threads=int(cfg[1]),
                  dirs_per_cta=int(cfg[2]), ilp=int(cfg[3]))
         if kind >= 5:
             d["min_ctas_per_sm"] = d.pop("dirs_per_cta")
-            if kind == 7:
-                d["tile_mode"] = d.pop("ilp")
+            if kind >= 7:
+                d.pop("ilp")
                 return d
             if d["ilp"] >= 2:
                 d["schedule"] += "+element prefetch"

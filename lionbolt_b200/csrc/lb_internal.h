@@ -106,6 +106,7 @@ struct Handle {
     std::vector<uint8_t> xtype;    // [NE] tile type of each element (empty: none)
     float4* d_xtab = nullptr;      // [nxtype][4] face vectors and the neighbour words
     int* d_xmat = nullptr;         // [nxtype] material of each tile type
+    uint8_t* d_xtype = nullptr;    // [NE] copy of xtype
     int nxtype = 0;
     bool tiles_ok = false;         // every direction's units are whole blocks of kClusterSize consecutive ids
     // cluster schedule: blocks of up to kClusterSize face-connected elements swept as units (0 blocks:

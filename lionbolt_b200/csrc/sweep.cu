@@ -22,12 +22,14 @@
 //    per direction.
 //  * block tiles: the cluster schedule's blocks moved through shared memory by their warp, without element
 //    records; for meshes of hexes split along their main diagonal, and the fastest there.
+//  * level relay: element levels walked by two halves of a CTA in turn, one making its next elements ready while
+//    the other finishes a pass; for small meshes with the direction in shared memory.
 //  * levels: one CTA owns whole directions and walks their element wavefront levels in order with a
 //    CTA barrier between levels; upstream values written by the same SM are re-read through its L1.
 //  * levels with next-level prefetch, element flags in shared memory, grouped same-schedule
 //    directions, and dataflow (warps claim 32-element chunks from a global counter and wait, with a
 //    bounded spin, on the completion counter of the previous level): candidates for other meshes.
-// Box-like meshes (hexes split along their main diagonal) take the tile schedule; elsewhere the launch shape
+// Meshes of hexes split along their main diagonal take the tile schedule or the resident relay; elsewhere the launch shape
 // (schedule, threads per CTA, directions or CTAs per SM, updates in flight per thread) is picked by timing the
 // first sweeps of a handle (the three fastest twice).  Every candidate computes bit-identical results.
 #include "lb_internal.h"
@@ -80,6 +82,7 @@ struct SweepArgs {
     int nclusters;                    // 0: no cluster schedule
     const float4* __restrict__ xtab;  // [nxtype][4] tile types: face vectors, neighbour words
     const int* __restrict__ xmat;     // [nxtype] material of the tile types
+    const uint8_t* __restrict__ xtype;   // [NE] tile type of each element
     int nxtype;
 };
 
@@ -553,6 +556,94 @@ __global__ void __launch_bounds__(1024, MINB) sweep_levels_pf_kernel(SweepArgs a
     }
 }
 
+__device__ __forceinline__ void cp_async16(const void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
+// An element's update in two parts, for the level relay below.
+//
+// The level kernel is bound by the chain of one level: level bounds, item, element record and source, upstream
+// values, arithmetic, store, barrier (about 4,200 cycles; a level of a 47,000-tet mesh has some 250 elements, a
+// few warps).  Only the upstream values depend on the level before, so while one half of a CTA finishes a pass
+// the other half makes its next elements ready: item, record and source loaded, face coefficients, element
+// matrix and capacitance factors computed.  Same operations as assemble_sys and solve_rank2 (bit-identical).
+// ---------------------------------------------------------------------------------------------
+struct Ready {          // an element whose system is assembled but for its upstream values
+    int item;           // kPad: none
+    unsigned nw[4];
+    float c[4], a[4], b[4];
+    float e00, e11, ba, idet, id;
+    float4 q;
+};
+
+__device__ __forceinline__ void ready_element(const SweepArgs& a, const float* base, float4 dir, int item,
+                                              const float* s_sigt, Ready& p) {
+    p.item = item;
+    if (item == kPad) return;
+    const int e = item & 0xFFFFFF;
+    p.q = ld4<false>(base + 4 * (size_t)e);
+    const Geom G = load_geom(a.geom, e);
+    p.nw[0] = (unsigned)G.gn.x;
+    p.nw[1] = (unsigned)G.gn.y;
+    p.nw[2] = (unsigned)G.gn.z;
+    p.nw[3] = (unsigned)G.gn.w;
+    const int matid = (int)((p.nw[0] >> 30) | ((p.nw[1] >> 30) << 2) | ((p.nw[2] >> 30) << 4) | ((p.nw[3] >> 30) << 6));
+    Update u;
+    auto none = [](int, float&, float&, float&) {};
+    assemble_sys(make_float4(0.f, 0.f, 0.f, 0.f), dir, 0, (item >> 28) & 0xF, G.gx, G.gy, G.gz, s_sigt[matid], none, u);
+    p.c[0] = fmaf(dir.x, G.gx.x, fmaf(dir.y, G.gy.x, dir.z * G.gz.x));
+    p.c[1] = fmaf(dir.x, G.gx.y, fmaf(dir.y, G.gy.y, dir.z * G.gz.y));
+    p.c[2] = fmaf(dir.x, G.gx.z, fmaf(dir.y, G.gy.z, dir.z * G.gz.z));
+    p.c[3] = fmaf(dir.x, G.gx.w, fmaf(dir.y, G.gy.w, dir.z * G.gz.w));
+    // the factors of solve_rank2
+    const float sa = (u.a[0] + u.a[1]) + (u.a[2] + u.a[3]);
+    const float sb = (u.b[0] + u.b[1]) + (u.b[2] + u.b[3]);
+    p.ba = fmaf(u.b[0], u.a[0], fmaf(u.b[1], u.a[1], fmaf(u.b[2], u.a[2], u.b[3] * u.a[3])));
+    p.e00 = u.d + sa;
+    p.e11 = u.d + sb;
+    p.idet = __fdividef(1.0f, fmaf(p.e00, p.e11, -4.0f * p.ba));
+    p.id = __fdividef(1.0f, u.d);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        p.a[k] = u.a[k];
+        p.b[k] = u.b[k];
+    }
+}
+
+__device__ __forceinline__ void finish_ready(float* base, const Ready& p) {
+    constexpr int F[4][3] = {{0, 1, 2}, {0, 1, 3}, {0, 2, 3}, {1, 2, 3}};
+    if (p.item == kPad) return;
+    const int upm = (p.item >> 24) & 0xF;
+    float4 uv[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        if ((upm >> f) & 1) uv[f] = ld4<false>(base + 4 * (size_t)(p.nw[f] & 0xFFFFFFu));
+    float r[4] = {p.q.x, p.q.y, p.q.z, p.q.w};
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+        if ((upm >> f) & 1) {
+            const float u0 = pick(uv[f], (p.nw[f] >> 24) & 3);
+            const float u1 = pick(uv[f], (p.nw[f] >> 26) & 3);
+            const float u2 = pick(uv[f], (p.nw[f] >> 28) & 3);
+            const float U = u0 + u1 + u2;
+            const float t3 = U * kThird;
+            r[F[f][0]] = fmaf(-p.c[f], fmaf(kFiveThirds, u0, t3), r[F[f][0]]);
+            r[F[f][1]] = fmaf(-p.c[f], fmaf(kFiveThirds, u1, t3), r[F[f][1]]);
+            r[F[f][2]] = fmaf(-p.c[f], fmaf(kFiveThirds, u2, t3), r[F[f][2]]);
+            r[3 - f] = fmaf(p.c[f] * kFourThirds, U, r[3 - f]);
+        }
+    }
+    const float v0 = (r[0] + r[1]) + (r[2] + r[3]);
+    const float v1 = fmaf(p.b[0], r[0], fmaf(p.b[1], r[1], fmaf(p.b[2], r[2], p.b[3] * r[3])));
+    const float z0 = fmaf(p.e11, v0, -4.0f * v1) * p.idet;
+    const float z1 = fmaf(p.e00, v1, -p.ba * v0) * p.idet;
+    *reinterpret_cast<float4*>(base + 4 * (size_t)(p.item & 0xFFFFFF)) =
+        make_float4((r[0] - fmaf(p.a[0], z0, z1)) * p.id, (r[1] - fmaf(p.a[1], z0, z1)) * p.id,
+                    (r[2] - fmaf(p.a[2], z0, z1)) * p.id, (r[3] - fmaf(p.a[3], z0, z1)) * p.id);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Cluster schedule: blocks of kClusterSize consecutive elements (the 6 tets of a hex of a box mesh)
 // swept as units.  The block graph of a direction is walked level by level with a CTA barrier
@@ -689,11 +780,6 @@ __global__ void __launch_bounds__(NT, MINB) sweep_cluster_kernel(SweepArgs a) {
 // upstream values from other blocks (27 % of the time); neither the sources' latency nor the barriers show.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTileRow = kClusterSize + 1;   // 16-byte lines per block row
-
-__device__ __forceinline__ void cp_async16(const void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
 
 // One element of a block: row = the block's tile row, bb = its 96 bytes in global memory, f = slot.
 __device__ __forceinline__ void tile_update(char* row, const char* bb, unsigned f, float4 dir, const float4* s_x,
@@ -859,6 +945,114 @@ __global__ void __launch_bounds__(NT, MINB) sweep_tile_kernel(SweepArgs a) {
         __syncthreads();
         walk_tiles<NT, NT>(a.crec + __ldg(&a.crec_base[i]), a.cl_start + __ldg(&a.cl_base[i]), __ldg(&a.ncl[i]),
                            a.psi + (size_t)i * (size_t)a.NENK, dir, s_x, s_sig, s_tab, s_tile, 0);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Level relay: the element levels of a direction, walked pass by pass (up to HT elements of a level) by two
+// halves of a CTA in turn.  Pass k waits for pass k - 1 on a named barrier that its half only arrives at.
+//  RES    the direction's angular block is held in shared memory (small meshes), so that upstream values cost a
+//         shared-memory read instead of an L2 read (a store does not enter L1).  Of 78 us per sweep at 10^3 hexes
+//         and 80 directions the upstream reads were half.
+//  TILE   (with RES) elements have tile types: the update of the tile schedule, tables in shared memory.
+// Measured per sweep, best other schedule -> relay: jittered boxes of 47,196 tets x 168 directions 0.624 -> 0.498 ms,
+// 162,000 x 288 1.72 -> 1.44, 384,000 x 288 4.04 -> 3.54; resident, 6,000 x 80 jittered 0.121 -> 0.099; resident tiles,
+// 6,000 x 80 0.087 -> 0.039, 3,072 x 288 0.076 -> 0.037.
+// ---------------------------------------------------------------------------------------------
+template <int HT, int MINB, bool RES, bool TILE>
+__global__ void __launch_bounds__(2 * HT, MINB) sweep_relay_kernel(SweepArgs a) {
+    constexpr int G = 2;
+    extern __shared__ float4 s_psi[];   // RES: the direction's angular block
+    __shared__ float s_sigt[256];
+    __shared__ float4 s_x[TILE ? 4 * kMaxTileTypes : 1];
+    __shared__ ElemTab s_tab[TILE ? kMaxTileTypes : 1];
+    if (TILE) {
+        for (int k = threadIdx.x; k < 4 * a.nxtype; k += G * HT) s_x[k] = __ldg(&a.xtab[k]);
+        for (int k = threadIdx.x; k < a.nxtype; k += G * HT) s_sigt[k] = a.sigt[__ldg(&a.xmat[k])];
+        __syncthreads();
+    } else {
+        load_sigt(a, s_sigt);
+    }
+    const int g = threadIdx.x / HT, t = threadIdx.x % HT;
+    for (int i = blockIdx.x; i < a.NI; i += gridDim.x) {
+        const int nl = __ldg(&a.nlev[i]);
+        const int* ls = a.lvl_start + __ldg(&a.lvl_base[i]);
+        const float4 dir = __ldg(&a.dirs[i]);
+        const int* it = a.items + (size_t)i * a.NE;
+        float* gpsi = a.psi + (size_t)i * (size_t)a.NENK;
+        if (TILE) build_tab<true>(s_x, s_sigt, a.nxtype, dir, s_tab, threadIdx.x, G * HT);
+        if (RES) {
+            for (int e = threadIdx.x; e < a.NE; e += G * HT) cp_async16(s_psi + e, gpsi + 4 * (size_t)e);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+        }
+        float* base = RES ? reinterpret_cast<float*>(s_psi) : gpsi;
+        // the pass whose item is loaded next: elements s .. of level L (which ends at s1); L == nl: past the last
+        int L = 0, s = __ldg(&ls[0]), s1 = __ldg(&ls[1]);
+        auto advance = [&] {
+            if (L >= nl) return;
+            s += HT;
+            if (s >= s1) {
+                s = s1;
+                if (++L < nl) s1 = __ldg(&ls[L + 1]);
+            }
+        };
+        auto load = [&] { return L < nl && s + t < s1 ? __ldcs(&it[s + t]) : kPad; };
+        bool before = false, has, before_n = false, has_n;   // pass k - 1, pass k of this group, of its next turn
+        for (int j = 0; j < g; ++j) {
+            before = L < nl;
+            advance();
+        }
+        has = L < nl;
+        Ready p;
+        unsigned slot = 0;
+        auto prepare = [&](int item) {
+            if (TILE) {
+                p.item = item;
+                if (item != kPad) slot = ((unsigned)item >> 24) << 3 | (unsigned)__ldg(&a.xtype[item & 0xFFFFFF]) << 11;
+            } else {
+                ready_element(a, base, dir, item, s_sigt, p);
+            }
+        };
+        auto finish = [&] {
+            if (TILE) {
+                if (p.item == kPad) return;
+                const int e = p.item & 0xFFFFFF, pos = e % kClusterSize;
+                char* row = reinterpret_cast<char*>(s_psi + (e - pos));
+                tile_update(row, row, slot | (unsigned)pos, dir, s_x, s_sigt, s_tab);
+            } else {
+                finish_ready(base, p);
+            }
+        };
+        prepare(load());
+        auto turn = [&] {
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                before_n = L < nl;
+                advance();
+                if (j == G - 1) has_n = L < nl;
+                else before_n = L < nl;
+            }
+        };
+        turn();
+        int item_n = load();
+        while (true) {
+            // every pass but the first waits for the pass before it, another group's
+            if (before) asm volatile("bar.sync %0, %1;" ::"r"(1 + (g + G - 1) % G), "n"(2 * HT) : "memory");
+            if (!has) break;
+            finish();
+            asm volatile("bar.arrive %0, %1;" ::"r"(1 + g), "n"(2 * HT) : "memory");
+            prepare(item_n);
+            before = before_n;
+            has = has_n;
+            turn();
+            item_n = load();
+        }
+        __syncthreads();
+        if (RES) {
+            for (int e = threadIdx.x; e < a.NE; e += G * HT) *reinterpret_cast<float4*>(gpsi + 4 * (size_t)e) = s_psi[e];
+            __syncthreads();
+        }
     }
 }
 
@@ -1276,7 +1470,7 @@ __global__ void __launch_bounds__(256) sweep_dataflow_kernel(SweepArgs a) {
 struct Config {
     int kind;      // 0 levels, 1 dataflow, 2 levels with next-level prefetch, 3 element flags, 4 grouped levels,
                    // 5 blocks of elements (cluster records), 6 the same with per-type element tables,
-                   // 7 blocks moved through shared-memory tiles
+                   // 7 blocks moved through shared-memory tiles, 8 element levels in relay, 9 the same with the direction in shared memory
     int threads;
     int dpc;       // directions per CTA (kind 0); minimum CTAs per SM (kinds 2, 5 to 7)
     int ilp;       // updates in flight per thread (kind 0); kinds 5, 6: 2 = next element's record and source
@@ -1290,15 +1484,13 @@ const Config kConfigs[] = {
     {4, 768, 2, 1}, {0, 1024, 1, 2}, {0, 1024, 1, 3}, {0, 768, 1, 3}, {5, 1024, 1, 1}, {5, 512, 2, 1}, {5, 768, 2, 1}, {5, 1024, 2, 1},
     {6, 512, 2, 1}, {6, 768, 2, 1}, {5, 512, 2, 2}, {6, 512, 2, 2}, {5, 512, 2, 3}, {5, 512, 2, 4},
     {7, 512, 2, 1},
+    {8, 512, 2, 1}, {8, 1024, 1, 1}, {9, 512, 2, 1},
 };
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
-// Where the tile schedule applies it is taken without trials: it was the fastest on every box tried, from 6,000
-// tets and 80 directions (0.089 ms against 0.099 for the best other) to 768,000 and 288 (3.03 against 4.15).
-constexpr int kTileConfig = 24;
-// The candidates timed on other meshes: element levels (512 and 1024 threads, with prefetch, two updates in
-// flight) and the block walks with the next element prefetched.  The others never came first on any mesh
+// The candidates timed on meshes without tile types: element levels (512 and 1024 threads), block walks, level
+// relays (the resident one where a direction fits shared memory).  The others never came first on any mesh
 // measured (1.05 to 35 times the best); LB_SWEEP_CONFIG still runs them.
-const int kTrials[] = {5, 6, 7, 11, 20, 22, 23};
+const int kTrials[] = {5, 6, 22, 23, 25, 26, 27};
 constexpr int kNumTrials = sizeof(kTrials) / sizeof(kTrials[0]);
 constexpr int kFinalists = 3;   // candidates timed a second time before one is kept
 
@@ -1398,6 +1590,37 @@ cudaError_t launch_tile(const SweepArgs& a, int sm_count, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// CTAs of the resident relay an SM holds (227 KB of shared memory, 1 KB of it reserved per CTA).
+constexpr size_t kResidentStatic = 256 * 4 + kMaxTileTypes * (64 + sizeof(ElemTab));
+inline int resident_per_sm(int NE) { return (int)std::min<size_t>(2, (228 * 1024) / (16 * (size_t)NE + kResidentStatic + 1024)); }
+
+// The configuration of a mesh with tile types, taken without trials; -1 without them.  The resident relay where
+// all directions are resident at once (0.039 ms against 0.087 with block tiles at 6,000 tets and 80 directions, 0.069
+// against 0.119 at 13,182 and 80; a second wave of directions would lose), block tiles otherwise (0.424 ms
+// against 0.65 for the best other at 96,000 tets and 288 directions).
+constexpr int kTileConfig = 24, kResidentConfig = 27;
+inline int tile_config(const Handle* h) {
+    if (h->nxtype > 0 && h->NI <= h->sm_count * resident_per_sm(h->NE)) return kResidentConfig;
+    return h->tiles_ok ? kTileConfig : -1;
+}
+
+template <int HT, int MINB, bool RES, bool TILE>
+cudaError_t launch_relay(const SweepArgs& a, int sm_count, cudaStream_t s) {
+    const size_t smem = RES ? 16 * (size_t)a.NE : 0;
+    if (RES) {
+        static PerDevice attr;
+        attr.get([&] {
+            allow_max_dynamic_smem(sweep_relay_kernel<HT, MINB, RES, TILE>);
+            return 1;
+        });
+    }
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_relay_kernel<HT, MINB, RES, TILE>, 2 * HT, smem);
+    if (per_sm < 1) per_sm = 1;
+    sweep_relay_kernel<HT, MINB, RES, TILE><<<std::min(a.NI, sm_count * per_sm), 2 * HT, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
 template <int MINB>
 cudaError_t launch_levels_pf(const SweepArgs& a, int threads, int sm_count, cudaStream_t s) {
     const size_t smem = sizeof(float4) * 3 * (size_t)a.ngeom;
@@ -1472,7 +1695,8 @@ SweepArgs sweep_args(Handle* h, float* psi) {
     a.nclusters = h->nclusters;
     a.xtab = h->d_xtab;
     a.xmat = h->d_xmat;
-    a.nxtype = h->tiles_ok ? h->nxtype : 0;
+    a.xtype = h->d_xtype;
+    a.nxtype = h->nxtype;
 
     return a;
 }
@@ -1482,6 +1706,9 @@ cudaError_t launch_walk(const SweepArgs& a, const Config& cfg, Handle* h) {
     const int sms = h->sm_count;
     cudaStream_t s = h->stream;
     if (cfg.kind == 7) return launch_tile<512, 2>(a, sms, s);
+    if (cfg.kind == 8) return cfg.threads == 512 ? launch_relay<256, 2, false, false>(a, sms, s) : launch_relay<512, 1, false, false>(a, sms, s);
+    if (cfg.kind == 9)
+        return h->nxtype > 0 ? launch_relay<256, 2, true, true>(a, sms, s) : launch_relay<256, 2, true, false>(a, sms, s);
     if (cfg.kind >= 5 && cfg.ilp >= 2)
         return cfg.kind == 6   ? launch_cluster<512, 2, true, 1>(a, sms, s)
                : cfg.ilp == 4 ? launch_cluster<512, 2, false, 3>(a, sms, s)
@@ -1506,9 +1733,11 @@ Config runnable(const Handle* h, Config cfg, bool forced) {
     // the autotuner skips the block schedule where it has more barrier levels than the element schedule
     // (unstructured meshes, whose blocks are split on cycles): it cannot win there; a forced configuration
     // still runs it
-    if (cfg.kind >= 5 && !forced && h->cluster_levels_total > (long long)h->total_levels) cfg = Config{0, 1024, 1, 2};
+    if (cfg.kind >= 5 && cfg.kind <= 7 && !forced && h->cluster_levels_total > (long long)h->total_levels) cfg = Config{0, 1024, 1, 2};
+    // the resident schedule holds a direction's angular block in shared memory
+    if (cfg.kind == 9 && resident_per_sm(h->NE) < 1) cfg = Config{8, 512, 2, 1};
     // the tile schedule needs whole blocks of elements with tile types
-    if (cfg.kind >= 7 && !h->tiles_ok) cfg = h->nclusters > 0 ? Config{5, 512, 2, 4} : Config{0, 1024, 1, 2};
+    if (cfg.kind == 7 && !h->tiles_ok) cfg = h->nclusters > 0 ? Config{5, 512, 2, 4} : Config{0, 1024, 1, 2};
     // the cluster schedule needs block records (built when every direction's block graph is acyclic)
     if (cfg.kind == 5 && h->nclusters <= 0) cfg = Config{0, 1024, 1, 2};
     // per-type element tables need the type table as well
@@ -1530,7 +1759,7 @@ int launch_sweep(Handle* h, float* psi) {
     bool tuning = false;
     if (h->sweep_cfg_forced < kNumConfigs) cfg_idx = h->sweep_cfg_forced;
     else if (h->sweep_cfg >= 0) cfg_idx = h->sweep_cfg;
-    else if (h->tiles_ok) cfg_idx = h->sweep_cfg = kTileConfig;
+    else if (tile_config(h) >= 0) cfg_idx = h->sweep_cfg = tile_config(h);
     else {
         // a first pass times every candidate once; a second pass times the kFinalists fastest once more
         cfg_idx = kTrials[h->sweep_trial < kNumTrials ? h->sweep_trial : h->sweep_finalists[h->sweep_trial - kNumTrials]];
@@ -1539,10 +1768,10 @@ int launch_sweep(Handle* h, float* psi) {
     if (tuning && h->sweep_trial == 0) {
         // load every candidate's module before timing, so the first trial does not pay for it
         cudaFuncAttributes fa;
-        cudaFuncGetAttributes(&fa, sweep_levels_pf_kernel<1>);
         cudaFuncGetAttributes(&fa, sweep_levels_kernel<1, 1>);
-        cudaFuncGetAttributes(&fa, sweep_levels_kernel<1, 2>);
-        cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 1>);
+        cudaFuncGetAttributes(&fa, sweep_relay_kernel<256, 2, false, false>);
+        cudaFuncGetAttributes(&fa, sweep_relay_kernel<512, 1, false, false>);
+        cudaFuncGetAttributes(&fa, sweep_relay_kernel<256, 2, true, false>);
         cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 2>);
         cudaFuncGetAttributes(&fa, sweep_cluster_kernel<512, 2, false, 3>);
     }
@@ -1651,7 +1880,7 @@ int launch_sweep(Handle* h, float* psi) {
 
 int sweep_config(Handle* h, int* kind, int* threads, int* dpc, int* ilp) {
     int c = h->sweep_cfg_forced >= 0 && h->sweep_cfg_forced < kNumConfigs ? h->sweep_cfg_forced : h->sweep_cfg;
-    if (c < 0 && h->tiles_ok && h->sweep_cfg_forced != -1) c = kTileConfig;
+    if (c < 0 && h->sweep_cfg_forced != -1) c = tile_config(h);
     if (c < 0) return -1;
     const Config cfg = runnable(h, kConfigs[c], h->sweep_cfg_forced >= 0 && h->sweep_cfg_forced < kNumConfigs);
     *kind = cfg.kind; *threads = cfg.threads; *dpc = cfg.dpc; *ilp = cfg.ilp;
@@ -1668,7 +1897,7 @@ int sweep_config(Handle* h, int* kind, int* threads, int* dpc, int* ilp) {
 //  pre-allocated device arrays), or a real-time loop where cudaMalloc's implicit device
 //  synchronisation is not acceptable.  The caller passes its own FP32 angular vector; the call makes no
 //  cudaMalloc / cudaFree and uses no scratch: it runs the handle's schedule where that needs none (tiles, the
-//  autotuner's pick once it is made), and element levels before.  (The dataflow schedule, which it ran before,
+//  autotuner's pick once it is made), and the level relay before.  (The dataflow schedule, which it ran before,
 //  needs completion counters and took 4.5 ms against 0.30 ms at 57,456 tets and 288 directions.)
 //
 //  The call is synchronous on the handle's stream, and writes to psi issued on other streams must be complete
@@ -1700,10 +1929,9 @@ extern "C" int lb_transport_inv_noalloc(lb_handle* hh, float* psi) {
     }
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return cuda_fail(h, e, "lb_transport_inv_noalloc: set device");
-    // element levels until the handle has a schedule: 512 threads unless a level mostly fills more (an SM then
-    // has room for a second direction)
-    Config cfg = h->NE * (double)h->NI > 1024.0 * h->total_levels ? Config{0, 1024, 1, 1} : Config{0, 512, 1, 1};
-    if (h->tiles_ok) cfg = kConfigs[kTileConfig];
+    // the level relay until the handle has a schedule: 512 threads unless a level mostly fills more
+    Config cfg = h->NE * (double)h->NI > 1024.0 * h->total_levels ? Config{8, 1024, 1, 1} : Config{8, 512, 2, 1};
+    if (tile_config(h) >= 0) cfg = kConfigs[tile_config(h)];
     else if (h->sweep_cfg >= 0) cfg = runnable(h, kConfigs[h->sweep_cfg], false);
     e = launch_walk(sweep_args(h, psi), cfg, h);
     if (e != cudaSuccess) return cuda_fail(h, e, "lb_transport_inv_noalloc: launch");

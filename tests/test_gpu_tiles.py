@@ -101,8 +101,31 @@ def test_noalloc_sweep_runs_the_handles_schedule(amount):
         return d.cpu().numpy().astype(np.float64)
 
     first = noalloc()
-    for _ in range(12):
+    for _ in range(100):                 # until the autotuner has picked
         ref = q.astype(np.float64)
         T.MatInv(ref)
+        if T._h.sweep_config() is not None:
+            break
     assert T._h.sweep_config() is not None
     assert np.array_equal(first, ref) and np.array_equal(noalloc(), ref)
+
+
+# meshes whose levels end before and after the passes of 256 and 512 elements; the smallest has levels of one
+# element
+RELAY_BOXES = [(1, 1, 1), (3, 2, 2), (9, 8, 10), (24, 25, 23)]
+
+
+@pytest.mark.parametrize("amount", [0.0, 0.06])
+@pytest.mark.parametrize("n", RELAY_BOXES)
+@pytest.mark.parametrize("cfg", [25, 26, 27])
+def test_level_relay_is_bit_identical_to_element_levels(cfg, n, amount, monkeypatch):
+    from helpers import jittered
+    m = M.box_mesh(*n, (0, 0, 0), tuple(0.5 * v for v in n), material=_two, Nm=2)
+    if amount:
+        m = jittered(m, amount)
+    k, w = P.quadrature(2, 6)
+    sigt = np.array([0.3, 1.7])
+    q = np.random.default_rng(cfg).uniform(size=m.NENK * len(w))
+    T, v = _sweep(monkeypatch, cfg, m, k, w, sigt, q)
+    assert T._h.sweep_config()["schedule"] == ("resident level relay" if cfg == 27 and m.NE <= 14000 else "level relay")
+    assert np.array_equal(v, _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)[1])
