@@ -40,10 +40,15 @@ constexpr int FS = 20;                       // stored feature stride (floats)
 constexpr int RS1 = 40, RS2 = 72, RS3 = 72, RSX = 40;
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
-// training: FP32 weights in shared memory with odd row strides (conflict-free row and column walks)
-constexpr int TS1 = 19, TS2 = 65, TS3 = 65;
-constexpr int T_W1 = 0, T_B1 = T_W1 + NH * TS1, T_W2 = T_B1 + NH, T_B2 = T_W2 + NH * TS2, T_W3 = T_B2 + NH,
-              T_B3 = T_W3 + NOUT * TS3, T_N = T_B3 + NOUT;
+// training: samples of a block's tile, and its shared-memory arrays (FP32): the weights, W1 and W2 and W3 input-major
+// for the forward pass ([input][unit], four units per 16-byte load), W2 and W3 unit-major as well for the backward
+// pass; sample rows of the activations and of their gradients (rows of 68 floats: 16-byte aligned, rows of
+// different samples in different banks)
+constexpr int TS = 32;
+constexpr int RA = 68;                       // row pitch of [TS][64] arrays and of the 64-wide weight rows
+constexpr int T_W1T = 0, T_W2T = T_W1T + FS * RA, T_W2 = T_W2T + NH * RA, T_W3T = T_W2 + NH * RA, T_W3 = T_W3T + NH * NOUT,
+              T_B = T_W3 + NOUT * RA, T_X = T_B + NH + NH + NOUT, T_H1 = T_X + TS * FS, T_H2 = T_H1 + TS * RA,
+              T_D2 = T_H2 + TS * RA, T_D3 = T_D2 + TS * RA, T_N = T_D3 + TS * FS;
 }  // namespace lp
 
 struct MlpState {
@@ -366,128 +371,281 @@ __global__ void lp_sample_kernel(const double* __restrict__ r, const double* __r
 }
 
 // Loss and gradient of L = 1/(2n) sum_samples w sum_i (o_i - t_i)^2 over a batch (w = feature
-// column 19), one warp per sample.
+// column 19).
 // The forward pass rounds weights, inputs and hidden activations to BF16 exactly like the
 // inference kernel; the backward pass treats the rounding as identity (straight-through) and
-// runs in FP32.  Each block accumulates its gradient in shared memory and writes one partial.
-// Samples: direct (s-th sample of the batch is sample s) or drawn by hash(seed, s) % nsamples.
-__global__ void __launch_bounds__(lp::kThreads) lp_grad_kernel(const float* __restrict__ w, const float* __restrict__ X,
-                                                              const float* __restrict__ T, long long nsamples, int batch,
-                                                              int direct, unsigned long long seed, float inv_n,
-                                                              float* __restrict__ part, double* __restrict__ lossp) {
+// runs in FP32.  Samples: direct (s-th sample of the batch is sample s) or drawn by hash(seed, s) % nsamples.
+//
+// A block takes tiles of TS samples.  Every product of the tile (forward, backward and the weight gradients) is a small
+// matrix product from shared memory with a register tile per thread (2 samples x 4 units; 4 x 4 weights), and the
+// weight gradients stay in registers over the block's tiles, so a tile costs about 2,200 FMAs per thread and no
+// atomics.  (One warp per sample with shared-memory atomics on every weight, some 400 per lane and sample: 16,384
+// samples took 0.75 ms against 0.05 ms.)  Bound by shared-memory loads and latency, two blocks per SM.
+// Each block writes one partial; sums run in a fixed order (deterministic).
+__global__ void __launch_bounds__(lp::kThreads, 2) lp_grad_kernel(const float* __restrict__ w, const float* __restrict__ X,
+                                                                 const float* __restrict__ T, long long nsamples, int batch,
+                                                                 int direct, unsigned long long seed, float inv_n,
+                                                                 float* __restrict__ part, double* __restrict__ lossp) {
     using namespace lp;
-    extern __shared__ __align__(16) float smf[];
-    float* sw = smf;            // [T_N] BF16-rounded weights (FP32 biases), padded rows
-    float* sg = smf + T_N;      // [NPARAM] gradient accumulator (unpadded parameter layout)
+    extern __shared__ __align__(16) float sm_[];
+    __shared__ long long sidx[TS];
     __shared__ double wl[kWarps];
-    for (int i = threadIdx.x; i < NH * NIN; i += blockDim.x) sw[T_W1 + (i / NIN) * TS1 + i % NIN] = bf16r(w[OFF_W1 + i]);
-    for (int i = threadIdx.x; i < NH * NH; i += blockDim.x) sw[T_W2 + (i / NH) * TS2 + i % NH] = bf16r(w[OFF_W2 + i]);
-    for (int i = threadIdx.x; i < NOUT * NH; i += blockDim.x) sw[T_W3 + (i / NH) * TS3 + i % NH] = bf16r(w[OFF_W3 + i]);
-    for (int i = threadIdx.x; i < NH; i += blockDim.x) {
-        sw[T_B1 + i] = w[OFF_B1 + i];
-        sw[T_B2 + i] = w[OFF_B2 + i];
-    }
-    for (int i = threadIdx.x; i < NOUT; i += blockDim.x) sw[T_B3 + i] = w[OFF_B3 + i];
-    for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) sg[i] = 0.f;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < FS * RA; i += kThreads) sm_[T_W1T + i] = 0.f;
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned FULL = 0xffffffffu;
-    float loss = 0.f;
-    for (int sidx = blockIdx.x * kWarps + warp; sidx < batch; sidx += gridDim.x * kWarps) {
-        const long long n = direct ? (long long)sidx
-                                   : (long long)(mix64(seed ^ mix64((unsigned long long)sidx)) % (unsigned long long)nsamples);
-        const float xk = lane < NIN ? bf16r(X[n * FS + lane]) : 0.f;
-        // layer 1 (lane owns hidden units lane, lane+32)
-        float z1a = sw[T_B1 + lane], z1b = sw[T_B1 + lane + 32];
+    for (int i = tid; i < NH * NIN; i += kThreads) sm_[T_W1T + (i % NIN) * RA + i / NIN] = bf16r(w[OFF_W1 + i]);
+    for (int i = tid; i < NH * NH; i += kThreads) {
+        const float v = bf16r(w[OFF_W2 + i]);
+        sm_[T_W2 + (i / NH) * RA + i % NH] = v;
+        sm_[T_W2T + (i % NH) * RA + i / NH] = v;
+    }
+    for (int i = tid; i < NOUT * NH; i += kThreads) {
+        const float v = bf16r(w[OFF_W3 + i]);
+        sm_[T_W3 + (i / NH) * RA + i % NH] = v;
+        sm_[T_W3T + (i % NH) * NOUT + i / NH] = v;
+    }
+    for (int i = tid; i < NH; i += kThreads) {
+        sm_[T_B + i] = w[OFF_B1 + i];
+        sm_[T_B + NH + i] = w[OFF_B2 + i];
+    }
+    for (int i = tid; i < NOUT; i += kThreads) sm_[T_B + 2 * NH + i] = w[OFF_B3 + i];
+    // register tiles: samples s0, s0 + 1 and units u0..u0+3 of the [TS][64] products; weights (r0.., u0..) of dW2
+    const int u0 = 4 * (tid & 15), s0 = 2 * (tid >> 4), r0 = 4 * (tid >> 4);
+    const int l3 = tid & 15, l3s = tid >> 4;              // layer 3: output, samples l3s and l3s + 16
+    const int w1u = tid >> 2, w1k = 5 * (tid & 3);        // dW1: unit, 5 inputs (the 20th is the loss weight: unused)
+    float g2w[4][4] = {}, g1w[5] = {}, g3w[4] = {}, gb = 0.f, loss = 0.f;
+    const int ntiles = (batch + TS - 1) / TS;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        __syncthreads();   // the previous tile's arrays are read; the first time, the weights are written
+        if (tid < TS) {
+            const int q = tile * TS + tid;
+            sidx[tid] = q >= batch ? -1
+                        : direct  ? (long long)q
+                                  : (long long)(mix64(seed ^ mix64((unsigned long long)q)) % (unsigned long long)nsamples);
+        }
+        __syncthreads();
+        for (int i = tid; i < TS * FS; i += kThreads) {
+            const int q = i / FS, k = i % FS;
+            const float x = sidx[q] < 0 ? 0.f : __ldg(&X[sidx[q] * FS + k]);
+            sm_[T_X + i] = k < NIN ? bf16r(x) : x;   // column NIN: the loss weight (0 past the batch)
+        }
+        __syncthreads();
+        float z1[2][4], z2[2][4];
+        {   // layer 1
+            const float4 bias = *reinterpret_cast<const float4*>(&sm_[T_B + u0]);
 #pragma unroll
-        for (int k = 0; k < NIN; ++k) {
-            const float xb = __shfl_sync(FULL, xk, k);
-            z1a = fmaf(sw[T_W1 + lane * TS1 + k], xb, z1a);
-            z1b = fmaf(sw[T_W1 + (lane + 32) * TS1 + k], xb, z1b);
+            for (int q = 0; q < 2; ++q) { z1[q][0] = bias.x; z1[q][1] = bias.y; z1[q][2] = bias.z; z1[q][3] = bias.w; }
+#pragma unroll
+            for (int k = 0; k < NIN; ++k) {
+                const float4 v = *reinterpret_cast<const float4*>(&sm_[T_W1T + k * RA + u0]);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float x = sm_[T_X + (s0 + q) * FS + k];
+                    z1[q][0] = fmaf(v.x, x, z1[q][0]);
+                    z1[q][1] = fmaf(v.y, x, z1[q][1]);
+                    z1[q][2] = fmaf(v.z, x, z1[q][2]);
+                    z1[q][3] = fmaf(v.w, x, z1[q][3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4*>(&sm_[T_H1 + (s0 + q) * RA + u0]) =
+                    make_float4(bf16r(fmaxf(z1[q][0], 0.f)), bf16r(fmaxf(z1[q][1], 0.f)), bf16r(fmaxf(z1[q][2], 0.f)),
+                                bf16r(fmaxf(z1[q][3], 0.f)));
         }
-        const float h1a = bf16r(fmaxf(z1a, 0.f)), h1b = bf16r(fmaxf(z1b, 0.f));
-        // layer 2
-        float z2a = sw[T_B2 + lane], z2b = sw[T_B2 + lane + 32];
-#pragma unroll 8
-        for (int j = 0; j < NH; ++j) {
-            const float hb = __shfl_sync(FULL, j < 32 ? h1a : h1b, j & 31);
-            z2a = fmaf(sw[T_W2 + lane * TS2 + j], hb, z2a);
-            z2b = fmaf(sw[T_W2 + (lane + 32) * TS2 + j], hb, z2b);
-        }
-        const float h2a = bf16r(fmaxf(z2a, 0.f)), h2b = bf16r(fmaxf(z2b, 0.f));
-        // layer 3: lane -> output lane&15 over the half lane>>4 of the hidden units
-        const int oi = lane & 15, jh = lane >> 4;
-        float o = 0.f;
-#pragma unroll 8
-        for (int jj = 0; jj < 32; ++jj) {
-            const float ha = __shfl_sync(FULL, h2a, jj), hb = __shfl_sync(FULL, h2b, jj);
-            o = fmaf(sw[T_W3 + oi * TS3 + jh * 32 + jj], jh ? hb : ha, o);
-        }
-        o += __shfl_xor_sync(FULL, o, 16);
-        o += sw[T_B3 + oi];
-        const float wt = X[n * FS + NIN];
-        const float diff = o - T[n * NOUT + oi];
-        if (lane < 16) loss = fmaf(wt * diff, diff, loss);
-        const float d3 = wt * diff * inv_n;   // dL/do_i (lanes i and i+16 hold the same value)
-        // output layer gradients
-        if (lane < 16) atomicAdd(&sg[OFF_B3 + lane], d3);
-        float g2a = 0.f, g2b = 0.f;
+        __syncthreads();
+        {   // layer 2
+            const float4 bias = *reinterpret_cast<const float4*>(&sm_[T_B + NH + u0]);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) { z2[q][0] = bias.x; z2[q][1] = bias.y; z2[q][2] = bias.z; z2[q][3] = bias.w; }
 #pragma unroll 4
-        for (int i = 0; i < NOUT; ++i) {
-            const float di = __shfl_sync(FULL, d3, i);
-            atomicAdd(&sg[OFF_W3 + i * NH + lane], di * h2a);
-            atomicAdd(&sg[OFF_W3 + i * NH + lane + 32], di * h2b);
-            g2a = fmaf(sw[T_W3 + i * TS3 + lane], di, g2a);
-            g2b = fmaf(sw[T_W3 + i * TS3 + lane + 32], di, g2b);
+            for (int k = 0; k < NH; k += 4) {
+                float4 h[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) h[q] = *reinterpret_cast<const float4*>(&sm_[T_H1 + (s0 + q) * RA + k]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(&sm_[T_W2T + (k + j) * RA + u0]);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float x = j == 0 ? h[q].x : j == 1 ? h[q].y : j == 2 ? h[q].z : h[q].w;
+                        z2[q][0] = fmaf(v.x, x, z2[q][0]);
+                        z2[q][1] = fmaf(v.y, x, z2[q][1]);
+                        z2[q][2] = fmaf(v.z, x, z2[q][2]);
+                        z2[q][3] = fmaf(v.w, x, z2[q][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4*>(&sm_[T_H2 + (s0 + q) * RA + u0]) =
+                    make_float4(bf16r(fmaxf(z2[q][0], 0.f)), bf16r(fmaxf(z2[q][1], 0.f)), bf16r(fmaxf(z2[q][2], 0.f)),
+                                bf16r(fmaxf(z2[q][3], 0.f)));
         }
-        const float d2a = z2a > 0.f ? g2a : 0.f, d2b = z2b > 0.f ? g2b : 0.f;
-        atomicAdd(&sg[OFF_B2 + lane], d2a);
-        atomicAdd(&sg[OFF_B2 + lane + 32], d2b);
-        float g1a = 0.f, g1b = 0.f;
-        for (int i = 0; i < NH; ++i) {
-            const float di = __shfl_sync(FULL, i < 32 ? d2a : d2b, i & 31);
-            if (di != 0.f) {
-                atomicAdd(&sg[OFF_W2 + i * NH + lane], di * h1a);
-                atomicAdd(&sg[OFF_W2 + i * NH + lane + 32], di * h1b);
-                g1a = fmaf(sw[T_W2 + i * TS2 + lane], di, g1a);
-                g1b = fmaf(sw[T_W2 + i * TS2 + lane + 32], di, g1b);
+        __syncthreads();
+        // layer 3 (two half sums over the hidden units), loss and its gradient at the outputs
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int sr = l3s + 16 * q;
+            float o0 = 0.f, o1 = 0.f;
+#pragma unroll 8
+            for (int k = 0; k < NH / 2; ++k) {
+                o0 = fmaf(sm_[T_W3T + k * NOUT + l3], sm_[T_H2 + sr * RA + k], o0);
+                o1 = fmaf(sm_[T_W3T + (k + NH / 2) * NOUT + l3], sm_[T_H2 + sr * RA + k + NH / 2], o1);
+            }
+            const float o = (o0 + o1) + sm_[T_B + 2 * NH + l3];
+            const float wt = sm_[T_X + sr * FS + NIN];
+            const float diff = sidx[sr] < 0 ? 0.f : o - __ldg(&T[sidx[sr] * NOUT + l3]);
+            loss = fmaf(wt * diff, diff, loss);
+            sm_[T_D3 + sr * FS + l3] = wt * diff * inv_n;
+        }
+        __syncthreads();
+        float d2[2][4];
+        {   // gradient at layer 2, and dW3 (output r0 / 4, units u0..)
+            float g[2][4] = {};
+#pragma unroll 4
+            for (int i = 0; i < NOUT; ++i) {
+                const float4 v = *reinterpret_cast<const float4*>(&sm_[T_W3 + i * RA + u0]);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float d = sm_[T_D3 + (s0 + q) * FS + i];
+                    g[q][0] = fmaf(v.x, d, g[q][0]);
+                    g[q][1] = fmaf(v.y, d, g[q][1]);
+                    g[q][2] = fmaf(v.z, d, g[q][2]);
+                    g[q][3] = fmaf(v.w, d, g[q][3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d2[q][j] = z2[q][j] > 0.f ? g[q][j] : 0.f;
+                *reinterpret_cast<float4*>(&sm_[T_D2 + (s0 + q) * RA + u0]) = make_float4(d2[q][0], d2[q][1], d2[q][2], d2[q][3]);
+            }
+#pragma unroll 8
+            for (int q = 0; q < TS; ++q) {
+                const float d = sm_[T_D3 + q * FS + (tid >> 4)];
+                const float4 h = *reinterpret_cast<const float4*>(&sm_[T_H2 + q * RA + u0]);
+                g3w[0] = fmaf(d, h.x, g3w[0]);
+                g3w[1] = fmaf(d, h.y, g3w[1]);
+                g3w[2] = fmaf(d, h.z, g3w[2]);
+                g3w[3] = fmaf(d, h.w, g3w[3]);
             }
         }
-        const float d1a = z1a > 0.f ? g1a : 0.f, d1b = z1b > 0.f ? g1b : 0.f;
-        atomicAdd(&sg[OFF_B1 + lane], d1a);
-        atomicAdd(&sg[OFF_B1 + lane + 32], d1b);
-        for (int i = 0; i < NH; ++i) {
-            const float di = __shfl_sync(FULL, i < 32 ? d1a : d1b, i & 31);
-            if (di != 0.f && lane < NIN) atomicAdd(&sg[OFF_W1 + i * NIN + lane], di * xk);
+        __syncthreads();
+        {   // gradient at layer 1 (into the array of h2, which is read), and dW2
+            float g[2][4] = {};
+#pragma unroll 4
+            for (int i = 0; i < NH; i += 4) {
+                float4 d[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) d[q] = *reinterpret_cast<const float4*>(&sm_[T_D2 + (s0 + q) * RA + i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(&sm_[T_W2 + (i + j) * RA + u0]);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float x = j == 0 ? d[q].x : j == 1 ? d[q].y : j == 2 ? d[q].z : d[q].w;
+                        g[q][0] = fmaf(v.x, x, g[q][0]);
+                        g[q][1] = fmaf(v.y, x, g[q][1]);
+                        g[q][2] = fmaf(v.z, x, g[q][2]);
+                        g[q][3] = fmaf(v.w, x, g[q][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4*>(&sm_[T_H2 + (s0 + q) * RA + u0]) =
+                    make_float4(z1[q][0] > 0.f ? g[q][0] : 0.f, z1[q][1] > 0.f ? g[q][1] : 0.f,
+                                z1[q][2] > 0.f ? g[q][2] : 0.f, z1[q][3] > 0.f ? g[q][3] : 0.f);
+#pragma unroll 4
+            for (int q = 0; q < TS; ++q) {
+                const float4 d = *reinterpret_cast<const float4*>(&sm_[T_D2 + q * RA + r0]);
+                const float4 h = *reinterpret_cast<const float4*>(&sm_[T_H1 + q * RA + u0]);
+                const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    g2w[j][0] = fmaf(dd[j], h.x, g2w[j][0]);
+                    g2w[j][1] = fmaf(dd[j], h.y, g2w[j][1]);
+                    g2w[j][2] = fmaf(dd[j], h.z, g2w[j][2]);
+                    g2w[j][3] = fmaf(dd[j], h.w, g2w[j][3]);
+                }
+            }
+        }
+        __syncthreads();
+        // dW1, and the biases: threads 0..63 b1, 64..127 b2, 128..143 b3
+#pragma unroll 4
+        for (int q = 0; q < TS; ++q) {
+            const float d = sm_[T_H2 + q * RA + w1u];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) g1w[k] = fmaf(d, sm_[T_X + q * FS + w1k + k], g1w[k]);
+        }
+        if (tid < 2 * NH + NOUT) {
+            const float* col = tid < NH ? &sm_[T_H2 + tid] : tid < 2 * NH ? &sm_[T_D2 + tid - NH] : &sm_[T_D3 + tid - 2 * NH];
+            const int ld = tid < 2 * NH ? RA : FS;
+#pragma unroll 8
+            for (int q = 0; q < TS; ++q) gb += col[q * ld];
         }
     }
-    // block loss
-    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(FULL, loss, o);
-    if (lane == 0) wl[warp] = (double)loss;
+    // block loss and partial gradient
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((tid & 31) == 0) wl[tid >> 5] = (double)loss;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < kWarps; ++k) s += wl[k];
-        lossp[blockIdx.x] = 0.5 * s * (double)inv_n;
+    if (tid == 0) {
+        double t = 0.0;
+        for (int k = 0; k < kWarps; ++k) t += wl[k];
+        lossp[blockIdx.x] = 0.5 * t * (double)inv_n;
     }
-    for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) part[(size_t)blockIdx.x * NPARAM + i] = sg[i];
+    float* out = part + (size_t)blockIdx.x * NPARAM;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[OFF_W2 + (r0 + j) * NH + u0 + k] = g2w[j][k];
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        if (w1k + k < NIN) out[OFF_W1 + w1u * NIN + w1k + k] = g1w[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[OFF_W3 + (tid >> 4) * NH + u0 + k] = g3w[k];
+    if (tid < NH) out[OFF_B1 + tid] = gb;
+    else if (tid < 2 * NH) out[OFF_B2 + tid - NH] = gb;
+    else if (tid < 2 * NH + NOUT) out[OFF_B3 + tid - 2 * NH] = gb;
 }
 
-// Sum of the block partials in block order (deterministic) and one Adam step; block 0 thread 0
-// also records the batch loss.
-__global__ void lp_adam_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                               const float* __restrict__ part, const double* __restrict__ lossp, int nparts, float lr,
-                               float beta1, float beta2, float eps, float bc1, float bc2, double* __restrict__ losshist,
-                               int step) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// Sum over the blocks' partials of parameter blockIdx.x * 32 + (threadIdx.x & 31): eight slices of consecutive
+// blocks, each in block order, then the slices in order (deterministic).  The sum is in the threads of slice 0.
+constexpr int kSumSlices = 8;
+__device__ __forceinline__ float sum_partials(const float* __restrict__ part, int nparts, int p) {
+    __shared__ float sl[kSumSlices][32];
+    const int slice = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = (nparts + kSumSlices - 1) / kSumSlices;
+    float g = 0.f;
+    if (p < NPARAM) {
+        const int b1 = min(nparts, (slice + 1) * per);
+#pragma unroll 4
+        for (int b = slice * per; b < b1; ++b) g += part[(size_t)b * NPARAM + p];
+    }
+    sl[slice][lane] = g;
+    __syncthreads();
+    float s = 0.f;
+    if (slice == 0)
+        for (int k = 0; k < kSumSlices; ++k) s += sl[k][lane];
+    return s;
+}
+
+// Sum of the block partials and one Adam step; block 0 thread 0 also records the batch loss.
+__global__ void __launch_bounds__(32 * kSumSlices) lp_adam_kernel(float* __restrict__ w, float* __restrict__ m,
+                                                                 float* __restrict__ v, const float* __restrict__ part,
+                                                                 const double* __restrict__ lossp, int nparts, float lr,
+                                                                 float beta1, float beta2, float eps, float bc1, float bc2,
+                                                                 double* __restrict__ losshist, int step) {
+    const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float g = sum_partials(part, nparts, p);
+    if (threadIdx.x >= 32) return;
     if (p == 0 && losshist) {
         double s = 0.0;
         for (int b = 0; b < nparts; ++b) s += lossp[b];
         losshist[step] = s;
     }
     if (p >= NPARAM) return;
-    float g = 0.f;
-    for (int b = 0; b < nparts; ++b) g += part[(size_t)b * NPARAM + p];
     const float mm = beta1 * m[p] + (1.f - beta1) * g;
     const float vv = beta2 * v[p] + (1.f - beta2) * g * g;
     m[p] = mm;
@@ -496,15 +654,14 @@ __global__ void lp_adam_kernel(float* __restrict__ w, float* __restrict__ m, flo
 }
 
 // Gradient sum without an update (gradient checks).
-__global__ void lp_gradsum_kernel(const float* __restrict__ part, int nparts, float* __restrict__ g) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NPARAM) return;
-    float s = 0.f;
-    for (int b = 0; b < nparts; ++b) s += part[(size_t)b * NPARAM + p];
-    g[p] = s;
+__global__ void __launch_bounds__(32 * kSumSlices) lp_gradsum_kernel(const float* __restrict__ part, int nparts,
+                                                                    float* __restrict__ g) {
+    const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float s = sum_partials(part, nparts, p);
+    if (threadIdx.x < 32 && p < NPARAM) g[p] = s;
 }
 
-constexpr size_t kGradSmem = sizeof(float) * (lp::T_N + lp::NPARAM);
+constexpr size_t kGradSmem = sizeof(float) * lp::T_N;
 
 }  // namespace
 
@@ -662,10 +819,9 @@ static int ensure_grad_bufs(Handle* h, MlpState* s, int parts, int hist) {
     return LB_OK;
 }
 
-// About 8 samples per warp: enough work per block to amortise the weight staging, few enough
-// partials for the deterministic block-order reduction.
+// One block per tile of samples, up to two per SM (each block stages the weights once and writes one partial).
 static int grad_blocks(Handle* h, int batch) {
-    return std::max(1, std::min((batch + 8 * lp::kWarps - 1) / (8 * lp::kWarps), h->sm_count));
+    return std::max(1, std::min((batch + lp::TS - 1) / lp::TS, 2 * h->sm_count));
 }
 
 }  // namespace lb
@@ -828,7 +984,7 @@ int lb_lp_loss_grad(lb_handle* h, int n, const float* x, const float* t, const f
     if (e == cudaSuccess) {
         lp_grad_kernel<<<parts, lp::kThreads, kGradSmem, h->stream>>>(s->d_w, dx, dt, n, n, 1, 0ull, 1.f / n, s->d_part,
                                                                        s->d_lossp);
-        lp_gradsum_kernel<<<(lp::NPARAM + 255) / 256, 256, 0, h->stream>>>(s->d_part, parts, dg);
+        lp_gradsum_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(s->d_part, parts, dg);
         e = cudaGetLastError();
     }
     std::vector<double> lp_(parts);
@@ -896,7 +1052,7 @@ int lb_lp_train(lb_handle* h, int steps, int batch, double lr, unsigned long lon
         lp_grad_kernel<<<parts, lp::kThreads, kGradSmem, h->stream>>>(
             s->d_w, s->d_X, s->d_T, s->nsamples, batch, 0, seed + 0x100000001B3ull * (unsigned long long)it,
             1.f / batch, s->d_part, s->d_lossp);
-        lp_adam_kernel<<<(lp::NPARAM + 255) / 256, 256, 0, h->stream>>>(s->d_w, s->d_m, s->d_v, s->d_part, s->d_lossp,
+        lp_adam_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(s->d_w, s->d_m, s->d_v, s->d_part, s->d_lossp,
                                                                          parts, lr_t, b1, b2, eps, bc1, bc2,
                                                                          s->d_losshist, it);
     }

@@ -179,3 +179,25 @@ def test_learned_path_is_gated_per_group_and_never_slower_in_applications():
             # answer shifted this group's source in the last digits)
             assert it_gated[g] <= it_plain[g] + (1 if enabled[:g].any() else 0), g
     assert it_gated.sum() <= it_plain.sum() + int(np.sum(enabled * plain_v))
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 300, 9500])
+def test_gradient_at_the_edges_of_its_sample_tiles(n):
+    """Loss and gradient for batches around the kernel's tiles of 32 samples, and for more tiles than it has
+    blocks, against the FP64 restatement; weights with a sample of weight zero.  Tolerance: BF16 rounding
+    points are the same on both sides, FP32 sums of up to 9,500 terms leave less than 2e-3 as in the other
+    gradient check."""
+    rng = np.random.default_rng(n)
+    w = _random_weights(5)
+    op = TransportOp()
+    op.lp_set_weights(w)
+    x = rng.normal(size=(n, 19)).astype(np.float32)
+    t = (0.3 * rng.normal(size=(n, 16))).astype(np.float32)
+    wt = rng.uniform(0.1, 1.0, size=n).astype(np.float32)
+    wt[n // 2] = 0.0 if n > 1 else 1.0
+    loss, g = op.lp_loss_grad(x, t, wt)
+    lref, gref = R.loss_grad(w, x, t, wt)
+    assert abs(loss - lref) < 1e-4 * abs(lref)
+    assert rel_l2(g, gref) < 2e-3
+    again = op.lp_loss_grad(x, t, wt)
+    assert again[0] == loss and np.array_equal(again[1], g)     # fixed summation order
