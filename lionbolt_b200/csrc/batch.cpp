@@ -61,6 +61,14 @@ int bcuda(lb_batch* b, cudaError_t e, const char* what) {
 
 cudaStream_t bstream(lb_batch* b) { return b->aux->stream; }
 
+// Lends the batch's large transfer buffers to a problem's handle, so that a batch has one pair and not one per
+// problem.  The problem's copies must be done (or its stream be the batch's) when the loan ends.
+struct PipeLoan {
+    Handle *a, *h;
+    PipeLoan(Handle* a_, Handle* h_) : a(a_), h(h_) { std::swap(a->pipe_large, h->pipe_large); }
+    ~PipeLoan() { std::swap(a->pipe_large, h->pipe_large); }
+};
+
 void free_graphs(lb_batch* b) {
     for (auto& g : b->gx)
         if (g) {
@@ -590,14 +598,17 @@ int lb_batch_add_problem(lb_batch* b, int NE, int NN, const double* rg, const in
     if (rc) return bfail(b, rc, "lb_batch_add_problem: cannot create a handle");
     if (!rc) rc = lb_set_mesh(h, NE, NN, rg, node, neighbors, mat, Nm);
     if (!rc) rc = lb_set_quadrature(h, NI, k, w);
-    if (!rc) rc = lb_mg_set_problem(h, G, Ls, sigt, sigs, dd, unc, beam_dir);
+    if (!rc) {
+        PipeLoan loan(b->aux, h);
+        rc = lb_mg_set_problem(h, G, Ls, sigt, sigs, dd, unc, beam_dir);
+        cudaStreamSynchronize(h->stream);
+    }
     if (rc) {
         const int p = (int)b->probs.size();
         prop_error(b, h, rc, p);
         lb_destroy(h);
         return rc;
     }
-    cudaStreamSynchronize(h->stream);
     b->own_streams.push_back(h->stream);
     h->stream = b->aux->stream;   // every launch of the batch goes to one stream (and its graphs)
     h->timing = false;
@@ -680,6 +691,7 @@ int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int*
 
 int lb_batch_get_results(lb_batch* b, int id, double* flux, double* dose) {
     if (!b || id < 0 || id >= (int)b->probs.size()) return LB_ERR_ARG;
+    PipeLoan loan(b->aux, b->probs[id]);
     int rc = lb_mg_get_results(b->probs[id], flux, dose);
     return rc ? prop_error(b, b->probs[id], rc, id) : LB_OK;
 }

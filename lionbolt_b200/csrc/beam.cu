@@ -34,7 +34,7 @@ struct BeamArgs {
     const double4* __restrict__ plane;  // [NE][4] outward unit normal and offset n . x of each face
     const double* __restrict__ attn;    // [Nm] total cross sections of the beam's group
     double* __restrict__ unc;           // [NE][4] DG coefficients of the uncollided fluence
-    int* __restrict__ stuck;            // rays whose walk hit the step limit
+    int* stuck;                         // set when a ray's walk hit the step limit
     double ox, oy, oz;                  // beam origin
     double ax, ay, az;                  // beam axis (unit)
     double e1x, e1y, e1z, e2x, e2y, e2z;   // unit vectors spanning the beam plane
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) beam_uncollided_kernel(BeamArgs a) {
                     z = fma(seg, dz, z);
                     cur = __ldg(&a.nbr[4 * cur + fexit]);
                     if (++steps > a.max_steps) {
-                        atomicAdd(a.stuck, 1);
+                        *a.stuck = 1;
                         tau = 0.0;
                         break;
                     }
@@ -173,18 +173,16 @@ extern "C" int lb_beam_uncollided(lb_handle* hh, const double* origin, const dou
     int rc = beam_prepare(h);
     if (rc) return rc;
     const size_t NENK = (size_t)h->NENK;
-    double* d_attn = nullptr;
-    int* d_stuck = nullptr;
-    cudaError_t e = cudaMalloc(&d_attn, sizeof(double) * h->Nm);
-    if (e == cudaSuccess) e = cudaMalloc(&d_stuck, sizeof(int));
-    if (e == cudaSuccess && !h->d_unc) e = cudaMalloc(&h->d_unc, sizeof(double) * NENK);
+    // scratch: the reduction buffers (idle between calls); the stuck flag is in pinned host memory, written by the
+    // device only for a ray that is stuck
+    double* d_attn = h->d_red;
+    int* stuck = reinterpret_cast<int*>(h->h_red);
+    cudaError_t e = cudaSuccess;
+    if (!h->d_unc) e = cudaMalloc(&h->d_unc, sizeof(double) * NENK);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);   // nothing of an earlier call still uses them
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_attn, attn, sizeof(double) * h->Nm, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_stuck, 0, sizeof(int), h->stream);
-    if (e != cudaSuccess) {
-        cudaFree(d_attn);
-        cudaFree(d_stuck);
-        return cuda_fail(h, e, "lb_beam_uncollided: buffers");
-    }
+    if (e != cudaSuccess) return cuda_fail(h, e, "lb_beam_uncollided: buffers");
+    *stuck = 0;
     BeamArgs a{};
     a.xyz = h->d_beam_xyz;
     a.node = h->d_beam_node;
@@ -193,7 +191,7 @@ extern "C" int lb_beam_uncollided(lb_handle* hh, const double* origin, const dou
     a.plane = h->d_beam_plane;
     a.attn = d_attn;
     a.unc = h->d_unc;
-    a.stuck = d_stuck;
+    a.stuck = stuck;
     a.ox = origin[0]; a.oy = origin[1]; a.oz = origin[2];
     a.ax = axis[0]; a.ay = axis[1]; a.az = axis[2];
     a.e1x = e1[0]; a.e1y = e1[1]; a.e1z = e1[2];
@@ -208,13 +206,10 @@ extern "C" int lb_beam_uncollided(lb_handle* hh, const double* origin, const dou
     beam_uncollided_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, h->stream>>>(a);
     timer_end(h, t);
     e = cudaGetLastError();
-    int stuck = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&stuck, d_stuck, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess && unc) e = cudaMemcpyAsync(unc, h->d_unc, sizeof(double) * NENK, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d_attn);
-    cudaFree(d_stuck);
     if (e != cudaSuccess) return cuda_fail(h, e, "lb_beam_uncollided");
-    if (stuck) return fail(h, LB_ERR_STATE, "lb_beam_uncollided: a ray walk did not reach the beam plane");
+    if (unc && (rc = pipe_down(h, unc, h->d_unc, sizeof(double) * NENK, "lb_beam_uncollided"))) return rc;
+    e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return cuda_fail(h, e, "lb_beam_uncollided");
+    if (*(volatile int*)stuck) return fail(h, LB_ERR_STATE, "lb_beam_uncollided: a ray walk did not reach the beam plane");
     return LB_OK;
 }

@@ -87,6 +87,7 @@ void timer_end(Handle* h, Timer& t) {
     if (!t.a) return;
     cudaEventRecord(t.b, h->stream);
     h->timers.push_back(t);
+    if (h->timers.size() >= 4096) timers_flush(h);   // events are reused from here on
 }
 
 void timers_flush(Handle* h) {
@@ -123,13 +124,28 @@ static int dev_upload(Handle* h, T** p, const T* src, size_t count, const char* 
     return LB_OK;
 }
 
+// Small tables replaced between solves: the buffer is kept, and the copy is ordered by the stream (a copy from
+// pageable memory has read its source when the call returns).
+template <class T>
+static int dev_replace(Handle* h, T** p, size_t* cap, const T* src, size_t count, const char* what) {
+    if (h->device < 0) return LB_OK;
+    if (*cap != count || !*p) {
+        const int rc = dev_alloc(h, p, count, what);
+        *cap = rc ? 0 : count;
+        if (rc) return rc;
+    }
+    const cudaError_t e = cudaMemcpyAsync(*p, src, sizeof(T) * count, cudaMemcpyHostToDevice, h->stream);
+    return e == cudaSuccess ? LB_OK : cuda_fail(h, e, what);
+}
+
 static void free_all(Handle* h) {
     void* ptrs[] = {h->d_geom, h->d_rec, h->d_crec, h->d_crec_base, h->d_blk_elem, h->d_beam_plane, h->d_beam_xyz,
-                    h->d_beam_node, h->d_beam_nbr, h->d_cl_start, h->d_cl_base, h->d_ncl, h->d_gtab, h->d_tmat, h->d_xtab, h->d_xmat, h->d_xtype, h->d_mat, h->d_items, h->d_groups, h->d_pitems, h->d_pbase, h->d_chunks, h->d_lvl_start, h->d_lvl_base, h->d_nlev, h->d_done, h->d_status, h->d_tc_err, h->d_dirs, h->d_sigt,
+                    h->d_beam_node, h->d_beam_nbr, h->d_cl_start, h->d_cl_base, h->d_ncl, h->d_gtab, h->d_tmat, h->d_xtab, h->d_xmat, h->d_xtype, h->d_mat, h->d_items, h->d_groups, h->d_pitems, h->d_pbase, h->d_chunks, h->d_lvl_start, h->d_lvl_base, h->d_nlev, h->d_done, h->d_status, h->d_dirs, h->d_sigt,
                     h->d_psi, h->d_qext, h->d_Ym2d, h->d_Yd2m, h->d_sigl, h->d_lofj, h->d_V, h->d_Z, h->d_x,
                     h->d_b, h->d_t, h->d_red, h->d_unc, h->d_phi_all, h->d_src, h->d_dose, h->d_flux,
                     h->d_sigl_mg, h->d_yb, h->d_dd};
     for (void* p : ptrs) if (p) cudaFree(p);
+    pipe_free(h);
     if (h->h_red) cudaFreeHost(h->h_red);
     if (h->d_seg) cudaFree(h->d_seg);
     if (h->h_seg) cudaFreeHost(h->h_seg);
@@ -235,12 +251,12 @@ int lb_create(int device, lb_handle** out) {
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) { delete h; return LB_ERR_CUDA; }
     cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (cudaMalloc(&h->d_status, sizeof(SweepStatus)) != cudaSuccess) { delete h; return LB_ERR_OOM; }
-    if (cudaMalloc(&h->d_tc_err, sizeof(int)) != cudaSuccess || cudaMemset(h->d_tc_err, 0, sizeof(int)) != cudaSuccess) {
-        delete h;
-        return LB_ERR_OOM;
-    }
-    if (cudaMallocHost(&h->h_red, sizeof(double) * 65536) != cudaSuccess) { delete h; return LB_ERR_OOM; }
-    if (cudaMalloc(&h->d_red, sizeof(double) * 65536) != cudaSuccess) { delete h; return LB_ERR_OOM; }
+    // one pinned allocation: reduction results, the small transfer buffers, the contractions' timeout flag
+    const size_t pinned = sizeof(double) * kRedHost + 2 * kPipeSmall;
+    if (cudaMallocHost(&h->h_red, pinned + 64) != cudaSuccess) { delete h; return LB_ERR_OOM; }
+    h->d_tc_err = reinterpret_cast<int*>(reinterpret_cast<char*>(h->h_red) + pinned);
+    *h->d_tc_err = 0;
+    if (cudaMalloc(&h->d_red, sizeof(double) * kRedValues) != cudaSuccess) { delete h; return LB_ERR_OOM; }
     *out = h;
     return LB_OK;
 }
@@ -1139,13 +1155,13 @@ int lb_set_xs(lb_handle* h, int Ls, const double* sigt, const double* sigs) {
     int rc;
     std::vector<float> st(Nm);
     for (int m = 0; m < Nm; ++m) st[m] = (float)sigt[m];
-    rc = dev_upload(h, &h->d_sigt, st.data(), st.size(), "upload sigt");
+    rc = dev_replace(h, &h->d_sigt, &h->sigt_cap, st.data(), st.size(), "upload sigt");
     if (rc) return rc;
     std::vector<float> sl((size_t)Nm * nmpad, 0.f);
     for (int m = 0; m < Nm; ++m)
         for (int l = 0; l <= Ls; ++l)
             for (int j = l * l; j < (l + 1) * (l + 1); ++j) sl[(size_t)m * nmpad + j] = (float)sigs[(size_t)m * (Ls + 1) + l];
-    rc = dev_upload(h, &h->d_sigl, sl.data(), sl.size(), "upload sigma_l");
+    rc = dev_replace(h, &h->d_sigl, &h->sigl_cap, sl.data(), sl.size(), "upload sigma_l");
     if (rc) return rc;
     if (rebuild || !h->d_Ym2d) {
         // split Y into three BF16 planes (hi + mid + lo carries 24 significant bits)

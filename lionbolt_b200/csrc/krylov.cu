@@ -225,16 +225,6 @@ __global__ void fill_kernel(double* y, double v, size_t n) {
     for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) y[q] = v;
 }
 
-__global__ void f64_to_f32_kernel(float* y, const double* x, size_t n) {
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-        y[q] = (float)x[q];
-}
-
-__global__ void f32_to_f64_kernel(double* y, const float* x, size_t n) {
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-        y[q] = (double)x[q];
-}
-
 // src[j][n] (+)= sigl[mat(n)][j] * phi[j][n]
 __global__ void moment_source_kernel(double* src, const double* __restrict__ phi, const float* __restrict__ sigl,
                                      const int* __restrict__ mat, long long NENK, int nm, int nmpad, int accumulate) {
@@ -424,6 +414,7 @@ inline int grid_for(Handle* h, size_t n) {
 
 // Sum of the per-block partials (block order: deterministic) for entries 0..cnt-1.
 static int reduce_partials(Handle* h, int grid, int cnt, double* out) {
+    if ((size_t)grid * kPartStride > kRedHost) return fail(h, LB_ERR_ARG, "Krylov reduction: too many blocks");
     cudaError_t e = cudaMemcpyAsync(h->h_red, h->d_red, sizeof(double) * (size_t)grid * kPartStride,
                                     cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -600,22 +591,6 @@ int k_fill(Handle* h, double* y, double v, size_t n) {
     return LB_OK;
 }
 
-int k_f64_to_f32(Handle* h, float* y, const double* x, size_t n) {
-    Timer t;
-    timer_begin(h, LB_T_COPY, t);
-    f64_to_f32_kernel<<<grid_for(h, n), 256, 0, h->stream>>>(y, x, n);
-    timer_end(h, t);
-    return LB_OK;
-}
-
-int k_f32_to_f64(Handle* h, double* y, const float* x, size_t n) {
-    Timer t;
-    timer_begin(h, LB_T_COPY, t);
-    f32_to_f64_kernel<<<grid_for(h, n), 256, 0, h->stream>>>(y, x, n);
-    timer_end(h, t);
-    return LB_OK;
-}
-
 int k_moment_source(Handle* h, double* src, const double* phi, const float* sigl, const int* mat, long long NENK, int nm,
                     int nmpad, int accumulate) {
     Timer t;
@@ -703,15 +678,19 @@ static int seg_upload(Handle* h, const std::vector<SegVec>& segs, const std::vec
 
 static int seg_reduce(Handle* h, const std::vector<SegVec>& segs, int cnt, std::vector<double>& out) {
     const int grid = segs.back().blk0 + segs.back().nblk;
-    cudaError_t e = cudaMemcpyAsync(h->h_red, h->d_red, sizeof(double) * (size_t)grid * kPartStride,
-                                    cudaMemcpyDeviceToHost, h->stream);
+    if ((size_t)grid * kPartStride > kRedValues) return fail(h, LB_ERR_ARG, "segmented reduction: too many blocks");
+    // (a batch of more than some 650 problems has more blocks than the pinned buffer holds)
+    std::vector<double> wide((size_t)grid * kPartStride > kRedHost ? (size_t)grid * kPartStride : 0);
+    const double* red = wide.empty() ? h->h_red : wide.data();
+    cudaError_t e = cudaMemcpyAsync(wide.empty() ? h->h_red : wide.data(), h->d_red,
+                                    sizeof(double) * (size_t)grid * kPartStride, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "segmented reduction");
     out.assign(segs.size() * (size_t)cnt, 0.0);
     for (size_t si = 0; si < segs.size(); ++si)
         for (int j = 0; j < cnt; ++j) {
             double acc = 0.0;
-            for (int b = segs[si].blk0; b < segs[si].blk0 + segs[si].nblk; ++b) acc += h->h_red[(size_t)b * kPartStride + j];
+            for (int b = segs[si].blk0; b < segs[si].blk0 + segs[si].nblk; ++b) acc += red[(size_t)b * kPartStride + j];
             out[si * cnt + j] = acc;
         }
     return LB_OK;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -15,6 +16,11 @@ constexpr int kClusterSize = 6;
 
 // tile types a slot of a block record can name (5 bits)
 constexpr int kMaxTileTypes = 32;
+
+// pinned memory of a handle, 510 KB in one allocation (a larger one takes milliseconds more)
+constexpr size_t kRedHost = 40960;               // reduction partials (at most 8 blocks per SM of 33 values)
+constexpr size_t kPipeSmall = 95 << 10;          // bytes of each small transfer buffer
+constexpr size_t kRedValues = 65536;             // reduction partials on the device
 
 // Packed schedule item (one per element-direction, in sweep order):
 //   bits 0-23 element id, bits 24-27 upstream-face mask, bits 28-31 outflow-face mask.
@@ -145,9 +151,11 @@ struct Handle {
     int* d_nlev = nullptr;         // [NI]
     int* d_done = nullptr;         // [total_levels]
     SweepStatus* d_status = nullptr;
-    int* d_tc_err = nullptr;      // set to LB_ERR_TIMEOUT by a contraction kernel whose pipeline wait gave up
+    int* d_tc_err = nullptr;      // set to LB_ERR_TIMEOUT by a contraction kernel whose pipeline wait gave up (pinned
+                                  // host memory, written by the device only then: reading it costs no copy)
     float4* d_dirs = nullptr;      // [NI] (kx, ky, kz, w)
     float* d_sigt = nullptr;       // [Nm]
+    size_t sigt_cap = 0, sigl_cap = 0;   // values d_sigt and d_sigl hold
     float* d_psi = nullptr;        // [NI][NENK] FP32 angular work vector
     float* d_qext = nullptr;       // [NI][NENK] FP32 angular external source (angular API)
     // moment-space operators (split BF16 hi/mid/lo planes)
@@ -166,7 +174,7 @@ struct Handle {
     double* d_b = nullptr;         // rhs
     double* d_t = nullptr;         // scratch
     double* d_red = nullptr;       // reduction partials
-    double* h_red = nullptr;       // pinned host copy of reductions
+    double* h_red = nullptr;       // pinned host copy of reductions [kRedHost], then the small transfer buffers
     size_t kry_n = 0;
 
     // ---- multigroup ----
@@ -199,6 +207,15 @@ struct Handle {
     int sweep_cfg_forced = -1;     // set through LB_SWEEP_CONFIG for experiments
 
     cudaEvent_t marks[16] = {};
+
+    // pinned transfer buffers (transfer.cpp): a small pair behind h_red, and a large one once it is needed
+    struct Pipe {
+        void* buf[2] = {nullptr, nullptr};
+        cudaEvent_t ev[2] = {nullptr, nullptr};   // the buffer's last copy
+        size_t bytes = 0;          // of each buffer
+        int next = 0;
+    };
+    Pipe pipe_small, pipe_large;
 
     // planar-beam ray walk (beam.cu): face planes, coordinates, connectivity, neighbours on the device
     double4* d_beam_plane = nullptr;
@@ -335,6 +352,18 @@ int seg_axpy_scale(Handle* h, const std::vector<SegVec>& segs, int nv, const std
 // w = a x + b w and out[s] = w . w
 int seg_axpby_norm(Handle* h, const std::vector<SegVec>& segs, std::vector<double>& out);
 
+// ---- transfers (transfer.cpp): through the handle's pinned buffers; an upload's source is free on return, a
+// download is complete on return ----
+int pipe_up_f32(Handle* h, float* dst, const double* src, size_t n, const char* what);
+// dst = src, or dst -= src
+int pipe_down_f32(Handle* h, double* dst, const float* src, size_t n, bool subtract, const char* what);
+int pipe_up(Handle* h, void* dst, const void* src, size_t bytes, const char* what);
+int pipe_down(Handle* h, void* dst, const void* src, size_t bytes, const char* what);
+// row(buffer, q) writes row q (row_bytes bytes); called from several threads
+int pipe_up_rows(Handle* h, void* dst, size_t rows, size_t row_bytes, const std::function<void(void*, size_t)>& row,
+                 const char* what);
+void pipe_free(Handle* h);
+
 // ---- timers ----
 void timer_begin(Handle* h, int kind, Timer& t);
 void timer_end(Handle* h, Timer& t);
@@ -384,8 +413,6 @@ constexpr int kMaxRowCoefs = 64;   // moment rows of k_scale_rows (P7)
 int k_scale_rows(Handle* h, double* z, const double* v, const double* coef, int nm, size_t NENK);   // z_j = c_j v_j
 int k_copy(Handle* h, double* y, const double* x, size_t n);
 int k_fill(Handle* h, double* y, double v, size_t n);
-int k_f64_to_f32(Handle* h, float* y, const double* x, size_t n);
-int k_f32_to_f64(Handle* h, double* y, const float* x, size_t n);
 int k_dose_tally(Handle* h, const double* phi00, const double* unc, double unc_scale, const double* dd_mat,
                  const int* mat, double* flux, double* dose, long long NENK);
 int k_moment_source(Handle* h, double* src, const double* phi, const float* sigl, const int* mat, long long NENK,

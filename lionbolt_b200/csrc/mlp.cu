@@ -55,10 +55,9 @@ struct MlpState {
     float* d_w = nullptr;          // [NPARAM] FP32 master weights
     float* d_m = nullptr;          // Adam first moment
     float* d_v = nullptr;          // Adam second moment
-    float* d_part = nullptr;       // [max_parts][NPARAM] per-block gradient partials
-    double* d_lossp = nullptr;     // [max_parts] per-block loss partials
+    void* d_ws = nullptr;          // workspace of the gradient and of host-supplied batches (workspace), grown by need
+    size_t ws_bytes = 0;
     double* d_losshist = nullptr;  // [hist_cap]
-    int max_parts = 0;
     int hist_cap = 0;
     float* d_X = nullptr;          // [cap][FS] sample features
     float* d_T = nullptr;          // [cap][16] sample targets
@@ -84,7 +83,7 @@ bool mlp_ready(Handle* h) { return h->mlp && S(h)->have_weights && S(h)->enabled
 void mlp_destroy(Handle* h) {
     MlpState* s = S(h);
     if (!s) return;
-    for (void* p : {(void*)s->d_w, (void*)s->d_m, (void*)s->d_v, (void*)s->d_part, (void*)s->d_lossp,
+    for (void* p : {(void*)s->d_w, (void*)s->d_m, (void*)s->d_v, s->d_ws,
                     (void*)s->d_losshist, (void*)s->d_X, (void*)s->d_T, (void*)s->d_chord, (void*)s->d_matxs})
         if (p) cudaFree(p);
     delete s;
@@ -792,18 +791,36 @@ int mlp_sample(Handle* h, const double* r, const double* err, long long count, u
     return LB_OK;
 }
 
-static int ensure_grad_bufs(Handle* h, MlpState* s, int parts, int hist) {
-    cudaError_t e = cudaSuccess;
-    if (parts > s->max_parts) {
-        if (s->d_part) cudaFree(s->d_part);
-        if (s->d_lossp) cudaFree(s->d_lossp);
-        s->d_part = nullptr;
-        s->d_lossp = nullptr;
-        e = cudaMalloc(&s->d_part, sizeof(float) * NPARAM * (size_t)parts);
-        if (e == cudaSuccess) e = cudaMalloc(&s->d_lossp, sizeof(double) * parts);
-        if (e != cudaSuccess) return cuda_fail(h, e, "gradient partials");
-        s->max_parts = parts;
+// Workspace of a gradient over `parts` blocks and of a host-supplied batch of n samples.
+struct Workspace {
+    double* lossp;   // [parts] per-block loss partials
+    float* part;     // [parts][NPARAM] per-block gradient partials
+    float* grad;     // [NPARAM]
+    float* x;        // [n][FS]
+    float* t;        // [n][NOUT] targets, or outputs
+};
+
+static int workspace(Handle* h, MlpState* s, int parts, size_t n, Workspace* w) {
+    const size_t head = (sizeof(double) * parts + 255) / 256 * 256;
+    const size_t bytes = head + sizeof(float) * ((size_t)NPARAM * (parts + 1) + (lp::FS + lp::NOUT) * n);
+    if (bytes > s->ws_bytes) {
+        if (s->d_ws) cudaFree(s->d_ws);
+        s->d_ws = nullptr;
+        s->ws_bytes = 0;
+        const cudaError_t e = cudaMalloc(&s->d_ws, bytes);
+        if (e != cudaSuccess) return cuda_fail(h, e, "gradient workspace");
+        s->ws_bytes = bytes;
     }
+    w->lossp = reinterpret_cast<double*>(s->d_ws);
+    w->x = reinterpret_cast<float*>(reinterpret_cast<char*>(s->d_ws) + head);
+    w->t = w->x + lp::FS * n;
+    w->grad = w->t + lp::NOUT * n;
+    w->part = w->grad + NPARAM;
+    return LB_OK;
+}
+
+static int ensure_grad_bufs(Handle* h, MlpState* s, int hist) {
+    cudaError_t e = cudaSuccess;
     if (hist > s->hist_cap) {
         if (s->d_losshist) cudaFree(s->d_losshist);
         e = cudaMalloc(&s->d_losshist, sizeof(double) * hist);
@@ -917,23 +934,19 @@ int lb_lp_forward(lb_handle* h, int n, const float* x, float* y) {
     if (!s || !s->have_weights) return fail(h, LB_ERR_STATE, "lb_lp_forward: no weights");
     if (n < 0 || (n > 0 && (!x || !y))) return fail(h, LB_ERR_ARG, "lb_lp_forward: bad arguments");
     if (n == 0) return LB_OK;
-    std::vector<float> xs((size_t)n * lp::FS, 0.f);
-    for (int i = 0; i < n; ++i) std::memcpy(&xs[(size_t)i * lp::FS], x + (size_t)i * lp::NIN, sizeof(float) * lp::NIN);
-    float *dx = nullptr, *dy = nullptr;
-    cudaError_t e = cudaMalloc(&dx, sizeof(float) * xs.size());
-    if (e == cudaSuccess) e = cudaMalloc(&dy, sizeof(float) * (size_t)n * lp::NOUT);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dx, xs.data(), sizeof(float) * xs.size(), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-        const long long ntiles = ((long long)n + 15) / 16;
-        lp_forward_kernel<<<infer_grid(h, (const void*)lp_forward_kernel, ntiles), lp::kThreads, sizeof(InferSmem),
-                            h->stream>>>(s->d_w, dx, n, dy);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(y, dy, sizeof(float) * (size_t)n * lp::NOUT, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (dx) cudaFree(dx);
-    if (dy) cudaFree(dy);
-    return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "lb_lp_forward");
+    Workspace ws;
+    if ((rc = workspace(h, s, 0, n, &ws))) return rc;
+    rc = pipe_up_rows(h, ws.x, n, sizeof(float) * lp::FS, [&](void* b, size_t i) {
+        std::memcpy(b, x + i * lp::NIN, sizeof(float) * lp::NIN);
+        ((float*)b)[lp::NIN] = 0.f;
+    }, "lb_lp_forward");
+    if (rc) return rc;
+    const long long ntiles = ((long long)n + 15) / 16;
+    lp_forward_kernel<<<infer_grid(h, (const void*)lp_forward_kernel, ntiles), lp::kThreads, sizeof(InferSmem),
+                        h->stream>>>(s->d_w, ws.x, n, ws.t);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(h, e, "lb_lp_forward");
+    return pipe_down(h, y, ws.t, sizeof(float) * (size_t)n * lp::NOUT, "lb_lp_forward");
 }
 
 int lb_lp_apply(lb_handle* h, const double* v, double* z) {
@@ -969,32 +982,23 @@ int lb_lp_loss_grad(lb_handle* h, int n, const float* x, const float* t, const f
     if (!s || !s->have_weights) return fail(h, LB_ERR_STATE, "lb_lp_loss_grad: no weights");
     if (n <= 0 || !x || !t) return fail(h, LB_ERR_ARG, "lb_lp_loss_grad: bad arguments");
     const int parts = grad_blocks(h, n);
-    if ((rc = ensure_grad_bufs(h, s, parts, 1))) return rc;
-    std::vector<float> xs((size_t)n * lp::FS, 0.f);
-    for (int i = 0; i < n; ++i) {
-        std::memcpy(&xs[(size_t)i * lp::FS], x + (size_t)i * lp::NIN, sizeof(float) * lp::NIN);
-        xs[(size_t)i * lp::FS + lp::NIN] = wts ? wts[i] : 1.f;
-    }
-    float *dx = nullptr, *dt = nullptr, *dg = nullptr;
-    cudaError_t e = cudaMalloc(&dx, sizeof(float) * xs.size());
-    if (e == cudaSuccess) e = cudaMalloc(&dt, sizeof(float) * (size_t)n * lp::NOUT);
-    if (e == cudaSuccess) e = cudaMalloc(&dg, sizeof(float) * lp::NPARAM);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dx, xs.data(), sizeof(float) * xs.size(), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, sizeof(float) * (size_t)n * lp::NOUT, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-        lp_grad_kernel<<<parts, lp::kThreads, kGradSmem, h->stream>>>(s->d_w, dx, dt, n, n, 1, 0ull, 1.f / n, s->d_part,
-                                                                       s->d_lossp);
-        lp_gradsum_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(s->d_part, parts, dg);
-        e = cudaGetLastError();
-    }
-    std::vector<double> lp_(parts);
-    if (e == cudaSuccess && grad) e = cudaMemcpyAsync(grad, dg, sizeof(float) * lp::NPARAM, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(lp_.data(), s->d_lossp, sizeof(double) * parts, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (dx) cudaFree(dx);
-    if (dt) cudaFree(dt);
-    if (dg) cudaFree(dg);
+    Workspace ws;
+    if ((rc = ensure_grad_bufs(h, s, 0)) || (rc = workspace(h, s, parts, n, &ws))) return rc;
+    rc = pipe_up_rows(h, ws.x, n, sizeof(float) * lp::FS, [&](void* b, size_t i) {
+        std::memcpy(b, x + i * lp::NIN, sizeof(float) * lp::NIN);
+        ((float*)b)[lp::NIN] = wts ? wts[i] : 1.f;
+    }, "lb_lp_loss_grad");
+    if (!rc) rc = pipe_up(h, ws.t, t, sizeof(float) * (size_t)n * lp::NOUT, "lb_lp_loss_grad");
+    if (rc) return rc;
+    lp_grad_kernel<<<parts, lp::kThreads, kGradSmem, h->stream>>>(s->d_w, ws.x, ws.t, n, n, 1, 0ull, 1.f / n, ws.part,
+                                                                   ws.lossp);
+    lp_gradsum_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(ws.part, parts, ws.grad);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(h, e, "lb_lp_loss_grad");
+    std::vector<double> lp_(parts);
+    if (grad) rc = pipe_down(h, grad, ws.grad, sizeof(float) * lp::NPARAM, "lb_lp_loss_grad");
+    if (!rc) rc = pipe_down(h, lp_.data(), ws.lossp, sizeof(double) * parts, "lb_lp_loss_grad");
+    if (rc) return rc;
     if (loss) {
         double sum = 0.0;
         for (double v : lp_) sum += v;
@@ -1040,7 +1044,8 @@ int lb_lp_train(lb_handle* h, int steps, int batch, double lr, unsigned long lon
     if (s->nsamples <= 0) return fail(h, LB_ERR_STATE, "lb_lp_train: no training samples");
     if (steps < 0 || batch < 1 || !(lr > 0.0)) return fail(h, LB_ERR_ARG, "lb_lp_train: bad arguments");
     const int parts = grad_blocks(h, batch);
-    if ((rc = ensure_grad_bufs(h, s, parts, std::max(steps, 1)))) return rc;
+    Workspace ws;
+    if ((rc = ensure_grad_bufs(h, s, std::max(steps, 1))) || (rc = workspace(h, s, parts, 0, &ws))) return rc;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const double pi = 3.14159265358979323846;
     for (int it = 0; it < steps; ++it) {
@@ -1051,8 +1056,8 @@ int lb_lp_train(lb_handle* h, int steps, int batch, double lr, unsigned long lon
         const float bc1 = 1.f - std::pow(b1, (float)s->adam_t), bc2 = 1.f - std::pow(b2, (float)s->adam_t);
         lp_grad_kernel<<<parts, lp::kThreads, kGradSmem, h->stream>>>(
             s->d_w, s->d_X, s->d_T, s->nsamples, batch, 0, seed + 0x100000001B3ull * (unsigned long long)it,
-            1.f / batch, s->d_part, s->d_lossp);
-        lp_adam_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(s->d_w, s->d_m, s->d_v, s->d_part, s->d_lossp,
+            1.f / batch, ws.part, ws.lossp);
+        lp_adam_kernel<<<(lp::NPARAM + 31) / 32, 32 * kSumSlices, 0, h->stream>>>(s->d_w, s->d_m, s->d_v, ws.part, ws.lossp,
                                                                          parts, lr_t, b1, b2, eps, bc1, bc2,
                                                                          s->d_losshist, it);
     }

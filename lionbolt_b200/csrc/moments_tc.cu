@@ -84,7 +84,7 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, int* er
         if (bar_try_wait(bar, parity)) return true;
         if ((it & 1023) == 1023 && *(volatile int*)err) return false;
     }
-    atomicExch(err, LB_ERR_TIMEOUT);
+    *(volatile int*)err = LB_ERR_TIMEOUT;
     return false;
 }
 
@@ -1175,14 +1175,11 @@ int tc_wait_probe(Handle* h, long long polls) {
 // when a tensor-core contraction gave up on a pipeline wait since the last check.
 int moments_tc_status(Handle* h) {
     if (!h->d_tc_err) return LB_OK;
-    int v = 0;
-    cudaError_t e = cudaMemcpyAsync(&v, h->d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "contraction status");
-    if (!v) return LB_OK;
-    e = cudaMemsetAsync(h->d_tc_err, 0, sizeof(int), h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return cuda_fail(h, e, "contraction status");
+    volatile int* flag = h->d_tc_err;
+    if (!*flag) return LB_OK;
+    *flag = 0;
     return fail(h, LB_ERR_TIMEOUT, "tensor-core moment kernel: pipeline wait timed out (results invalid)");
 }
 

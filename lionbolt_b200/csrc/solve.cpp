@@ -48,7 +48,7 @@ int ensure_krylov(Handle* h, int m, bool flexible) {
         h->kry_m = m;
     }
     if (!h->d_red) {
-        cudaError_t e = cudaMalloc(&h->d_red, sizeof(double) * 65536);
+        cudaError_t e = cudaMalloc(&h->d_red, sizeof(double) * kRedValues);
         if (e != cudaSuccess) return cuda_fail(h, e, "reduction buffer");
     }
     if (flexible && !h->d_Z) {
@@ -329,45 +329,14 @@ static KrylovResult moment_solve(Handle* h, const double* b, double* phi, int so
     return gmres_device(h, n, b, phi, m, rtol, atol, maxit, mv, nullptr, &mz);
 }
 
-// ---------------------------------------------------------------------------------------------
-//  angular <-> device transfers (FP64 host, FP32 device), chunked through a pinned staging area
-// ---------------------------------------------------------------------------------------------
+// angular vectors: FP64 on the host, FP32 on the device
 static int upload_angular(Handle* h, const double* hs, float* d) {
-    const size_t total = h->psi_elems;
-    const size_t chunk = (size_t)1 << 24;
-    double* stage = nullptr;
-    cudaError_t e = cudaMalloc(&stage, sizeof(double) * std::min(total, chunk));
-    if (e != cudaSuccess) return cuda_fail(h, e, "staging buffer");
-    for (size_t o = 0; o < total; o += chunk) {
-        size_t c = std::min(chunk, total - o);
-        e = cudaMemcpyAsync(stage, hs + o, sizeof(double) * c, cudaMemcpyHostToDevice, h->stream);
-        if (e != cudaSuccess) break;
-        k_f64_to_f32(h, d + o, stage, c);
-        e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) break;
-    }
-    cudaFree(stage);
-    return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "upload angular vector");
+    return pipe_up_f32(h, d, hs, h->psi_elems, "upload angular vector");
 }
 
-static int download_angular(Handle* h, const float* d, double* hs) {
-    const size_t total = h->psi_elems;
-    const size_t chunk = (size_t)1 << 24;
-    double* stage = nullptr;
-    cudaError_t e = cudaMalloc(&stage, sizeof(double) * std::min(total, chunk));
-    if (e != cudaSuccess) return cuda_fail(h, e, "staging buffer");
-    for (size_t o = 0; o < total; o += chunk) {
-        size_t c = std::min(chunk, total - o);
-        k_f32_to_f64(h, stage, d + o, c);
-        e = cudaMemcpyAsync(hs + o, stage, sizeof(double) * c, cudaMemcpyDeviceToHost, h->stream);
-        if (e != cudaSuccess) break;
-        e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) break;
-    }
-    cudaFree(stage);
-    return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "download angular vector");
+static int download_angular(Handle* h, const float* d, double* hs, bool subtract = false) {
+    return pipe_down_f32(h, hs, d, h->psi_elems, subtract, "download angular vector");
 }
-
 
 }  // namespace lb
 
@@ -386,8 +355,8 @@ float* mg_table(Handle* h, int gp, int g) {
 void mg_prepare(Handle* h) {
     std::vector<double> yb(h->nm);
     real_sh(h->Ls, h->beam_dir.data(), yb.data());
+    // (a copy from pageable memory has read it when the call returns)
     cudaMemcpyAsync(h->d_yb, yb.data(), sizeof(double) * h->nm, cudaMemcpyHostToDevice, h->stream);
-    cudaStreamSynchronize(h->stream);
 }
 
 // Source and operator of group g from the solved groups g' < g in d_phi_all:
@@ -468,12 +437,8 @@ int lb_boltzmann_matvec(lb_handle* h, double* x) {
     if ((rc = launch_d2m(h, h->d_psi, nullptr, 0.0, 1.0, h->d_t))) return rc;
     if ((rc = launch_m2d(h, h->d_t, h->d_sigl, nullptr, nullptr, h->d_psi))) return rc;
     if ((rc = launch_sweep(h, h->d_psi))) return rc;
-    std::vector<double> y(h->psi_elems);
-    if ((rc = download_angular(h, h->d_psi, y.data()))) return rc;
-    if ((rc = moments_tc_status(h))) return rc;
-#pragma omp parallel for schedule(static)
-    for (size_t q = 0; q < y.size(); ++q) x[q] = x[q] - y[q];
-    return LB_OK;
+    if ((rc = moments_tc_status(h))) return rc;   // x stays as it was when a contraction gave up
+    return download_angular(h, h->d_psi, x, true);
 }
 
 int lb_boltzmann_solve(lb_handle* h, double* s, int solver, int m, double rtol, double atol, int maxit, int* iters,
@@ -559,15 +524,11 @@ int lb_mg_set_problem(lb_handle* h, int G, int Ls, const double* sigt, const dou
         if ((rc = realloc(&h->d_dd, (size_t)G * Nm, "dose cross sections"))) return rc;
         h->mg_alloc_G = G; h->mg_alloc_nm = nm; h->mg_alloc_NENK = (long long)NENK; h->mg_alloc_tab = tab.size();
     }
-    cudaError_t e = cudaMemcpyAsync(h->d_sigl_mg, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_dd, dd, sizeof(double) * (size_t)G * Nm, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-        if (unc) e = cudaMemcpyAsync(h->d_unc, unc, sizeof(double) * NENK, cudaMemcpyHostToDevice, h->stream);
-        else e = cudaMemsetAsync(h->d_unc, 0, sizeof(double) * NENK, h->stream);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return cuda_fail(h, e, "upload problem");
-    return LB_OK;
+    if ((rc = pipe_up(h, h->d_sigl_mg, tab.data(), sizeof(float) * tab.size(), "upload problem"))) return rc;
+    if ((rc = pipe_up(h, h->d_dd, dd, sizeof(double) * (size_t)G * Nm, "upload problem"))) return rc;
+    if (unc) return pipe_up(h, h->d_unc, unc, sizeof(double) * NENK, "upload problem");
+    const cudaError_t e = cudaMemsetAsync(h->d_unc, 0, sizeof(double) * NENK, h->stream);
+    return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "upload problem");
 }
 
 int lb_mg_update_inputs(lb_handle* h, const double* sigt, const double* sigs, const double* dd, const double* unc,
@@ -652,11 +613,10 @@ int lb_lp_calibrate(lb_handle* h, int m, double rtol, int* plain_iters, int* lea
 int lb_mg_get_results(lb_handle* h, double* flux, double* dose) {
     if (!h || h->device < 0 || !h->d_dose) return LB_ERR_STATE;
     cudaSetDevice(h->device);
-    cudaError_t e = cudaSuccess;
-    if (flux) e = cudaMemcpyAsync(flux, h->d_flux, sizeof(double) * (size_t)h->G * h->NENK, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess && dose)
-        e = cudaMemcpyAsync(dose, h->d_dose, sizeof(double) * (size_t)h->NENK, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    int rc = flux ? pipe_down(h, flux, h->d_flux, sizeof(double) * (size_t)h->G * h->NENK, "read results") : LB_OK;
+    if (!rc && dose) rc = pipe_down(h, dose, h->d_dose, sizeof(double) * (size_t)h->NENK, "read results");
+    if (rc || flux || dose) return rc;
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
     return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "read results");
 }
 
