@@ -412,12 +412,11 @@ inline int grid_for(Handle* h, size_t n) {
 
 }  // namespace
 
-// Sum of the per-block partials (block order: deterministic) for entries 0..cnt-1.
+// Sum of the per-block partials (block order: deterministic) for entries 0..cnt-1.  The blocks write their
+// partials straight into pinned host memory (a few values per block: some 20 KB over the bus as the kernel
+// drains), so that a reduction ends with its kernel instead of a 150 to 300 KB copy behind it.
 static int reduce_partials(Handle* h, int grid, int cnt, double* out) {
-    if ((size_t)grid * kPartStride > kRedHost) return fail(h, LB_ERR_ARG, "Krylov reduction: too many blocks");
-    cudaError_t e = cudaMemcpyAsync(h->h_red, h->d_red, sizeof(double) * (size_t)grid * kPartStride,
-                                    cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "Krylov reduction");
     for (int j = 0; j < cnt; ++j) {
         double s = 0.0;
@@ -426,6 +425,9 @@ static int reduce_partials(Handle* h, int grid, int cnt, double* out) {
     }
     return LB_OK;
 }
+
+// Blocks of a reduction over the whole chip at `occ` resident blocks per SM, as many as the partials' buffer holds.
+static int red_grid(const Handle* h, int occ) { return std::min(h->sm_count * occ, (int)(kRedHost / kPartStride)); }
 
 static bool check_args(Handle* h, int nv, size_t n, const char* what, int* rc) {
     if (nv < 0 || nv > kMaxDots) { *rc = fail(h, LB_ERR_ARG, std::string(what) + ": too many vectors"); return false; }
@@ -447,13 +449,13 @@ int k_dots_norm(Handle* h, const double* V, size_t ldv, int nv, const double* w,
         if (zm) {
             if constexpr (NV >= 1) {
                 static const int occ = blocks_per_sm(dots_t<NV, true>);
-                grid = h->sm_count * occ;
-                dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(V, ldv, w, n / 2, h->d_red);
+                grid = red_grid(h, occ);
+                dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(V, ldv, w, n / 2, h->h_red);
             }
         } else {
             static const int occ = blocks_per_sm(dots_t<NV>);
-            grid = h->sm_count * occ;
-            dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(V, ldv, w, n / 2, h->d_red);
+            grid = red_grid(h, occ);
+            dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(V, ldv, w, n / 2, h->h_red);
         }
     });
     timer_end(h, t);
@@ -485,17 +487,17 @@ int k_axpy_dots(Handle* h, double* w, const double* V, size_t ldv, int nv, const
         if (zm) {
             if constexpr (NV >= 1) {
                 static const int occ = blocks_per_sm(axpy_dots_t<NV, true, true>);
-                grid = h->sm_count * occ;
-                axpy_dots_t<NV, true, true><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->d_red);
+                grid = red_grid(h, occ);
+                axpy_dots_t<NV, true, true><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->h_red);
             }
         } else if (dots) {
             static const int occ = blocks_per_sm(axpy_dots_t<NV, true>);
-            grid = h->sm_count * occ;
-            axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->d_red);
+            grid = red_grid(h, occ);
+            axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->h_red);
         } else {
             static const int occ = blocks_per_sm(axpy_dots_t<NV, false>);
-            grid = h->sm_count * occ;
-            axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->d_red);
+            grid = red_grid(h, occ);
+            axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(w, V, ldv, cf, n / 2, h->h_red);
         }
     });
     timer_end(h, t);
@@ -538,10 +540,10 @@ int k_axpby_norm(Handle* h, double* y, const double* x, double a, double b, size
     int rc = 0;
     if (!check_args(h, 0, n, "axpby", &rc)) return rc;
     static const int occ = blocks_per_sm(axpby_norm_kernel);
-    const int grid = h->sm_count * occ;
+    const int grid = red_grid(h, occ);
     Timer t;
     timer_begin(h, LB_T_KRYLOV, t);
-    axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(y, x, a, b, n / 2, h->d_red);
+    axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(y, x, a, b, n / 2, h->h_red);
     timer_end(h, t);
     double tmp[1];
     if ((rc = reduce_partials(h, grid, 1, tmp))) return rc;
@@ -676,14 +678,21 @@ static int seg_upload(Handle* h, const std::vector<SegVec>& segs, const std::vec
     return LB_OK;
 }
 
+// Where a segmented reduction's blocks write their partials: pinned host memory, as reduce_partials, or the
+// device buffer in a batch of more than some 650 problems, which has more blocks than the pinned one holds.
+static double* seg_partials(Handle* h, int grid) { return (size_t)grid * kPartStride <= kRedHost ? h->h_red : h->d_red; }
+
 static int seg_reduce(Handle* h, const std::vector<SegVec>& segs, int cnt, std::vector<double>& out) {
     const int grid = segs.back().blk0 + segs.back().nblk;
     if ((size_t)grid * kPartStride > kRedValues) return fail(h, LB_ERR_ARG, "segmented reduction: too many blocks");
-    // (a batch of more than some 650 problems has more blocks than the pinned buffer holds)
-    std::vector<double> wide((size_t)grid * kPartStride > kRedHost ? (size_t)grid * kPartStride : 0);
-    const double* red = wide.empty() ? h->h_red : wide.data();
-    cudaError_t e = cudaMemcpyAsync(wide.empty() ? h->h_red : wide.data(), h->d_red,
-                                    sizeof(double) * (size_t)grid * kPartStride, cudaMemcpyDeviceToHost, h->stream);
+    const double* red = seg_partials(h, grid);
+    std::vector<double> wide;
+    cudaError_t e = cudaSuccess;
+    if (red == h->d_red) {
+        wide.resize((size_t)grid * kPartStride);
+        e = cudaMemcpyAsync(wide.data(), h->d_red, sizeof(double) * wide.size(), cudaMemcpyDeviceToHost, h->stream);
+        red = wide.data();
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "segmented reduction");
     out.assign(segs.size() * (size_t)cnt, 0.0);
@@ -705,7 +714,7 @@ int seg_dots_norm(Handle* h, const std::vector<SegVec>& segs, int nv, std::vecto
     const int grid = segs.back().blk0 + segs.back().nblk;
     NvDispatch<kMaxDots>::run(nv, [&](auto c) {
         constexpr int NV = decltype(c)::value;
-        seg_dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), h->d_red);
+        seg_dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), seg_partials(h, grid));
     });
     return seg_reduce(h, segs, nv + 1, out);
 }
@@ -721,8 +730,8 @@ int seg_axpy_dots(Handle* h, const std::vector<SegVec>& segs, int nv, const std:
     const int grid = segs.back().blk0 + segs.back().nblk;
     NvDispatch<kMaxDots>::run(nv, [&](auto c) {
         constexpr int NV = decltype(c)::value;
-        if (dots) seg_axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, h->d_red);
-        else seg_axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, h->d_red);
+        if (dots) seg_axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, seg_partials(h, grid));
+        else seg_axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, seg_partials(h, grid));
     });
     return seg_reduce(h, segs, nv + 1, out);
 }
@@ -749,7 +758,7 @@ int seg_axpby_norm(Handle* h, const std::vector<SegVec>& segs, std::vector<doubl
     int rc = seg_upload(h, segs, nullptr, &ds, nullptr);
     if (rc) return rc;
     const int grid = segs.back().blk0 + segs.back().nblk;
-    seg_axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), h->d_red);
+    seg_axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), seg_partials(h, grid));
     return seg_reduce(h, segs, 1, out);
 }
 
