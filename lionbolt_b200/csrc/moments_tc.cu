@@ -52,6 +52,15 @@ __device__ __forceinline__ void mma_bf16_ss(uint32_t tmem_d, uint64_t da, uint64
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc));
 }
 
+// The same with A in tensor memory (32-bit columns of two BF16 along K, one lane per row).
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc));
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
@@ -109,6 +118,14 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
 }
+
+// Four columns of the calling warp's 32 lanes (eight BF16 along K per lane).
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, uint4 v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z),
+                 "r"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // The warp calling this allocates ncols TMEM columns (power of two >= 32) and publishes the base.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
@@ -638,63 +655,68 @@ __global__ void __launch_bounds__(kD2mThreads, 1) d2m_tc_kernel(const int* __res
 
 // ---------------------------------------------------------------------------------------------
 // D2M with the angular vector streamed by the tensor-memory accelerator: the same product as
-// d2m_tc_kernel, with psi brought into a ring of kT32 shared-memory stages by
-// cp.async.bulk.tensor (a 2-D tensor map over psi[NI][NENK], box = 128 nodes x kKT directions;
-// directions past NI and nodes past NENK are filled with zeros), so no thread waits on a global
-// load.  Chunks of kKT = 32 directions (two MMA K-steps):
+// d2m_tc_kernel, with psi brought into a ring of shared-memory stages by cp.async.bulk.tensor (a 2-D tensor map
+// over psi[NI][NENK], box = 128 nodes x kKT directions; directions past NI and nodes past NENK are filled with
+// zeros), so no thread waits on a global load.  Chunks of kKT = 32 directions (two MMA K-steps):
 //   warp 0 lane 0    TMA issue: waits for a free FP32 stage, arms its barrier with the byte count and
 //                    issues the copy;
-//   warps 1-8        converters (kD2tSets sets of 8 warps taking alternate chunks; one set: 14 warps,
-//                    at most 4 per SM sub-partition, so up to 128 registers a thread): threads t and
-//                    t + 128 of a set take node t & 127 of the tile and 16 directions each, read them
-//                    from the FP32 stage (then release it), split them into BF16 planes and write the
-//                    A stage;
+//   warps 1-8        converters: the two warps of a TMEM lane quarter (warp % 4) take its 32 nodes, 16
+//                    directions each: read them from the FP32 stage (then release it), split them into BF16
+//                    planes and write those to an A stage in tensor memory;
 //   warps 9-12       epilogue, as d2m_tc_kernel (the warps index nodes by their TMEM lane quarter);
 //   warp 13          lane 0 issues the MMAs; the warp owns the TMEM allocation.
-// The leading split product (hi x hi) accumulates in its own TMEM accumulator and the five smaller
-// products in a second one, added in the epilogue: the tensor core's accumulation of the full-size
-// terms then runs over 18 MMAs per tile (288 directions) instead of all 108, which is where the split
-// product lost accuracy against an FP32 GEMM (the small terms' accumulator is 2^-8 of the result).
+// The B planes are interleaved along N ([hi; mid; lo] rows per K column), so that one MMA of N = 3 nmpad takes
+// hi x {hi, mid, lo}, one of N = 2 nmpad mid x {hi, mid} and one of N = nmpad lo x hi.  The accumulator of a tile
+// holds three column groups (the hi x hi product, the 2^-8 products, the 2^-16 products), summed by the epilogue:
+// the tensor core's accumulation of the full-size terms then runs over 18 MMAs per tile (288 directions) instead
+// of 108, which is where the split product lost accuracy against an FP32 GEMM.
+//
+// A in tensor memory: with A in shared memory a chunk of 16 KB of psi moved about 100 KB through shared memory
+// (stage in and out 32 KB, A planes written and read 49 KB, B 18 KB), 0.61 ms of the 0.87 ms at 3,072,000 nodes and
+// 288 directions at the SM's 128 bytes per clock; without the A planes it is half.  The A stages use what the two tile
+// accumulators (3 nmpad columns each) leave of the 512 TMEM columns, 48 columns a stage.
+// Measured there: a first call 0.87 ms against 0.93, repeated without a pause (the chip's power limit then holds the
+// clock down) 0.992 against 1.049; 192,000 nodes, 288 directions, P5: 71 us against 75.
 // Every wait is bounded (error flag), as in the other kernels.  No cluster, no multicast.
 // ---------------------------------------------------------------------------------------------
 constexpr int kKT = 32;        // directions per K chunk
-constexpr int kT32 = 5;        // FP32 stages (TMA ring)
-constexpr int kTA = 2;         // BF16 A stages
-constexpr int kD2tSets = 1;    // converter sets of 8 warps, taking alternate chunks
+constexpr int kT32 = 8;        // FP32 stages (TMA ring)
+constexpr int kTA = 4;         // A stages at most
+constexpr int kACols = 3 * kKT / 2;   // TMEM columns of an A stage (three planes)
 constexpr int kD2tConv = 1;    // first converter warp
-constexpr int kD2tEpi = kD2tConv + 8 * kD2tSets;   // first epilogue warp
+constexpr int kD2tEpi = kD2tConv + 8;              // first epilogue warp
 constexpr int kD2tMma = kD2tEpi + 4;               // the MMA warp
 constexpr int kD2tThreads = 32 * (kD2tMma + 1);
+// A stages of KT = nmpad / 16
+__host__ __device__ constexpr int d2m_a_stages(int KT) {
+    const int n = (512 - 6 * 16 * KT) / kACols;
+    return n < kTA ? n : kTA;
+}
 
-// STACK: the three B planes are interleaved along N ([hi; mid; lo] rows per K column), so that one MMA of
-// N = 3 nmpad takes hi x {hi, mid, lo}, one of N = 2 nmpad mid x {hi, mid} and one of N = nmpad lo x hi: each A
-// plane is read from shared memory once per K step instead of once per product.  The accumulator of a tile
-// holds three column groups (the hi x hi product, the 2^-8 products, the 2^-16 products), summed by the epilogue.
-template <int KT, bool STACK>
+template <int KT>
 __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_constant__ CUtensorMap psi_map,
                                                       const int* __restrict__ active,
                                                       const __nv_bfloat16* __restrict__ Dw, const double* xin,
                                                       double alpha, double beta, double* out, long long NENK, int NI,
                                                       int NIpad, int nm, int nmpad, long long ntiles, int* err) {
     if (active && *active == 0) return;
+    constexpr int NS = d2m_a_stages(KT);
+    static_assert(NS >= 2, "two A stages");
     extern __shared__ __align__(1024) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int NKpad = (NIpad + kKT - 1) / kKT * kKT;
     const size_t bplane = (size_t)nmpad * NKpad * 2;
-    const size_t aplane = (size_t)kTM * kKT * 2;
-    const size_t abuf = ((3 * aplane + 1023) / 1024) * 1024;
     constexpr size_t fbuf = (size_t)kTM * kKT * 4;                       // one FP32 stage
     unsigned char* sB = sm;
     unsigned char* sF = sm + ((3 * bplane + 1023) / 1024) * 1024;       // [kT32] FP32 stages
-    unsigned char* sA = sF + kT32 * fbuf;                                // [kTA] A stages
-    uint64_t* tfull = reinterpret_cast<uint64_t*>(sA + kTA * abuf);      // [kT32]
+    uint64_t* tfull = reinterpret_cast<uint64_t*>(sF + kT32 * fbuf);     // [kT32]
     uint64_t* tempty = tfull + kT32;                                     // [kT32]
     uint64_t* afull = tempty + kT32;                                     // [kTA]
     uint64_t* adone = afull + kTA;                                       // [kTA]
     uint64_t* dfull = adone + kTA;                                       // [2]
     uint64_t* dempty = dfull + 2;                                        // [2]
     uint32_t* tslot = reinterpret_cast<uint32_t*>(dempty + 2);
-    {   // B = Dw planes [3][nmpad][NIpad] staged K-major: rows = moments, K = directions
+    {   // B = Dw planes [3][nmpad][NIpad] staged K-major: rows = moments of the three planes, K = directions
         const int cc = NKpad / 8;
         const int total = 3 * nmpad * cc;
         for (int u = tid; u < total; u += blockDim.x) {
@@ -703,20 +725,17 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
             const int r = rem / cc, c = rem % cc;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (c * 8 < NIpad) v = __ldg(reinterpret_cast<const uint4*>(Dw + ((size_t)p * nmpad + r) * NIpad) + c);
-            if (STACK)
-                *reinterpret_cast<uint4*>(sB + (size_t)c * 3 * nmpad * 16 + (size_t)(p * nmpad + r) * 16) = v;
-            else
-                *reinterpret_cast<uint4*>(sB + p * bplane + (size_t)c * nmpad * 16 + (size_t)r * 16) = v;
+            *reinterpret_cast<uint4*>(sB + (size_t)c * 3 * nmpad * 16 + (size_t)(p * nmpad + r) * 16) = v;
         }
     }
-    // TMEM columns per tile buffer: two groups of up to 64 (leading, corrections), or three of nmpad (STACK)
-    constexpr uint32_t kBufCols = STACK ? 256u : 128u;
+    constexpr uint32_t kBufCols = 3 * 16 * KT;   // accumulator columns of a tile buffer
+    constexpr uint32_t kA0 = 2 * kBufCols;       // first column of the A stages
     if (tid == 0) {
         for (int k = 0; k < kT32; ++k) {
             bar_init(&tfull[k], 1);
             bar_init(&tempty[k], 256);
         }
-        for (int k = 0; k < kTA; ++k) {
+        for (int k = 0; k < NS; ++k) {
             bar_init(&afull[k], 256);
             bar_init(&adone[k], 1);
         }
@@ -725,7 +744,7 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
             bar_init(&dempty[k], 128);
         }
     }
-    if (warp == kD2tMma) tmem_alloc(tslot, 2 * kBufCols);   // two tile buffers
+    if (warp == kD2tMma) tmem_alloc(tslot, 512);   // one CTA per SM
     fence_async_smem();
     tc_before_sync();
     __syncthreads();
@@ -737,24 +756,25 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
     if (warp == 0) {
         // ---- TMA issue ----
         if ((tid & 31) == 0) {
+            int s = 0, ch = 0;
+            uint32_t u = 0;
+            long long tile = blockIdx.x;
             for (long long c = 0; c < nch; ++c) {
-                const int s = (int)(c % kT32);
-                const uint32_t u = (uint32_t)(c / kT32);
                 if (u > 0 && !bar_wait(&tempty[s], (u - 1) & 1u, err)) break;
-                const long long tile = blockIdx.x + (c / nchunks) * gridDim.x;
-                const int ch = (int)(c % nchunks);
                 bar_expect_tx(&tfull[s], (uint32_t)fbuf);
                 tma_load_2d(sF + s * fbuf, &psi_map, (int)(tile * kTM), ch * kKT, &tfull[s]);
+                if (++s == kT32) { s = 0; ++u; }
+                if (++ch == nchunks) { ch = 0; tile += gridDim.x; }
             }
         }
     } else if (warp < kD2tEpi) {
-        // ---- converters: FP32 stage -> BF16 planes of the A stage; set `set` takes chunks c = set mod kD2tSets ----
-        const int t = tid - 32 * kD2tConv;
-        const int row = t & 127, side = (t >> 7) & 1, set = t >> 8;
-        for (long long c = set; c < nch; c += kD2tSets) {
-            const int s = (int)(c % kT32);
-            const int sa = (int)(c % kTA);
-            if (!bar_wait(&tfull[s], (uint32_t)(c / kT32) & 1u, err)) break;
+        // ---- converters: FP32 stage -> BF16 planes of the A stage ----
+        const int row = ((warp & 3) << 5) | (tid & 31), side = (warp - kD2tConv) >> 2;
+        const uint32_t a_lane = tmem + kA0 + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(side * 8);
+        int s = 0, sa = 0;
+        uint32_t u = 0, ua = 0;
+        for (long long c = 0; c < nch; ++c) {
+            if (!bar_wait(&tfull[s], u & 1u, err)) break;
             const float* F = reinterpret_cast<const float*>(sF + s * fbuf) + (size_t)(side * 16) * kTM + row;
             float v[16];
 #pragma unroll
@@ -762,23 +782,31 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
             // the stage is refilled by the TMA (async proxy): order these generic reads before that write
             fence_async_smem();
             bar_arrive(&tempty[s]);
-            const uint32_t ua = (uint32_t)(c / kTA);
-            if (ua > 0 && !bar_wait(&adone[sa], (ua - 1) & 1u, err)) break;
-            unsigned char* A = sA + sa * abuf;
+            uint4 hi[2], mid[2], lo[2];
 #pragma unroll
             for (int cl = 0; cl < 2; ++cl) {
                 float w[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) w[k] = v[cl * 8 + k];
-                uint4 hi, mid, lo;
-                split8(w, hi, mid, lo);
-                unsigned char* rp = A + (size_t)(side * 2 + cl) * kTM * 16 + (size_t)row * 16;
-                *reinterpret_cast<uint4*>(rp) = hi;
-                *reinterpret_cast<uint4*>(rp + aplane) = mid;
-                *reinterpret_cast<uint4*>(rp + 2 * aplane) = lo;
+                split8(w, hi[cl], mid[cl], lo[cl]);
             }
-            fence_async_smem();
+            if (ua > 0) {
+                if (!bar_wait(&adone[sa], (ua - 1) & 1u, err)) break;
+                tc_after_sync();
+            }
+            __syncwarp();
+            const uint32_t at = a_lane + (uint32_t)(sa * kACols);
+#pragma unroll
+            for (int cl = 0; cl < 2; ++cl) {
+                tmem_st4(at + cl * 4, hi[cl]);
+                tmem_st4(at + kKT / 2 + cl * 4, mid[cl]);
+                tmem_st4(at + kKT + cl * 4, lo[cl]);
+            }
+            tmem_st_wait();
+            tc_before_sync();
             bar_arrive(&afull[sa]);
+            if (++s == kT32) { s = 0; ++u; }
+            if (++sa == NS) { sa = 0; ++ua; }
         }
     } else if (warp < kD2tMma) {
         // ---- epilogue: a warp reads TMEM lanes 32(w%4).. (the hardware's lane quarter of warp w), i.e.
@@ -806,18 +834,13 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
             tc_after_sync();
 #pragma unroll
             for (int g = 0; g < KT; ++g) {
-                // the leading product's accumulator plus the correction products' accumulator(s) (IEEE FP32)
+                // the leading product's accumulator plus the correction products' accumulators (IEEE FP32)
                 float v[16], w[16];
-                if (STACK) {
-                    tmem_ld16(lane_base + (uint32_t)(b * kBufCols + nmpad + g * 16), w);
-                    tmem_ld16(lane_base + (uint32_t)(b * kBufCols + 2 * nmpad + g * 16), v);
+                tmem_ld16(lane_base + (uint32_t)(b * kBufCols + nmpad + g * 16), w);
+                tmem_ld16(lane_base + (uint32_t)(b * kBufCols + 2 * nmpad + g * 16), v);
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) w[k] += v[k];
-                    tmem_ld16(lane_base + (uint32_t)(b * kBufCols + g * 16), v);
-                } else {
-                    tmem_ld16(lane_base + (uint32_t)(b * kBufCols + g * 16), v);
-                    tmem_ld16(lane_base + (uint32_t)(b * kBufCols + 64 + g * 16), w);
-                }
+                for (int k = 0; k < 16; ++k) w[k] += v[k];
+                tmem_ld16(lane_base + (uint32_t)(b * kBufCols + g * 16), v);
 #pragma unroll
                 for (int k = 0; k < 16; ++k) v[k] += w[k];
                 if (valid) {
@@ -844,62 +867,47 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
         }
     } else if ((tid & 31) == 0) {
         // ---- MMA issue ----
-        const uint32_t idesc = idesc_bf16(kTM, nmpad);
-        const uint32_t lboA = kTM * 16, lboB = (uint32_t)nmpad * 16 * (STACK ? 3u : 1u);
-        const uint32_t aBase = smem_u32(sA), bBase = smem_u32(sB);
-        long long c = 0;
-        int it = 0;
+        constexpr uint32_t i1 = idesc_bf16(kTM, 16 * KT), i2 = idesc_bf16(kTM, 32 * KT), i3 = idesc_bf16(kTM, 48 * KT);
+        const uint32_t lboB = (uint32_t)nmpad * 48u;
+        const uint32_t bBase = smem_u32(sB);
+        int it = 0, sa = 0;
+        uint32_t ua = 0;
         bool ok = true;
         for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
             const int b = it & 1;
             const uint32_t ut = (uint32_t)(it >> 1);
             if (ut > 0 && !bar_wait(&dempty[b], (ut - 1) & 1u, err)) break;
-            for (int ch = 0; ch < nchunks; ++ch, ++c) {
-                const int sa = (int)(c % kTA);
-                if (!bar_wait(&afull[sa], (uint32_t)(c / kTA) & 1u, err)) {
+            for (int ch = 0; ch < nchunks; ++ch) {
+                if (!bar_wait(&afull[sa], ua & 1u, err)) {
                     ok = false;
                     break;
                 }
                 tc_after_sync();
-                const uint32_t a0 = aBase + sa * (uint32_t)abuf;
-                if (STACK) {
-                    // hi x [hi; mid; lo] -> groups 0, 1, 2; mid x [hi; mid] -> groups 1, 2; lo x hi -> group 2
-                    const uint32_t d0 = tmem + (uint32_t)b * kBufCols;
-                    for (int ks = 0; ks < kKT / 16; ++ks) {
-                        const uint64_t db = sdesc(bBase + (uint32_t)(ch * (kKT / 8) + ks * 2) * lboB, lboB, 128);
-                        const uint32_t ka = a0 + ks * 2 * lboA;
-                        mma_bf16_ss(d0, sdesc(ka, lboA, 128), db, idesc_bf16(kTM, 3 * nmpad), (ch | ks) ? 1u : 0u);
-                        mma_bf16_ss(d0 + nmpad, sdesc(ka + (uint32_t)aplane, lboA, 128), db, idesc_bf16(kTM, 2 * nmpad),
-                                    1u);
-                        mma_bf16_ss(d0 + 2 * nmpad, sdesc(ka + 2 * (uint32_t)aplane, lboA, 128), db, idesc, 1u);
-                    }
-                } else {
-                    for (int ks = 0; ks < kKT / 16; ++ks)
-                        for (int pr = 0; pr < 6; ++pr) {
-                            const uint64_t da = sdesc(a0 + kProdA[pr] * (uint32_t)aplane + ks * 2 * lboA, lboA, 128);
-                            const uint64_t db = sdesc(bBase + kProdB[pr] * (uint32_t)bplane +
-                                                          (uint32_t)(ch * (kKT / 8) + ks * 2) * lboB, lboB, 128);
-                            // product 5 (hi x hi) alone in columns b*128.., the five smaller ones in b*128 + 64..
-                            const bool lead = pr == 5;
-                            const uint32_t acc = lead ? (uint32_t)(ch | ks) : (uint32_t)(ch | ks | pr);
-                            mma_bf16_ss(tmem + b * kBufCols + (lead ? 0u : 64u), da, db, idesc, acc ? 1u : 0u);
-                        }
+                const uint32_t a0 = tmem + kA0 + (uint32_t)(sa * kACols);
+                // hi x [hi; mid; lo] -> groups 0, 1, 2; mid x [hi; mid] -> groups 1, 2; lo x hi -> group 2
+                const uint32_t d0 = tmem + (uint32_t)b * kBufCols;
+                for (int ks = 0; ks < kKT / 16; ++ks) {
+                    const uint64_t db = sdesc(bBase + (uint32_t)(ch * (kKT / 8) + ks * 2) * lboB, lboB, 128);
+                    const uint32_t ka = a0 + ks * 8;
+                    mma_bf16_ts(d0, ka, db, i3, (ch | ks) ? 1u : 0u);
+                    mma_bf16_ts(d0 + nmpad, ka + kKT / 2, db, i2, 1u);
+                    mma_bf16_ts(d0 + 2 * nmpad, ka + kKT, db, i1, 1u);
                 }
                 mma_commit(&adone[sa]);
                 if (ch == nchunks - 1) mma_commit(&dfull[b]);
+                if (++sa == NS) { sa = 0; ++ua; }
             }
         }
     }
     tc_before_sync();
     __syncthreads();
-    if (warp == kD2tMma) tmem_free(tmem, 2 * kBufCols);
+    if (warp == kD2tMma) tmem_free(tmem, 512);
 }
 
 size_t d2m_tma_smem(int NIpad, int nmpad) {
     const int NKpad = (NIpad + kKT - 1) / kKT * kKT;
     const size_t b = ((3 * (size_t)nmpad * NKpad * 2 + 1023) / 1024) * 1024;
-    const size_t a = ((3 * (size_t)kTM * kKT * 2 + 1023) / 1024) * 1024;
-    return b + kT32 * (size_t)kTM * kKT * 4 + kTA * a + 8 * (2 * kT32 + 2 * kTA + 4) + 16;
+    return b + kT32 * (size_t)kTM * kKT * 4 + 8 * (2 * kT32 + 2 * kTA + 4) + 16;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
@@ -955,15 +963,6 @@ bool moments_tma_enabled() {
         on = (e && *e == '0') ? 0 : 1;
     }
     return on == 1;
-}
-
-// D2M's B planes stacked along N, three MMAs per K step (LB_D2M_STACK=0: six MMAs, one per product).
-bool d2m_stack_enabled() {
-    static const bool on = [] {
-        const char* e = std::getenv("LB_D2M_STACK");
-        return !(e && *e == '0');
-    }();
-    return on;
 }
 
 // M2D's output written by TMA stores (LB_M2D_TMA_STORE=0: per-thread stores).
@@ -1071,6 +1070,7 @@ int launch_d2m_tma(Handle* h, const float* psi, const double* xin, double alpha,
     if (h->nmpad > 64 || h->nmpad % 16 || h->NIpad % 8 || ((uintptr_t)psi & 15) || (h->NENK * 4) % 16 ||
         h->NENK >= (1LL << 31) || h->NI < 1)
         return LB_ERR_ARG;
+    // (B planes of up to 98 KB fit beside the stages; wider quadratures take the register-fed kernel)
     const size_t smem = std::max<size_t>(d2m_tma_smem(h->NIpad, h->nmpad), 116 * 1024);
     if (smem > 227 * 1024) return LB_ERR_ARG;
     int* err = h->d_tc_err;
@@ -1087,24 +1087,17 @@ int launch_d2m_tma(Handle* h, const float* psi, const double* xin, double alpha,
         return LB_ERR_ARG;
     static PerDevice attr;
     attr.get([&] {
-#define LB_D2MATTR(K, S) cudaFuncSetAttribute(d2m_tma_kernel<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
-        LB_D2MATTR(1, false); LB_D2MATTR(2, false); LB_D2MATTR(3, false); LB_D2MATTR(4, false);
-        LB_D2MATTR(1, true); LB_D2MATTR(2, true); LB_D2MATTR(3, true); LB_D2MATTR(4, true);
+#define LB_D2MATTR(K) cudaFuncSetAttribute(d2m_tma_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
+        LB_D2MATTR(1); LB_D2MATTR(2); LB_D2MATTR(3); LB_D2MATTR(4);
 #undef LB_D2MATTR
         return 1;
     });
     const long long ntiles = (h->NENK + kTM - 1) / kTM;
     const long long grid = std::min<long long>(ntiles, (long long)h->sm_count);
-    const bool stack = d2m_stack_enabled();
-#define LB_D2MTMA(K)                                                                                                    \
-    if (stack)                                                                                                          \
-        d2m_tma_kernel<K, true><<<(int)grid, kD2tThreads, smem, h->stream>>>(map, h->d_active, h->d_Yd2m, xin, alpha,   \
-                                                                           beta, out, h->NENK, h->NI, h->NIpad, h->nm, \
-                                                                           h->nmpad, ntiles, err);                     \
-    else                                                                                                                \
-        d2m_tma_kernel<K, false><<<(int)grid, kD2tThreads, smem, h->stream>>>(map, h->d_active, h->d_Yd2m, xin, alpha,  \
-                                                                            beta, out, h->NENK, h->NI, h->NIpad, h->nm, \
-                                                                            h->nmpad, ntiles, err)
+#define LB_D2MTMA(K)                                                                                                   \
+    d2m_tma_kernel<K><<<(int)grid, kD2tThreads, smem, h->stream>>>(map, h->d_active, h->d_Yd2m, xin, alpha, beta, out, \
+                                                                  h->NENK, h->NI, h->NIpad, h->nm, h->nmpad, ntiles, \
+                                                                  err)
     switch (h->nmpad / 16) {
         case 1: LB_D2MTMA(1); break;
         case 2: LB_D2MTMA(2); break;
