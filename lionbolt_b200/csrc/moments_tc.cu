@@ -206,24 +206,33 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
 
 // ---------------------------------------------------------------------------------------------
 // M2D: q[i][n] = sum_j Y[i][j] xt[j][n] (+ qadd[i][n]),  xt[j][n] = sigl[mat(n)][j] x[j][n] + a[j][n].
-// One CTA per SM, warp-specialised, directions [half*NH, half*NH + NH) of every tile it takes:
+// One CTA per SM, warp-specialised, directions [half*NH, half*NH + NH) of every tile it takes (nhalves parts of the
+// directions, so that both accumulators and both A buffers fit the 512 TMEM columns):
 //   warps 0-7   producers: threads t and t + 128 read node tile*128 + (t & 127), half of its moments
-//               each, split them into BF16 planes and write the A buffer (two buffers);
+//               each, split them into BF16 planes and write the A buffer (in tensor memory, where the node is the
+//               lane of its warp's quarter; na = 2 buffers, or 1 where two do not fit);
 //   warps 8-19  epilogue: warps 8+e, 12+e and 16+e read TMEM lanes 32e.. (the tile's nodes), a third
 //               of the direction columns each, and write q rows (two accumulators);
 //   warp 20     lane 0 issues the MMAs; the warp owns the TMEM allocation.
 // Barriers per buffer b: full[b] (producers -> MMA), done[b] (MMA commit -> producers, epilogue),
 // empty[b] (epilogue -> MMA).  The k-th use of a buffer waits on phase parity k & 1.
+// With the A buffers in shared memory a tile half moved 450 KB through it (moments in and out 74 KB, A written once
+// and read by six products 110 KB, B 83 KB, the output staged 147 KB): 3,500 of its 5,400 clocks at 288 directions and
+// P5.  A in tensor memory leaves 300 KB.  At 3,072,000 nodes a first call fell from 1.00 to 0.96 ms; repeated without
+// a pause the chip's power limit holds the clock down and it is 1.029 ms against 1.051.  168 directions at P7 (192,000
+// nodes): 67 us against 81, since one part of the directions now holds them all; 288 at P7: 100 against 128.
 // ---------------------------------------------------------------------------------------------
 constexpr int kM2dEpi = 12;                          // epilogue warps (three per TMEM lane quarter)
 constexpr int kM2dMma = 8 + kM2dEpi;                 // the MMA warp
 constexpr int kM2dThreads = 32 * (kM2dMma + 1);
 constexpr int kM2dTma = kM2dMma + 1;                 // MODE 2: the warp whose lane 0 loads the moment tiles
 constexpr int kM2dThreadsTma = 32 * (kM2dTma + 1);
+// MODE 2: stages of the moment ring.  Two: more in flight only takes the write stream's place (128 directions, P3,
+// 648,000 nodes: 2 stages 89.1 us, 3 and 8 stages 94.3; 32 directions, P1: 21.8 against 23.5).
+constexpr int kM2dX = 2;
 
 // MODE 0: per-thread output stores; 1: TMA output stores (two staging buffers per epilogue warp); 2: TMA
-// output stores (one buffer per warp) and the moment tiles x[0..nm)[128 nodes] brought into a two-stage
-// shared-memory ring by TMA, from which the producers read (nodes past NENK arrive as zeros).
+// output stores and the moment tiles x[0..nm)[128 nodes] brought into a shared-memory ring by TMA, from which the producers read (nodes past NENK arrive as zeros).
 template <int KT, int MODE>
 __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m2d_tc_kernel(
                                                       const __grid_constant__ CUtensorMap q_map,
@@ -233,27 +242,26 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                                                       const float* __restrict__ qadd, const int* __restrict__ mat,
                                                       const __nv_bfloat16* __restrict__ Y, float* __restrict__ q,
                                                       long long NENK, int NI, int NIpad, int nm, int nmpad, int NH,
-                                                      int nhalves, long long ntiles, int* err) {
+                                                      int nhalves, int na, long long ntiles, int* err) {
     if (active && *active == 0) return;
     extern __shared__ __align__(1024) unsigned char sm[];
     constexpr int NMP = KT * 16;
     const int tid = threadIdx.x, warp = tid >> 5;
     const size_t bplane = (size_t)NH * nmpad * 2;
-    const size_t aplane = (size_t)kTM * nmpad * 2;
-    const size_t abuf = ((3 * aplane + 1023) / 1024) * 1024;
     unsigned char* sB = sm;
-    unsigned char* sA = sm + ((3 * bplane + 1023) / 1024) * 1024;   // [2] buffers of 3 planes
-    uint64_t* full = reinterpret_cast<uint64_t*>(sA + 2 * abuf);
+    unsigned char* sT = sm + ((3 * bplane + 1023) / 1024) * 1024;
+    uint64_t* full = reinterpret_cast<uint64_t*>(sT);
     uint64_t* done = full + 2;
     uint64_t* empty = full + 4;
-    uint64_t* xfull = full + 6;     // MODE 2: [2] moment stages loaded
-    uint64_t* xempty = full + 8;    // MODE 2: [2] moment stages read
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 10);
+    uint64_t* xfull = full + 6;              // MODE 2: [kM2dX] moment stages loaded
+    uint64_t* xempty = xfull + kM2dX;        // MODE 2: [kM2dX] moment stages read
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(xempty + kM2dX);
     // MODE >= 1: per epilogue warp NB 2 KB staging buffers [16 directions][32 nodes] for the TMA stores
-    constexpr int NB = MODE == 2 ? 1 : 2;
-    float* sS = reinterpret_cast<float*>(sA + 2 * abuf + 1024);
-    const size_t xbuf = (size_t)kTM * nm * 8;                                    // MODE 2: one moment stage
-    unsigned char* sX = sA + 2 * abuf + 1024 + (size_t)kM2dEpi * NB * 2048;       // MODE 2: [2] stages
+    constexpr int NB = 2;
+    float* sS = reinterpret_cast<float*>(sT + 1024);
+    const size_t xbuf = (size_t)kTM * nm * 8;                           // MODE 2: one moment stage
+    unsigned char* sX = sT + 1024 + (size_t)kM2dEpi * NB * 2048;         // MODE 2: [kM2dX] stages
+    const uint32_t acols = 3u * NMP / 2;                                // TMEM columns of an A buffer
     const int half = blockIdx.x % nhalves;
     stage_kmajor(Y, NIpad, nmpad, half * NH, NH, sB, bplane);
     if (tid == 0) {
@@ -263,7 +271,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             bar_init(&empty[k], 32 * kM2dEpi);
         }
         if (MODE == 2)
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < kM2dX; ++k) {
                 bar_init(&xfull[k], 1);
                 bar_init(&xempty[k], 256);
             }
@@ -280,12 +288,14 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
         constexpr int HM = NMP / 2;
         const int r = tid & 127, side = tid >> 7;
         const double* src = x ? x : add;
+        const uint32_t a_lane = tmem + 2u * NH + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(side * (HM / 2));
+        int xs = 0;
+        uint32_t xu = 0;
         // the node's material (it selects the sigma row) is loaded one tile ahead, off the tile's load chain
         int m_next = (t0 * kTM + r < NENK) ? __ldg(&mat[(t0 * kTM + r) >> 2]) : 0;
         int it = 0;
         for (long long tile = t0; tile < ntiles; tile += tstep, ++it) {
             const int b = it & 1;
-            const uint32_t u = (uint32_t)(it >> 1);
             const long long n = tile * kTM + r;
             const bool valid = n < NENK;
             const int m = valid ? m_next : 0;
@@ -297,14 +307,14 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             if (MODE == 2) {
                 // the tile's moments from the stage, then the stage back to the TMA: the proxy fence orders
                 // these generic reads before its next (async-proxy) write into the stage
-                const int xs = it & 1;
-                if (!bar_wait(&xfull[xs], (uint32_t)(it >> 1) & 1u, err)) break;
+                if (!bar_wait(&xfull[xs], xu & 1u, err)) break;
                 const double* X = reinterpret_cast<const double*>(sX + xs * xbuf) + (size_t)(side * HM) * kTM + r;
                 const int jn = nm - side * HM;
 #pragma unroll
                 for (int k = 0; k < HM; ++k) raw[k] = k < jn ? X[(size_t)k * kTM] : 0.0;
                 fence_async_smem();
                 bar_arrive(&xempty[xs]);
+                if (++xs == kM2dX) { xs = 0; ++xu; }
             } else {
                 // one pointer stepped by a row (NENK) per moment instead of a 64-bit index per load
                 const double* sp = src + (size_t)(side * HM) * (size_t)NENK + (valid ? n : 0);
@@ -315,8 +325,12 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                     sp += NENK;
                 }
             }
-            if (u > 0 && !bar_wait(&done[b], (u - 1) & 1u, err)) break;
-            unsigned char* A = sA + b * abuf;
+            if (it >= na) {   // the A buffer's last use, tile it - na
+                if (!bar_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err)) break;
+                tc_after_sync();
+            }
+            __syncwarp();
+            const uint32_t at = a_lane + (na == 2 ? b : 0) * acols;
             // this half's sigma_l(j) row of the node's material (the table is padded to nmpad with zeros, and
             // raw[] is zero past the moments that exist, so no per-value bounds test is needed)
             const float* sg = sigl + (size_t)m * nmpad + side * HM;
@@ -337,12 +351,12 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                 }
                 uint4 hi, mid, lo;
                 split8(v, hi, mid, lo);
-                unsigned char* row = A + (size_t)(side * (HM / 8) + cl) * kTM * 16 + (size_t)r * 16;
-                *reinterpret_cast<uint4*>(row) = hi;
-                *reinterpret_cast<uint4*>(row + aplane) = mid;
-                *reinterpret_cast<uint4*>(row + 2 * aplane) = lo;
+                tmem_st4(at + cl * 4, hi);
+                tmem_st4(at + NMP / 2 + cl * 4, mid);
+                tmem_st4(at + NMP + cl * 4, lo);
             }
-            fence_async_smem();
+            tmem_st_wait();
+            tc_before_sync();
             bar_arrive(&full[b]);
         }
     } else if (warp < kM2dMma) {
@@ -365,14 +379,13 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             const bool valid = n < NENK;
             for (int g = g0; g < g1; ++g) {
                 float v[16];
-                tmem_ld16(lane_base + (uint32_t)(b * 256 + g * 16), v);
+                tmem_ld16(lane_base + (uint32_t)(b * NH + g * 16), v);
                 if (MODE >= 1) {
                     // the warp's 32 nodes x 16 directions through shared memory and one TMA store (nodes past
                     // NENK and directions past NI lie outside the tensor and are not written)
                     float* st = stage + sidx * 512;
                     if (lane == 0) {
-                        if (NB == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     }
                     __syncwarp();
 #pragma unroll
@@ -415,8 +428,8 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     } else if (warp == kM2dMma && (tid & 31) == 0) {
         // ---- MMA issue ----
         const uint32_t idesc = idesc_bf16(kTM, NH);
-        const uint32_t lboA = kTM * 16, lboB = (uint32_t)NH * 16;
-        const uint32_t aBase = smem_u32(sA), bBase = smem_u32(sB);
+        const uint32_t lboB = (uint32_t)NH * 16;
+        const uint32_t bBase = smem_u32(sB);
         int it = 0;
         for (long long tile = t0; tile < ntiles; tile += tstep, ++it) {
             const int b = it & 1;
@@ -424,23 +437,23 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             if (!bar_wait(&full[b], u & 1u, err)) break;
             if (u > 0 && !bar_wait(&empty[b], (u - 1) & 1u, err)) break;
             tc_after_sync();
-            const uint32_t a0 = aBase + b * (uint32_t)abuf;
+            const uint32_t a0 = tmem + 2u * NH + (na == 2 ? b : 0) * acols;
             for (int ks = 0; ks < KT; ++ks)
                 for (int pr = 0; pr < 6; ++pr) {
-                    const uint64_t da = sdesc(a0 + kProdA[pr] * (uint32_t)aplane + ks * 2 * lboA, lboA, 128);
                     const uint64_t db = sdesc(bBase + kProdB[pr] * (uint32_t)bplane + ks * 2 * lboB, lboB, 128);
-                    mma_bf16_ss(tmem + b * 256, da, db, idesc, (ks | pr) ? 1u : 0u);
+                    mma_bf16_ts(tmem + b * NH, a0 + kProdA[pr] * (NMP / 2) + ks * 8, db, idesc, (ks | pr) ? 1u : 0u);
                 }
             mma_commit(&done[b]);
         }
     } else if (MODE == 2 && warp == kM2dTma && (tid & 31) == 0) {
-        // ---- moment tiles by TMA, up to two ahead of the producers ----
-        int it = 0;
-        for (long long tile = t0; tile < ntiles; tile += tstep, ++it) {
-            const int xs = it & 1;
-            if (it >= 2 && !bar_wait(&xempty[xs], (uint32_t)((it >> 1) - 1) & 1u, err)) break;
+        // ---- moment tiles by TMA, up to kM2dX ahead of the producers ----
+        int xs = 0;
+        uint32_t xu = 0;
+        for (long long tile = t0; tile < ntiles; tile += tstep) {
+            if (xu > 0 && !bar_wait(&xempty[xs], (xu - 1) & 1u, err)) break;
             bar_expect_tx(&xfull[xs], (uint32_t)xbuf);
             tma_load_2d(sX + xs * xbuf, &x_map, (int)(tile * kTM), 0, &xfull[xs]);
+            if (++xs == kM2dX) { xs = 0; ++xu; }
         }
     }
     tc_before_sync();
@@ -929,12 +942,10 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-size_t m2d_tc_smem(int NH, int nmpad, int mode = 0, int nm = 0) {
-    const size_t b = ((3 * (size_t)NH * nmpad * 2 + 1023) / 1024) * 1024;
-    const size_t a = ((3 * (size_t)kTM * nmpad * 2 + 1023) / 1024) * 1024;
-    if (mode == 0) return b + 2 * a + 96;
-    if (mode == 1) return b + 2 * a + 1024 + (size_t)kM2dEpi * 2 * 2048;
-    return b + 2 * a + 1024 + (size_t)kM2dEpi * 2048 + 2 * (size_t)kTM * nm * 8;
+size_t m2d_tc_smem(int NH, int nmpad, int mode, int nm) {
+    const size_t b = ((3 * (size_t)NH * nmpad * 2 + 1023) / 1024) * 1024 + 1024;
+    if (mode == 0) return b;
+    return b + (size_t)kM2dEpi * 2 * 2048 + (mode == 2 ? kM2dX * (size_t)kTM * nm * 8 : 0);
 }
 
 size_t d2m_tc_smem(int NIpad, int nmpad) {
@@ -987,10 +998,15 @@ bool moments_tma_load_enabled() {
 
 // Returns LB_ERR_ARG when the shape does not fit the tensor-core kernels (caller falls back).
 int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a, const float* qadd, float* q) {
-    const int nhalves = h->NIpad > 256 ? 2 : 1;
-    const int NH = ((h->NIpad + nhalves - 1) / nhalves + 15) / 16 * 16;
-    if (NH > 256 || h->nmpad % 16 || h->nmpad > 64 || h->NIpad % 8) return LB_ERR_ARG;
-    // one CTA per SM (it holds all 512 TMEM columns: two accumulators of up to 256)
+    if (h->NIpad > 512 || h->nmpad % 16 || h->nmpad > 64 || h->NIpad % 8) return LB_ERR_ARG;
+    // parts of the directions such that two accumulators of NH columns and an A buffer of 3 nmpad / 2 fit the 512 TMEM
+    // columns (288 directions at P5: two parts of 144; the moments are then read twice, the second time from
+    // L2), and a second A buffer where it fits
+    int nhalves = 1, NH;
+    const int acols = 3 * h->nmpad / 2;
+    while (NH = ((h->NIpad + nhalves - 1) / nhalves + 15) / 16 * 16, NH > 256 || 2 * NH + acols > 512) ++nhalves;
+    const int na = 2 * NH + 2 * acols <= 512 ? 2 : 1;
+    // one CTA per SM (it holds all TMEM columns)
     int* err = h->d_tc_err;
     if (!err) return LB_ERR_STATE;
     // TMA stores of the output when there is no added source and a tensor map can be made
@@ -999,7 +1015,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
     CUtensorMap xmap;
     std::memset(&xmap, 0, sizeof(xmap));
     EncodeTiledFn enc = encode_tiled();
-    bool ts = enc && !qadd && moments_tma_store_enabled() && m2d_tc_smem(NH, h->nmpad, 1) <= 227 * 1024 &&
+    bool ts = enc && !qadd && moments_tma_store_enabled() && m2d_tc_smem(NH, h->nmpad, 1, h->nm) <= 227 * 1024 &&
               !((uintptr_t)q & 15) && h->NENK < (1LL << 31);
     if (ts) {
         const cuuint64_t dims[2] = {(cuuint64_t)h->NENK, (cuuint64_t)h->NI};
@@ -1011,7 +1027,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
     // the moment tiles by TMA as well, from whichever operand holds them (x, or the add operand when x is
-    // null: the group sources), not when both are given; the two stages must fit
+    // null: the group sources), not when both are given
     const double* src = x ? x : a;
     bool tl = ts && src && !(x && a) && moments_tma_load_enabled() && h->nm <= 256 &&
               m2d_tc_smem(NH, h->nmpad, 2, h->nm) <= 227 * 1024 && !((uintptr_t)src & 15);
@@ -1046,7 +1062,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
 #define LB_M2DTC(K, M)                                                                                              \
     m2d_tc_kernel<K, M><<<(int)grid, M == 2 ? kM2dThreadsTma : kM2dThreads, smem, h->stream>>>(                      \
         map, xmap, h->d_active, x, sigl, a, qadd, h->d_mat, h->d_Ym2d, q, h->NENK, h->NI, h->NIpad, h->nm, h->nmpad, \
-        NH, nhalves, ntiles, err)
+        NH, nhalves, na, ntiles, err)
 #define LB_M2DK(K)                           \
     if (mode == 2) LB_M2DTC(K, 2);           \
     else if (mode == 1) LB_M2DTC(K, 1);      \
