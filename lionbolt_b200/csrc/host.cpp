@@ -667,10 +667,15 @@ static void form_blocks(Handle* h, std::vector<int>& blk_elem, std::vector<int>&
 
 // Units per group of the block schedule: the sweep's CTA size (512 threads), LB_CLUSTER_GROUP=<n> for
 // another cap, 0 for uncapped groups (Kahn's levels).
-static int cluster_group_cap() {
+// The tile sweep takes two passes per group where a second CTA shares its SM (more directions than SMs): warps done
+// with the first pass start the second at once, so half as many barriers find slow warps (768,000 tets x 288
+// directions 3.02 -> 2.85 ms, 393,216 x 288 1.49 -> 1.41, 279,936 x 288 1.085 -> 1.029; caps of 1536 and 2048 gave 3.1).
+// With an SM to itself the CTA has nothing to run beside a part-filled second pass (161,280 x 128 0.433 -> 0.467 ms),
+// and the cluster kernel gains nothing (279,936 x 288 1.54 -> 1.59 ms).
+static int cluster_group_cap(const Handle* h) {
     const char* e = std::getenv("LB_CLUSTER_GROUP");
     if (e && *e) return std::max(0, std::atoi(e));
-    return 512;
+    return h->nxtype > 0 && h->sm_count > 0 && h->NI > h->sm_count ? 1024 : 512;
 }
 
 // Block schedule of every direction: units in groups (a group's units depend only on units of earlier
@@ -708,10 +713,10 @@ static int build_cluster_schedule(Handle* h) {
     std::vector<std::vector<int4>> crec(NI);
     std::vector<std::vector<int>> cstart(NI);
     bool cyclic = false;
-    // Units per group.  A group is one pass of the sweep CTA's threads between two barriers, so a group of
+    // Units per group.  A group is one or two passes of the sweep CTA's threads between two barriers, so a group of
     // Kahn's levels (all ready units) with more units than threads takes several passes, the last one part
     // empty; capped groups pack every pass (list scheduling: ready units wait at most until a pass has room).
-    const int cap = cluster_group_cap();
+    const int cap = cluster_group_cap(h);
 #pragma omp parallel reduction(|| : cyclic)
     {
         std::vector<int> lev(NE), unit(NE), ublk, pend, epend, dstart(NE + 1), ddst, cur, nxt, members, ord, waiting;
@@ -831,7 +836,7 @@ static int build_cluster_schedule(Handle* h) {
             cstart[i].clear();
             int ndone = 0;
             while (ndone < NE) {
-                // at most `cap` units per group (one per thread of the sweep CTA): the ready units past it wait
+                // at most `cap` units per group (one or two per thread of the sweep CTA): the ready units past it wait
                 // for the next group, ahead of the units that become ready now
                 rest.clear();
                 if (cap > 0 && (int)cur.size() > cap) {
