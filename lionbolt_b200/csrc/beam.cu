@@ -14,6 +14,13 @@
 // with the 4-point rule (barycentric a on the point's vertex, b on the others, weights 1/24 on the
 // reference tet) the projection M^-1 sum_q w_q N_k(q) phi_q is c_k = sqrt(5) phi_k + (1 - sqrt(5))/4
 // sum_q phi_q (point k nearest vertex k).
+//
+// Bound by the chain of a ray's steps (up to some 200 in a 40-hex-deep box) and the FP64 pipe: a step's four FP64
+// divisions cost as much as the rest.  So the exit face is chosen from FP32 quotients and only its own division is
+// done in FP64 (the same exit face and the same bits; all four where FP32 cannot order them), the four neighbours are
+// read with the planes and the cross section before the division, off the chain of the next step.  384,000 rays,
+// 5 x 5 cm beam in a 10 x 10 x 20 cm box: 0.215 -> 0.150 ms; four FP64 divisions side by side instead of one after
+// another took 0.267.
 #include "lb_internal.h"
 #include <cmath>
 #include <cstring>
@@ -42,6 +49,20 @@ struct BeamArgs {
     int NE;
     int max_steps;
 };
+
+__device__ __forceinline__ double4 ld_plane(const double4* p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ double pick4(const double (&v)[4], int i) {
+    return i < 2 ? (i ? v[1] : v[0]) : (i == 2 ? v[2] : v[3]);
+}
+
+// FP32 quotients of FP64 operands rounded to FP32 are within 2^-24 + 2^-24 + 2 ulp < 4e-7 of the FP64 ones: two that
+// differ by more than this relative to their magnitudes are ordered as the FP64 ones.
+constexpr float kNear = 2e-6f;
 
 __global__ void __launch_bounds__(256) beam_uncollided_kernel(BeamArgs a) {
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -80,31 +101,54 @@ __global__ void __launch_bounds__(256) beam_uncollided_kernel(BeamArgs a) {
                 dy *= il;
                 dz *= il;
                 int cur = e, steps = 0;
+                const int4* nbr4 = reinterpret_cast<const int4*>(a.nbr);
                 while (cur >= 0) {
-                    // exit face: the nearest face plane ahead of the ray
-                    double tmin = 1e300;
+                    // exit face: the nearest face plane ahead of the ray, found with FP32 quotients; the FP64 quotient of
+                    // that face alone, or of all where two are too close to tell
+                    const int4 nb = __ldg(nbr4 + cur);
+                    const int m = __ldg(&a.mat[cur]);
+                    double num[4], den[4], tmin = 1e300;
+                    float ta[4], amin = INFINITY;
                     int fexit = -1;
 #pragma unroll
                     for (int f = 0; f < 4; ++f) {
-                        const double4 pl = a.plane[4 * cur + f];
-                        const double den = pl.x * dx + pl.y * dy + pl.z * dz;
-                        if (den > 0.0) {
-                            const double t = (pl.w - (pl.x * x + pl.y * y + pl.z * z)) / den;
-                            if (t < tmin) {
-                                tmin = t;
-                                fexit = f;
-                            }
+                        const double4 pl = ld_plane(a.plane + 4 * (size_t)cur + f);
+                        den[f] = pl.x * dx + pl.y * dy + pl.z * dz;
+                        num[f] = pl.w - (pl.x * x + pl.y * y + pl.z * z);
+                        ta[f] = den[f] > 0.0 ? __fdividef((float)num[f], (float)den[f]) : INFINITY;
+                        if (ta[f] < amin) {
+                            amin = ta[f];
+                            fexit = f;
                         }
+                    }
+                    bool sure = fexit >= 0 && amin > -INFINITY;
+#pragma unroll
+                    for (int f = 0; f < 4; ++f)
+                        if (f != fexit && den[f] > 0.0) sure = sure && ta[f] - amin > kNear * (fabsf(ta[f]) + fabsf(amin));
+                    const double sig = __ldg(&a.attn[m]);
+                    if (sure) {
+                        tmin = pick4(num, fexit) / pick4(den, fexit);
+                    } else {
+                        fexit = -1;
+#pragma unroll
+                        for (int f = 0; f < 4; ++f)
+                            if (den[f] > 0.0) {
+                                const double t = num[f] / den[f];
+                                if (t < tmin) {
+                                    tmin = t;
+                                    fexit = f;
+                                }
+                            }
                     }
                     if (fexit < 0) break;
                     const double seg = fmin(fmax(tmin, 0.0), remaining);
-                    tau = fma(__ldg(&a.attn[__ldg(&a.mat[cur])]), seg, tau);
+                    tau = fma(sig, seg, tau);
                     remaining -= seg;
                     if (remaining <= 0.0) break;
                     x = fma(seg, dx, x);
                     y = fma(seg, dy, y);
                     z = fma(seg, dz, z);
-                    cur = __ldg(&a.nbr[4 * cur + fexit]);
+                    cur = fexit < 2 ? (fexit ? nb.y : nb.x) : (fexit == 2 ? nb.z : nb.w);
                     if (++steps > a.max_steps) {
                         *a.stuck = 1;
                         tau = 0.0;

@@ -57,6 +57,19 @@ def test_oblique_beam_on_a_two_material_box_matches_oracle(theta):
     assert np.abs(gpu - ref).max() < ATOL
 
 
+@pytest.mark.parametrize("theta,phi", [(0.0, 0.0), (45.0, 0.0), (54.735610317245346, 45.0)])
+def test_beam_along_the_edges_of_the_tets_matches_oracle(theta, phi):
+    """Along an axis, a face diagonal and the hexes' main diagonal rays run parallel to faces and meet others in one
+    point: the exit face is then decided by the FP64 quotients, not by the FP32 ones."""
+    prob = P.config1_small(n=(6, 6, 12))
+    axis, e1, e2 = _frame(theta, phi)
+    args = (np.array([10.0, 10.0, 20.0]) - 40.0 * axis, axis, e1, e2, 9.0, 7.0, [0.11, 0.297])
+    gpu = _op(prob.mesh).beam_uncollided(*args)
+    ref = O.Oracle(prob.mesh).beam_uncollided(*args)
+    assert 500 < np.count_nonzero(ref) < ref.size
+    assert np.abs(gpu - ref).max() < ATOL
+
+
 def test_reference_het_cube_mesh_matches_oracle():
     m = golden_mesh("het_cube_spherical_beam")                   # unit cube, 78,771 tets, 2 materials
     axis, e1, e2 = _frame(25.0, 40.0)
