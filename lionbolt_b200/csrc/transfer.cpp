@@ -36,6 +36,16 @@ Handle::Pipe* pipe_for(Handle* h, size_t bytes) {
             else p.buf[b] = reinterpret_cast<char*>(h->h_red + kRedHost) + b * kPipeSmall;
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p.ev[b], cudaEventDisableTiming);
         }
+        if (e != cudaSuccess && large) {
+            // no pinned memory for the large pair: the handle's own small one, in more chunks
+            for (int b = 0; b < 2; ++b) {
+                if (p.buf[b]) cudaFreeHost(p.buf[b]);
+                if (p.ev[b]) cudaEventDestroy(p.ev[b]);
+            }
+            p = Handle::Pipe{};
+            cudaGetLastError();
+            return pipe_for(h, 0);
+        }
         if (e != cudaSuccess) {
             pipe_free(h);
             cuda_fail(h, e, "transfer buffers");
