@@ -263,6 +263,20 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     unsigned char* sX = sT + 1024 + (size_t)kM2dEpi * NB * 2048;         // MODE 2: [kM2dX] stages
     const uint32_t acols = 3u * NMP / 2;                                // TMEM columns of an A buffer
     const int half = blockIdx.x % nhalves;
+    const long long t0 = blockIdx.x / nhalves, tstep = gridDim.x / nhalves;
+    if (MODE == 2 && tid == 32 * kM2dTma) {
+        // the first moment tiles are on their way while the B planes are staged below (48,672 nodes, 168 directions, P3:
+        // 17.5 us against 19.0; the same in D2M, whose ring is deeper, gained nothing)
+        for (int k = 0; k < kM2dX; ++k) {
+            bar_init(&xfull[k], 1);
+            bar_init(&xempty[k], 256);
+        }
+        fence_async_smem();
+        for (int k = 0; k < kM2dX && t0 + k * tstep < ntiles; ++k) {
+            bar_expect_tx(&xfull[k], (uint32_t)xbuf);
+            tma_load_2d(sX + k * xbuf, &x_map, (int)((t0 + k * tstep) * kTM), 0, &xfull[k]);
+        }
+    }
     stage_kmajor(Y, NIpad, nmpad, half * NH, NH, sB, bplane);
     if (tid == 0) {
         for (int k = 0; k < 2; ++k) {
@@ -270,11 +284,6 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             bar_init(&done[k], 1);
             bar_init(&empty[k], 32 * kM2dEpi);
         }
-        if (MODE == 2)
-            for (int k = 0; k < kM2dX; ++k) {
-                bar_init(&xfull[k], 1);
-                bar_init(&xempty[k], 256);
-            }
     }
     if (warp == kM2dMma) tmem_alloc(tslot, 512);
     fence_async_smem();
@@ -282,7 +291,6 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     __syncthreads();
     tc_after_sync();
     const uint32_t tmem = *tslot;
-    const long long t0 = blockIdx.x / nhalves, tstep = gridDim.x / nhalves;
     if (warp < 8) {
         // ---- producers: threads t and t + 128 share node tile*128 + (t & 127), each half the moments ----
         constexpr int HM = NMP / 2;
@@ -448,9 +456,9 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     } else if (MODE == 2 && warp == kM2dTma && (tid & 31) == 0) {
         // ---- moment tiles by TMA, up to kM2dX ahead of the producers ----
         int xs = 0;
-        uint32_t xu = 0;
-        for (long long tile = t0; tile < ntiles; tile += tstep) {
-            if (xu > 0 && !bar_wait(&xempty[xs], (xu - 1) & 1u, err)) break;
+        uint32_t xu = 1;
+        for (long long tile = t0 + kM2dX * tstep; tile < ntiles; tile += tstep) {
+            if (!bar_wait(&xempty[xs], (xu - 1) & 1u, err)) break;
             bar_expect_tx(&xfull[xs], (uint32_t)xbuf);
             tma_load_2d(sX + xs * xbuf, &x_map, (int)(tile * kTM), 0, &xfull[xs]);
             if (++xs == kM2dX) { xs = 0; ++xu; }
