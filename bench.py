@@ -379,7 +379,9 @@ def real_sh(Ls, dirs):
 
 
 # kernel of each sweep schedule the autotuner can pick
-SWEEP_KERNELS = {"cluster levels": "sweep_cluster_kernel", "cluster levels+type tables": "sweep_cluster_kernel",
+SWEEP_KERNELS = {"block tiles": "sweep_tile_kernel", "level relay": "sweep_relay_kernel",
+                 "resident level relay": "sweep_relay_kernel",
+                 "cluster levels": "sweep_cluster_kernel", "cluster levels+type tables": "sweep_cluster_kernel",
                  "cluster levels+element prefetch": "sweep_cluster_kernel",
                  "cluster levels+element prefetch+previous in registers": "sweep_cluster_kernel",
                  "cluster levels+element prefetch+two previous in registers": "sweep_cluster_kernel",
