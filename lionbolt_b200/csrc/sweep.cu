@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_cluster_kernel(SweepArgs a) {
 //    indices of a face are the same in every tet up to one swap: no selection by index.
 // The next pass's record and sources are requested before the barrier that ends a group: no other thread
 // writes them.  Element arithmetic as in the other schedules (bit-identical results).
-// Measured per sweep, cluster kernel -> this one: 768,000 tets x 288 directions 4.15 -> 3.03 ms, 96,000 x 288
+// Measured per sweep, cluster kernel -> this one: 768,000 tets x 288 directions 4.15 -> 2.85 ms, 96,000 x 288
 // 0.647 -> 0.424, 57,456 x 288 0.489 -> 0.301, 24,480 x 168 0.246 -> 0.174, 6,000 x 80 0.105 -> 0.089 (144 instead of 270
 // warp instructions per warp and element step).  What is left is the L1 pipe (61 % busy) and the gathers of
 // upstream values from other blocks (27 % of the time); neither the sources' latency nor the barriers show.

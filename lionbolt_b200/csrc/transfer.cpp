@@ -1,7 +1,7 @@
 // Host vectors to and from the device through two pinned buffers per handle.
 //
 // Callers pass ordinary (pageable) arrays, FP64 where the device works in FP32.  A copy from pageable memory runs
-// through the driver's single-threaded staging, and converting on the device moves eight bytes per value over
+// through the CUDA driver's single-threaded staging, and converting on the device moves eight bytes per value over
 // the bus and needs a device buffer.  Here host threads convert or copy chunk after chunk into (out of) one
 // pinned buffer while the other one is on the bus, so the bus carries the device's own type and nothing is
 // allocated per call.  An operator application on a 132 MB angular vector took 82 ms with pageable copies.
