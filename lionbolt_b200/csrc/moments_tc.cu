@@ -97,6 +97,13 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, int* er
     return false;
 }
 
+// The same for a whole warp that goes on to warp-wide operations (tensor-memory loads and stores, __syncwarp): true only
+// when every lane saw the phase.  Each lane counts its own polls, so near the limit some may give up and
+// others not; lanes leaving the loop one by one would leave the rest waiting for them without end.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, long long limit = kSpinLimit) {
+    return __all_sync(0xffffffffu, bar_wait(bar, parity, err, limit));
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile(
@@ -315,7 +322,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             if (MODE == 2) {
                 // the tile's moments from the stage, then the stage back to the TMA: the proxy fence orders
                 // these generic reads before its next (async-proxy) write into the stage
-                if (!bar_wait(&xfull[xs], xu & 1u, err)) break;
+                if (!warp_wait(&xfull[xs], xu & 1u, err)) break;
                 const double* X = reinterpret_cast<const double*>(sX + xs * xbuf) + (size_t)(side * HM) * kTM + r;
                 const int jn = nm - side * HM;
 #pragma unroll
@@ -334,7 +341,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                 }
             }
             if (it >= na) {   // the A buffer's last use, tile it - na
-                if (!bar_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err)) break;
+                if (!warp_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err)) break;
                 tc_after_sync();
             }
             __syncwarp();
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
         for (long long tile = t0; tile < ntiles; tile += tstep, ++it) {
             const int b = it & 1;
             const uint32_t u = (uint32_t)(it >> 1);
-            if (!bar_wait(&done[b], u & 1u, err)) break;
+            if (!warp_wait(&done[b], u & 1u, err)) break;
             tc_after_sync();
             const long long n = tile * kTM + r;
             const bool valid = n < NENK;
@@ -596,7 +603,7 @@ __global__ void __launch_bounds__(kD2mThreads, 1) d2m_tc_kernel(const int* __res
                     if (hx) xp += NENK;
                 }
             }
-            if (!bar_wait(&dfull[b], u & 1u, err)) break;
+            if (!warp_wait(&dfull[b], u & 1u, err)) break;
             tc_after_sync();
 #pragma unroll
             for (int g = 0; g < KT; ++g) {
@@ -795,7 +802,7 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
         int s = 0, sa = 0;
         uint32_t u = 0, ua = 0;
         for (long long c = 0; c < nch; ++c) {
-            if (!bar_wait(&tfull[s], u & 1u, err)) break;
+            if (!warp_wait(&tfull[s], u & 1u, err)) break;
             const float* F = reinterpret_cast<const float*>(sF + s * fbuf) + (size_t)(side * 16) * kTM + row;
             float v[16];
 #pragma unroll
@@ -812,7 +819,7 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
                 split8(w, hi[cl], mid[cl], lo[cl]);
             }
             if (ua > 0) {
-                if (!bar_wait(&adone[sa], (ua - 1) & 1u, err)) break;
+                if (!warp_wait(&adone[sa], (ua - 1) & 1u, err)) break;
                 tc_after_sync();
             }
             __syncwarp();
@@ -851,7 +858,7 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
                     if (hx) xp += NENK;
                 }
             }
-            if (!bar_wait(&dfull[b], u & 1u, err)) break;
+            if (!warp_wait(&dfull[b], u & 1u, err)) break;
             tc_after_sync();
 #pragma unroll
             for (int g = 0; g < KT; ++g) {
@@ -1169,14 +1176,23 @@ int launch_d2m_tc(Handle* h, const float* psi, const double* xin, double alpha, 
 }
 
 namespace {
-// One thread waits on a pipeline barrier that nothing arrives at, with the contraction kernels' bounded wait
-// cut to `limit` polls: it gives up, raises the handle's error flag and returns, as a stuck stage would.
+// One warp waits as the contraction kernels' warps do, with the wait cut to `limit` polls, on a pipeline barrier that
+// nothing arrives at in its even lanes and on one whose phase is complete in its odd lanes: the even lanes give up
+// and raise the handle's error flag, as in a stuck stage.  Should any lane take the wait for successful (the warp would come
+// apart), the flag is withdrawn, so that the host sees no timeout.
 __global__ void tc_wait_probe_kernel(int* err, long long limit) {
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) {
-        bar_init(&bar, 1);
-        bar_wait(&bar, 0u, err, limit);
+    __shared__ __align__(8) uint64_t bar[2];
+    const int lane = threadIdx.x;
+    if (lane == 0) {
+        bar_init(&bar[0], 1);
+        bar_init(&bar[1], 1);
+        bar_arrive(&bar[1]);
     }
+    __syncwarp();
+    const bool ok = warp_wait(&bar[lane & 1], 0u, err, (lane & 1) ? kSpinLimit : limit);
+    const bool apart = __any_sync(0xffffffffu, ok);
+    __syncwarp();
+    if (apart && lane == 0) *(volatile int*)err = 0;
 }
 }  // namespace
 

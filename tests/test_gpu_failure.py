@@ -42,3 +42,15 @@ def test_pipeline_wait_timeout_is_reported_and_the_handle_stays_usable():
     out = x.copy()
     K.MatVec(out)
     assert rel_l2(out, ref) < 1e-5
+
+
+@pytest.mark.parametrize("polls", [1, 1023, 1024, 5000])
+def test_a_wait_that_half_a_warp_gives_up_is_given_up_by_all_of_it(polls):
+    """The contractions' warps go on from their waits to warp-wide operations, so a wait that runs out in some lanes has to
+    count as run out in all.  In the probe the even lanes give up after `polls` polls while the odd lanes' phase is
+    complete; it withdraws the flag if any lane came out with success."""
+    m = M.box_mesh(1, 1, 1, (0, 0, 0), (1, 1, 1))
+    k, w = P.quadrature(2, 4)
+    K = ScatteringOp().Build(m, AngularClass(k=k, w=w), XSType(np.array([0.5]), np.array([[0.2]])))
+    assert K._h.lib.lb_probe_pipeline_timeout(K._h.h, polls) == _lib.LB_ERR_TIMEOUT
+    assert K._h.lib.lb_synchronize(K._h.h) == 0
