@@ -126,6 +126,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// Bounded wait that neither reads nor raises the error flag, for the end of a kernel: what the calling thread set in
+// motion into the CTA's shared or tensor memory (TMA loads, MMAs) is done, also where a role gave up before it used it.
+__device__ __forceinline__ void bar_drain(uint64_t* bar, uint32_t parity) {
+    for (long long it = 0; it < kSpinLimit; ++it)
+        if (bar_try_wait(bar, parity)) return;
+}
+
 // Four columns of the calling warp's 32 lanes (eight BF16 along K per lane).
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint4 v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z),
@@ -319,16 +326,17 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                 m_next = nn < NENK ? __ldg(&mat[nn >> 2]) : 0;
             }
             double raw[HM];
+            bool gave_up = false;   // a lane whose wait ran out goes on until the vote below: the warp leaves together
             if (MODE == 2) {
                 // the tile's moments from the stage, then the stage back to the TMA: the proxy fence orders
                 // these generic reads before its next (async-proxy) write into the stage
-                if (!warp_wait(&xfull[xs], xu & 1u, err)) break;
+                gave_up = !bar_wait(&xfull[xs], xu & 1u, err);
                 const double* X = reinterpret_cast<const double*>(sX + xs * xbuf) + (size_t)(side * HM) * kTM + r;
                 const int jn = nm - side * HM;
 #pragma unroll
                 for (int k = 0; k < HM; ++k) raw[k] = k < jn ? X[(size_t)k * kTM] : 0.0;
                 fence_async_smem();
-                bar_arrive(&xempty[xs]);
+                if (!gave_up) bar_arrive(&xempty[xs]);
                 if (++xs == kM2dX) { xs = 0; ++xu; }
             } else {
                 // one pointer stepped by a row (NENK) per moment instead of a 64-bit index per load
@@ -340,11 +348,10 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                     sp += NENK;
                 }
             }
-            if (it >= na) {   // the A buffer's last use, tile it - na
-                if (!warp_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err)) break;
-                tc_after_sync();
-            }
-            __syncwarp();
+            // the A buffer's last use, tile it - na
+            if (it >= na) gave_up |= !bar_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err);
+            if (__any_sync(0xffffffffu, gave_up)) break;
+            tc_after_sync();
             const uint32_t at = a_lane + (na == 2 ? b : 0) * acols;
             // this half's sigma_l(j) row of the node's material (the table is padded to nmpad with zeros, and
             // raw[] is zero past the moments that exist, so no per-value bounds test is needed)
@@ -460,6 +467,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                 }
             mma_commit(&done[b]);
         }
+        if (it > 0) bar_drain(&done[(it - 1) & 1], (uint32_t)((it - 1) >> 1) & 1u);
     } else if (MODE == 2 && warp == kM2dTma && (tid & 31) == 0) {
         // ---- moment tiles by TMA, up to kM2dX ahead of the producers ----
         int xs = 0;
@@ -470,6 +478,8 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             tma_load_2d(sX + xs * xbuf, &x_map, (int)(tile * kTM), 0, &xfull[xs]);
             if (++xs == kM2dX) { xs = 0; ++xu; }
         }
+        // stages below xs hold load xu of their stage (counted from 0), the others load xu - 1
+        for (int k = 0; k < kM2dX && t0 + k * tstep < ntiles; ++k) bar_drain(&xfull[k], (k < xs ? xu : xu - 1) & 1u);
     }
     tc_before_sync();
     __syncthreads();
@@ -675,6 +685,7 @@ __global__ void __launch_bounds__(kD2mThreads, 1) d2m_tc_kernel(const int* __res
                 if (ch == nchunks - 1) mma_commit(&dfull[b]);
             }
         }
+        if (c > 0) bar_drain(&done[(c - 1) % kStages], (uint32_t)((c - 1) / kStages) & 1u);
     }
     tc_before_sync();
     __syncthreads();
@@ -794,6 +805,10 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
                 if (++s == kT32) { s = 0; ++u; }
                 if (++ch == nchunks) { ch = 0; tile += gridDim.x; }
             }
+            // stages below s hold load u of their stage (counted from 0), the others load u - 1
+#pragma unroll 1
+            for (int k = 0; k < kT32; ++k)
+                if (k < s || u > 0) bar_drain(&tfull[k], (k < s ? u : u - 1) & 1u);
         }
     } else if (warp < kD2tEpi) {
         // ---- converters: FP32 stage -> BF16 planes of the A stage ----
@@ -802,14 +817,15 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
         int s = 0, sa = 0;
         uint32_t u = 0, ua = 0;
         for (long long c = 0; c < nch; ++c) {
-            if (!warp_wait(&tfull[s], u & 1u, err)) break;
+            // (a lane whose wait ran out goes on until the vote below: the warp leaves together)
+            bool gave_up = !bar_wait(&tfull[s], u & 1u, err);
             const float* F = reinterpret_cast<const float*>(sF + s * fbuf) + (size_t)(side * 16) * kTM + row;
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = F[(size_t)k * kTM];
             // the stage is refilled by the TMA (async proxy): order these generic reads before that write
             fence_async_smem();
-            bar_arrive(&tempty[s]);
+            if (!gave_up) bar_arrive(&tempty[s]);
             uint4 hi[2], mid[2], lo[2];
 #pragma unroll
             for (int cl = 0; cl < 2; ++cl) {
@@ -818,11 +834,9 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
                 for (int k = 0; k < 8; ++k) w[k] = v[cl * 8 + k];
                 split8(w, hi[cl], mid[cl], lo[cl]);
             }
-            if (ua > 0) {
-                if (!warp_wait(&adone[sa], (ua - 1) & 1u, err)) break;
-                tc_after_sync();
-            }
-            __syncwarp();
+            if (ua > 0) gave_up |= !bar_wait(&adone[sa], (ua - 1) & 1u, err);
+            if (__any_sync(0xffffffffu, gave_up)) break;
+            tc_after_sync();
             const uint32_t at = a_lane + (uint32_t)(sa * kACols);
 #pragma unroll
             for (int cl = 0; cl < 2; ++cl) {
@@ -926,6 +940,9 @@ __global__ void __launch_bounds__(kD2tThreads, 1) d2m_tma_kernel(const __grid_co
                 if (++sa == NS) { sa = 0; ++ua; }
             }
         }
+        // the last stage used (commits complete in order)
+        if (sa > 0) bar_drain(&adone[sa - 1], ua & 1u);
+        else if (ua > 0) bar_drain(&adone[NS - 1], (ua - 1) & 1u);
     }
     tc_before_sync();
     __syncthreads();
