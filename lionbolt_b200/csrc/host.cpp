@@ -257,6 +257,7 @@ int lb_create(int device, lb_handle** out) {
     h->d_tc_err = reinterpret_cast<int*>(reinterpret_cast<char*>(h->h_red) + pinned);
     *h->d_tc_err = 0;
     if (cudaMalloc(&h->d_red, sizeof(double) * kRedValues) != cudaSuccess) { delete h; return LB_ERR_OOM; }
+    h->red_cap = kRedValues;
     *out = h;
     return LB_OK;
 }

@@ -696,18 +696,30 @@ static int seg_upload(Handle* h, const std::vector<SegVec>& segs, const std::vec
     return LB_OK;
 }
 
-// Where a segmented reduction's blocks write their partials: pinned host memory, as reduce_partials, or the
-// device buffer in a batch of more than some 650 problems, which has more blocks than the pinned one holds.
-static double* seg_partials(Handle* h, int grid) { return (size_t)grid * kPartStride <= kRedHost ? h->h_red : h->d_red; }
+// Where the blocks of a segmented reduction write their rows of cnt values, settled before the launch: pinned host memory,
+// as reduce_partials, or device memory in a batch of so many problems (a block each at least, from some 1,200 problems at
+// 33 values a row) that the pinned buffer does not hold them; it grows with the batch.
+static int seg_partials(Handle* h, const std::vector<SegVec>& segs, int cnt, double** part) {
+    const size_t n = (size_t)(segs.back().blk0 + segs.back().nblk) * cnt;
+    *part = h->h_red;
+    if (n <= kRedHost) return LB_OK;
+    if (n > h->red_cap) {
+        if (h->d_red) cudaFree(h->d_red);
+        h->d_red = nullptr;
+        h->red_cap = 0;
+        const cudaError_t e = cudaMalloc(&h->d_red, sizeof(double) * n);
+        if (e != cudaSuccess) return cuda_fail(h, e, "reduction buffer");
+        h->red_cap = n;
+    }
+    *part = h->d_red;
+    return LB_OK;
+}
 
-static int seg_reduce(Handle* h, const std::vector<SegVec>& segs, int cnt, std::vector<double>& out) {
-    const int grid = segs.back().blk0 + segs.back().nblk;
-    if ((size_t)grid * kPartStride > kRedValues) return fail(h, LB_ERR_ARG, "segmented reduction: too many blocks");
-    const double* red = seg_partials(h, grid);
+static int seg_reduce(Handle* h, const std::vector<SegVec>& segs, int cnt, const double* red, std::vector<double>& out) {
     std::vector<double> wide;
-    cudaError_t e = cudaSuccess;
-    if (red == h->d_red) {
-        wide.resize((size_t)grid * cnt);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && red == h->d_red) {
+        wide.resize((size_t)(segs.back().blk0 + segs.back().nblk) * cnt);
         e = cudaMemcpyAsync(wide.data(), h->d_red, sizeof(double) * wide.size(), cudaMemcpyDeviceToHost, h->stream);
         red = wide.data();
     }
@@ -723,14 +735,16 @@ int seg_dots_norm(Handle* h, const std::vector<SegVec>& segs, int nv, std::vecto
     if (segs.empty()) { out.clear(); return LB_OK; }
     if (nv < 0 || nv > kMaxDots) return fail(h, LB_ERR_ARG, "segmented dots: too many vectors");
     SegVec* ds = nullptr;
-    int rc = seg_upload(h, segs, nullptr, &ds, nullptr);
+    double* part = nullptr;
+    int rc = seg_partials(h, segs, nv + 1, &part);
+    if (!rc) rc = seg_upload(h, segs, nullptr, &ds, nullptr);
     if (rc) return rc;
     const int grid = segs.back().blk0 + segs.back().nblk;
     NvDispatch<kMaxDots>::run(nv, [&](auto c) {
         constexpr int NV = decltype(c)::value;
-        seg_dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), seg_partials(h, grid));
+        seg_dots_t<NV><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), part);
     });
-    return seg_reduce(h, segs, nv + 1, out);
+    return seg_reduce(h, segs, nv + 1, part, out);
 }
 
 int seg_axpy_dots(Handle* h, const std::vector<SegVec>& segs, int nv, const std::vector<double>& coef, bool dots,
@@ -739,15 +753,17 @@ int seg_axpy_dots(Handle* h, const std::vector<SegVec>& segs, int nv, const std:
     if (nv < 0 || nv > kMaxDots) return fail(h, LB_ERR_ARG, "segmented axpy: too many vectors");
     SegVec* ds = nullptr;
     double* dc = nullptr;
-    int rc = seg_upload(h, segs, &coef, &ds, &dc);
+    double* part = nullptr;
+    int rc = seg_partials(h, segs, nv + 1, &part);
+    if (!rc) rc = seg_upload(h, segs, &coef, &ds, &dc);
     if (rc) return rc;
     const int grid = segs.back().blk0 + segs.back().nblk;
     NvDispatch<kMaxDots>::run(nv, [&](auto c) {
         constexpr int NV = decltype(c)::value;
-        if (dots) seg_axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, seg_partials(h, grid));
-        else seg_axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, seg_partials(h, grid));
+        if (dots) seg_axpy_dots_t<NV, true><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, part);
+        else seg_axpy_dots_t<NV, false><<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), dc, part);
     });
-    return seg_reduce(h, segs, nv + 1, out);
+    return seg_reduce(h, segs, nv + 1, part, out);
 }
 
 int seg_axpy_scale(Handle* h, const std::vector<SegVec>& segs, int nv, const std::vector<double>& coef) {
@@ -769,11 +785,13 @@ int seg_axpy_scale(Handle* h, const std::vector<SegVec>& segs, int nv, const std
 int seg_axpby_norm(Handle* h, const std::vector<SegVec>& segs, std::vector<double>& out) {
     if (segs.empty()) { out.clear(); return LB_OK; }
     SegVec* ds = nullptr;
-    int rc = seg_upload(h, segs, nullptr, &ds, nullptr);
+    double* part = nullptr;
+    int rc = seg_partials(h, segs, 1, &part);
+    if (!rc) rc = seg_upload(h, segs, nullptr, &ds, nullptr);
     if (rc) return rc;
     const int grid = segs.back().blk0 + segs.back().nblk;
-    seg_axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), seg_partials(h, grid));
-    return seg_reduce(h, segs, 1, out);
+    seg_axpby_norm_kernel<<<grid, kRedThreads, 0, h->stream>>>(ds, (int)segs.size(), part);
+    return seg_reduce(h, segs, 1, part, out);
 }
 
 }  // namespace lb

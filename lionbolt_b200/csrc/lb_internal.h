@@ -173,7 +173,8 @@ struct Handle {
     double* d_x = nullptr;         // solution
     double* d_b = nullptr;         // rhs
     double* d_t = nullptr;         // scratch
-    double* d_red = nullptr;       // reduction partials
+    double* d_red = nullptr;       // reduction partials that do not fit the pinned buffer [red_cap]; scratch of the beam walk
+    size_t red_cap = 0;
     double* h_red = nullptr;       // pinned host copy of reductions [kRedHost], then the small transfer buffers
     size_t kry_n = 0;
 

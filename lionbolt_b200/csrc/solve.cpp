@@ -50,6 +50,7 @@ int ensure_krylov(Handle* h, int m, bool flexible) {
     if (!h->d_red) {
         cudaError_t e = cudaMalloc(&h->d_red, sizeof(double) * kRedValues);
         if (e != cudaSuccess) return cuda_fail(h, e, "reduction buffer");
+        h->red_cap = kRedValues;
     }
     if (flexible && !h->d_Z) {
         cudaError_t e = cudaMalloc(&h->d_Z, sizeof(double) * n * (size_t)h->kry_m);
