@@ -43,6 +43,7 @@ struct lb_batch {
     cudaGraphExec_t gx[3] = {nullptr, nullptr, nullptr};   // residual, a->b, b->a
     cudaEvent_t ev[2] = {nullptr, nullptr};
     double last_ms = 0.0;
+    std::mutex loan;                           // PipeLoan
     long long graph_launches = 0, sweep_launches = 0;
     std::string err;
 };
@@ -62,10 +63,12 @@ int bcuda(lb_batch* b, cudaError_t e, const char* what) {
 cudaStream_t bstream(lb_batch* b) { return b->aux->stream; }
 
 // Lends the batch's large transfer buffers to a problem's handle, so that a batch has one pair and not one per
-// problem.  The problem's copies must be done (or its stream be the batch's) when the loan ends.
+// problem.  The problem's copies must be done (or its stream be the batch's) when the loan ends.  One loan at a time:
+// threads that read results of different problems wait for one another.
 struct PipeLoan {
+    std::lock_guard<std::mutex> one;
     Handle *a, *h;
-    PipeLoan(Handle* a_, Handle* h_) : a(a_), h(h_) { std::swap(a->pipe_large, h->pipe_large); }
+    PipeLoan(lb_batch* b, Handle* h_) : one(b->loan), a(b->aux), h(h_) { std::swap(a->pipe_large, h->pipe_large); }
     ~PipeLoan() { std::swap(a->pipe_large, h->pipe_large); }
 };
 
@@ -599,7 +602,7 @@ int lb_batch_add_problem(lb_batch* b, int NE, int NN, const double* rg, const in
     if (!rc) rc = lb_set_mesh(h, NE, NN, rg, node, neighbors, mat, Nm);
     if (!rc) rc = lb_set_quadrature(h, NI, k, w);
     if (!rc) {
-        PipeLoan loan(b->aux, h);
+        PipeLoan loan(b, h);
         rc = lb_mg_set_problem(h, G, Ls, sigt, sigs, dd, unc, beam_dir);
         cudaStreamSynchronize(h->stream);
     }
@@ -691,7 +694,7 @@ int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int*
 
 int lb_batch_get_results(lb_batch* b, int id, double* flux, double* dose) {
     if (!b || id < 0 || id >= (int)b->probs.size()) return LB_ERR_ARG;
-    PipeLoan loan(b->aux, b->probs[id]);
+    PipeLoan loan(b, b->probs[id]);
     int rc = lb_mg_get_results(b->probs[id], flux, dose);
     return rc ? prop_error(b, b->probs[id], rc, id) : LB_OK;
 }
