@@ -214,6 +214,7 @@ struct Handle {
         void* buf[2] = {nullptr, nullptr};
         cudaEvent_t ev[2] = {nullptr, nullptr};   // the buffer's last copy
         size_t bytes = 0;          // of each buffer
+        size_t moved = 0;          // through the pair so far
         int next = 0;
     };
     Pipe pipe_small, pipe_large;

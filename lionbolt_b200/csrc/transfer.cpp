@@ -5,9 +5,12 @@
 // the bus and needs a device buffer.  Here host threads convert or copy chunk after chunk into (out of) one
 // pinned buffer while the other one is on the bus, so the bus carries the device's own type and nothing is
 // allocated per call.  An operator application on a 132 MB angular vector took 82 ms with pageable copies.
-// Transfers up to 4 MB use a pair of 95 KB buffers that come with the handle (allocating pinned memory takes
-// milliseconds, more than such a transfer); larger ones a pair of 8 MB that is allocated when first needed.
-// Both go with the handle.  Only large transfers use several threads: waking them costs a small one more than it
+// Transfers up to 4 MB use a pair of 95 KB buffers that come with the handle; larger ones a pair of 512 KB that is allocated
+// when first needed, and one of 4 MB once the handle has moved 512 MB through it.  Pinning costs 0.5 ms per MB, paid by the
+// call that needs it, and so has to be small against that call: the first sweep of a handle on a vector of 31 MB (7.7 MB)
+// took 11.4 (3.9) ms with pageable copies, 23 (10) with a pair of 8 MB, 6.2 (3.1) with 1 MB and 3.4 (1.6) with 512 KB.
+// Later ones take 65.8 MB there and back in 7.0 ms with 512 KB and 5.2 with 4 MB, which is worth its 4.4 ms from then on.
+// All go with the handle.  Only chunks of 256 KB up use several threads: waking them costs a small one more than it
 // saves, and they are half the host's (at most 8), so that threads still spinning after a transfer leave the
 // caller its core.
 #include "lb_internal.h"
@@ -19,9 +22,11 @@ namespace lb {
 
 namespace {
 
-constexpr size_t kPipeMax = (size_t)8 << 20;      // bytes of a large buffer
+constexpr size_t kPipeLarge = (size_t)1 << 19;    // bytes of a large buffer at first
+constexpr size_t kPipeMax = (size_t)4 << 20;      // and after kGrowAfter bytes
+constexpr size_t kGrowAfter = (size_t)1 << 29;
 constexpr size_t kLarge = (size_t)4 << 20;        // transfers above take the large buffers (and smaller ones once they exist)
-constexpr size_t kThreaded = (size_t)1 << 20;     // bytes of a buffer from which several threads do the work
+constexpr size_t kThreaded = (size_t)1 << 18;     // bytes of a chunk from which several threads do the work
 
 int threads_for(size_t bytes) { return bytes >= kThreaded ? std::max(1, std::min(8, omp_get_max_threads() / 2)) : 1; }
 
@@ -29,36 +34,40 @@ int threads_for(size_t bytes) { return bytes >= kThreaded ? std::max(1, std::min
 Handle::Pipe* pipe_for(Handle* h, size_t bytes) {
     const bool large = bytes > kLarge || (h->pipe_large.bytes && bytes > 2 * kPipeSmall);
     Handle::Pipe& p = large ? h->pipe_large : h->pipe_small;
+    const size_t want = !large ? kPipeSmall : p.moved < kGrowAfter ? kPipeLarge : kPipeMax;
+    p.moved += bytes;
+    if (p.bytes >= want) return &p;
+    void* buf[2] = {nullptr, nullptr};
     cudaError_t e = cudaSuccess;
-    if (!p.bytes) {
-        for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-            if (large) e = cudaMallocHost(&p.buf[b], kPipeMax);
-            else p.buf[b] = reinterpret_cast<char*>(h->h_red + kRedHost) + b * kPipeSmall;
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p.ev[b], cudaEventDisableTiming);
-        }
-        if (e != cudaSuccess && large) {
-            // no pinned memory for the large pair: the handle's own small one, in more chunks
-            for (int b = 0; b < 2; ++b) {
-                if (p.buf[b]) cudaFreeHost(p.buf[b]);
-                if (p.ev[b]) cudaEventDestroy(p.ev[b]);
-            }
-            p = Handle::Pipe{};
-            cudaGetLastError();
-            return pipe_for(h, 0);
-        }
-        if (e != cudaSuccess) {
-            pipe_free(h);
-            cuda_fail(h, e, "transfer buffers");
-            return nullptr;
-        }
-        p.bytes = large ? kPipeMax : kPipeSmall;
+    for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
+        if (large) e = cudaMallocHost(&buf[b], want);
+        else buf[b] = reinterpret_cast<char*>(h->h_red + kRedHost) + b * kPipeSmall;
+    }
+    if (e != cudaSuccess) {
+        // no pinned memory: the pair there is, or the handle's own small one, in more chunks
+        if (buf[0]) cudaFreeHost(buf[0]);
+        cudaGetLastError();
+        p.moved = 0;
+        return p.bytes ? &p : pipe_for(h, 0);
+    }
+    for (int b = 0; b < 2 && e == cudaSuccess; ++b)
+        e = p.ev[b] ? cudaEventSynchronize(p.ev[b]) : cudaEventCreateWithFlags(&p.ev[b], cudaEventDisableTiming);
+    for (int b = 0; b < 2; ++b) {
+        if (p.buf[b]) cudaFreeHost(p.buf[b]);   // (of a pair that grows: its last copies are done)
+        p.buf[b] = buf[b];
+    }
+    p.bytes = want;
+    if (e != cudaSuccess) {
+        pipe_free(h);
+        cuda_fail(h, e, "transfer buffers");
+        return nullptr;
     }
     return &p;
 }
 
 void copy_bytes(void* dst, const void* src, size_t bytes) {
     const int nt = threads_for(bytes);
-    const size_t part = nt > 1 ? (size_t)1 << 18 : bytes;
+    const size_t part = nt > 1 ? (size_t)1 << 17 : bytes;
     const long long parts = (long long)((bytes + part - 1) / part);
 #pragma omp parallel for schedule(static) num_threads(nt) if (nt > 1)
     for (long long p = 0; p < parts; ++p) {
