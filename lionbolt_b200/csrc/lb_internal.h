@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -218,6 +219,8 @@ struct Handle {
         int next = 0;
     };
     Pipe pipe_small, pipe_large;
+    std::unique_ptr<float[]> hold;   // [hold_cap] a vector that has come whole before it is used (pipe_down_f32)
+    size_t hold_cap = 0;
 
     // planar-beam ray walk (beam.cu): face planes, coordinates, connectivity, neighbours on the device
     double4* d_beam_plane = nullptr;
@@ -357,7 +360,7 @@ int seg_axpby_norm(Handle* h, const std::vector<SegVec>& segs, std::vector<doubl
 // ---- transfers (transfer.cpp): through the handle's pinned buffers; an upload's source is free on return, a
 // download is complete on return ----
 int pipe_up_f32(Handle* h, float* dst, const double* src, size_t n, const char* what);
-// dst = src, or dst -= src
+// dst = src, or dst -= src (all of it or, after an error, nothing)
 int pipe_down_f32(Handle* h, double* dst, const float* src, size_t n, bool subtract, const char* what);
 int pipe_up(Handle* h, void* dst, const void* src, size_t bytes, const char* what);
 int pipe_down(Handle* h, void* dst, const void* src, size_t bytes, const char* what);

@@ -16,6 +16,7 @@
 #include "lb_internal.h"
 #include <algorithm>
 #include <cstring>
+#include <new>
 #include <omp.h>
 
 namespace lb {
@@ -26,6 +27,7 @@ constexpr size_t kPipeLarge = (size_t)1 << 19;    // bytes of a large buffer at 
 constexpr size_t kPipeMax = (size_t)4 << 20;      // and after kGrowAfter bytes
 constexpr size_t kGrowAfter = (size_t)1 << 29;
 constexpr size_t kLarge = (size_t)4 << 20;        // transfers above take the large buffers (and smaller ones once they exist)
+constexpr size_t kHoldMax = (size_t)256 << 20;     // bytes of a vector on its way that a handle keeps the place of
 constexpr size_t kThreaded = (size_t)1 << 18;     // bytes of a chunk from which several threads do the work
 
 int threads_for(size_t bytes) { return bytes >= kThreaded ? std::max(1, std::min(8, omp_get_max_threads() / 2)) : 1; }
@@ -156,8 +158,25 @@ int pipe_up_f32(Handle* h, float* dst, const double* src, size_t n, const char* 
 }
 
 int pipe_down_f32(Handle* h, double* dst, const float* src, size_t n, bool subtract, const char* what) {
-    return down(h, src, n, sizeof(float), what,
-                [&](const void* b, size_t o, size_t c) { to_f64(dst + o, (const float*)b, c, subtract); });
+    auto drain = [&](const void* b, size_t o, size_t c) { to_f64(dst + o, (const float*)b, c, subtract); };
+    if (!subtract || n * sizeof(float) <= kPipeSmall) return down(h, src, n, sizeof(float), what, drain);
+    // what dst holds is an operand: it changes only when all of src is here, or a copy that fails half way would leave it
+    // half changed.  (A vector that fits one buffer is drained when all of it has come.)  The handle keeps the place
+    // up to 256 MB: page faults on a fresh one cost as much as the rest (65.8 MB: an operator application takes 11.4 ms
+    // with a fresh place, 7.5 with a kept one, 6.0 if every chunk were subtracted as it comes).
+    if (h->hold_cap < n) {
+        h->hold_cap = 0;
+        h->hold.reset(new (std::nothrow) float[n]);
+        if (!h->hold) return fail(h, LB_ERR_OOM, std::string(what) + ": no host memory");
+        h->hold_cap = n;
+    }
+    const int rc = pipe_down(h, h->hold.get(), src, n * sizeof(float), what);
+    if (!rc) drain(h->hold.get(), 0, n);
+    if (h->hold_cap * sizeof(float) > kHoldMax) {
+        h->hold.reset();
+        h->hold_cap = 0;
+    }
+    return rc;
 }
 
 int pipe_up(Handle* h, void* dst, const void* src, size_t bytes, const char* what) {

@@ -153,3 +153,21 @@ def test_a_handle_that_moves_much_gets_larger_buffers(lib, handle, refused):
         assert lib.t_up(handle, _p(dev), _p(src), src.size) == 0
         assert lib.t_pinned() - before == (8 * MB if k == 8 and not refused else MB)
     _round_trip(lib, handle, 9 * MB + 17)
+
+
+@pytest.mark.parametrize("nbytes", BYTES)
+def test_a_difference_is_taken_whole_or_not_at_all(lib, handle, nbytes):
+    """The subtracted-from vector is the caller's operand: a copy that fails, whichever it is, leaves it as it was."""
+    n = max(1, nbytes // 4)
+    r = np.random.default_rng(3)
+    x, y = r.normal(size=n), r.normal(size=n).astype(np.float32)
+    failed = 0
+    for k in range(64):
+        lib.t_fail_after(k)
+        out = x.copy()
+        rc = lib.t_down_f32(handle, _p(out), _p(y), n, 1)
+        assert np.array_equal(out, x if rc else x - y)
+        failed += rc != 0
+        if rc == 0:
+            break
+    assert failed >= 1
