@@ -231,7 +231,7 @@ int lb_givens(double x, double y, double* c, double* s, double* r);
  *     (optional) = block members (-1: empty), *max_records = largest record count of a direction.
  *   lb_get_cluster_schedule: rec[rec_base[NI]][4] records in execution order (x = block index; y, z, w =
  *     two 16-bit slots each in execution order: member position in the block (3 b, 7 = empty),
- *     upstream-face mask << 3, outflow-face mask << 7, tile type << 11), starts[NI][max_records + 1] block-level
+ *     upstream-face mask << 3, outflow-face mask << 7), starts[NI][max_records + 1] block-level
  *     starts (relative to rec_base[i]), nlevels[NI].
  * Diagnostics for tests; no counterpart in the reference. */
 int lb_cluster_info(lb_handle* h, int* nblocks, int* max_levels);

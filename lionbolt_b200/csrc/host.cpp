@@ -1298,6 +1298,10 @@ int lb_get_cluster_schedule(lb_handle* h, int* rec, int* starts, int* nlevels) {
         cudaError_t e = cudaMemcpy(rec, h->d_crec, sizeof(int4) * n, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(h, e, "lb_get_cluster_schedule");
     }
+    // the slots' tile types stay inside
+    if (h->nxtype > 0)
+        for (size_t q = 0; q < 4 * n; ++q)
+            if (q % 4) rec[q] &= 0x07FF07FF;
     const size_t ld = (size_t)h->max_cluster_records + 1;
     for (int i = 0; i < h->NI; ++i) {
         nlevels[i] = h->ncl_h[i];

@@ -360,3 +360,25 @@ def test_cluster_queries_need_a_block_schedule():
     assert hs.mesh(M.box_mesh(1, 1, 1)) == 0
     one = np.zeros(4, np.int32)
     assert hs.lib.lb_get_cluster_schedule(hs.h, _lib.iptr(one), _lib.iptr(one), _lib.iptr(one)) == _lib.LB_ERR_STATE
+
+
+def test_cluster_schedule_records_are_positions_and_masks():
+    """A slot is position | upstream mask << 3 | outflow mask << 7: the tile types that the sweep keeps with them (a box of two
+    materials has 12) are no part of what a caller reads."""
+    m = M.box_mesh(4, 3, 5, (0, 0, 0), (2.0, 1.5, 2.5), material=lambda c: (c[:, 0] > 1.0).astype(np.int32), Nm=2)
+    k, w = P.quadrature(2, 6)
+    cs, split = _check_cluster_schedule(m, k, w)
+    assert split == 0
+    words = cs["rec"][:, 1:]
+    assert np.all((words & ~0x07FF07FF) == 0)
+    hh = HostHandle()
+    assert hh.mesh(m) == 0 and hh.quad(k, w) == 0
+    sl, up, nlev, ls = hh.schedule(m.NE, len(w))
+    for i in range(len(w)):
+        rec = cs["rec"][cs["base"][i]:cs["base"][i + 1]]
+        slots = np.stack([rec[:, 1:] & 0xFFFF, (rec[:, 1:] >> 16) & 0xFFFF], axis=2).reshape(len(rec), 6)
+        upm = np.zeros(m.NE, np.int64)
+        upm[sl[i]] = up[i]
+        e = cs["members"][rec[:, :1], slots & 7]
+        assert np.array_equal((slots >> 3) & 15, upm[e])
+        assert np.all(((slots >> 7) & upm[e]) == 0)         # no face is both
