@@ -308,7 +308,7 @@ int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int*
 /* flux[G][NENK], dose[NENK] of problem id (either may be NULL). */
 int lb_batch_get_results(lb_batch* b, int id, double* flux, double* dose);
 /* Problem count, largest group count, device time of the last solve (ms), threads per CTA of the batched
- * sweep, graph replays and batched sweep launches so far.  Any pointer may be NULL. */
+ * sweep (0 before the first solve), graph replays and batched sweep launches so far.  Any pointer may be NULL. */
 int lb_batch_info(lb_batch* b, int* nproblems, int* max_groups, double* last_ms, int* sweep_threads,
                   long long* graph_launches, long long* sweep_launches);
 

@@ -707,7 +707,7 @@ int lb_batch_info(lb_batch* b, int* nproblems, int* max_groups, double* last_ms,
     if (nproblems) *nproblems = (int)b->probs.size();
     if (max_groups) *max_groups = Gmax;
     if (last_ms) *last_ms = b->last_ms;
-    if (sweep_threads) *sweep_threads = kBatchThreads;
+    if (sweep_threads) *sweep_threads = b->sweep_team ? kBatchThreads : 0;
     if (graph_launches) *graph_launches = b->graph_launches;
     if (sweep_launches) *sweep_launches = b->sweep_launches;
     return LB_OK;

@@ -66,3 +66,14 @@ def test_batch_resolve_is_repeatable():
     assert np.array_equal(it1, it2)
     for a, b in zip(d1, d2):
         assert rel_l2(a, b) < 1e-12
+
+
+def test_batch_info_before_and_after_the_first_solve():
+    bs = BatchSolver()
+    for p in _small_batch(count=2, seed=3):
+        bs.add_problem(p)
+    info = bs.info()
+    assert info["problems"] == 2 and info["sweep_threads"] == 0 and info["sweep_launches"] == 0
+    bs.solve(m=10, rtol=1e-4)
+    info = bs.info()
+    assert info["sweep_threads"] > 0 and info["sweep_launches"] > 0
