@@ -247,7 +247,8 @@ constexpr int kM2dX = 2;
 
 // MODE 0: per-thread output stores; 1: TMA output stores (two staging buffers per epilogue warp); 2: TMA
 // output stores and the moment tiles x[0..nm)[128 nodes] brought into a shared-memory ring by TMA, from which the producers read (nodes past NENK arrive as zeros).
-template <int KT, int MODE>
+// AS: the A buffers (two) in shared memory instead, for directions that would need more parts otherwise (launch_m2d_tc).
+template <int KT, int MODE, bool AS>
 __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m2d_tc_kernel(
                                                       const __grid_constant__ CUtensorMap q_map,
                                                       const __grid_constant__ CUtensorMap x_map,
@@ -262,8 +263,10 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     constexpr int NMP = KT * 16;
     const int tid = threadIdx.x, warp = tid >> 5;
     const size_t bplane = (size_t)NH * nmpad * 2;
+    constexpr size_t aplane = (size_t)kTM * NMP * 2;
     unsigned char* sB = sm;
-    unsigned char* sT = sm + ((3 * bplane + 1023) / 1024) * 1024;
+    unsigned char* sA = sm + ((3 * bplane + 1023) / 1024) * 1024;       // AS: [2] buffers of 3 planes
+    unsigned char* sT = sA + (AS ? 6 * aplane : 0);
     uint64_t* full = reinterpret_cast<uint64_t*>(sT);
     uint64_t* done = full + 2;
     uint64_t* empty = full + 4;
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
     uint64_t* xempty = xfull + kM2dX;        // MODE 2: [kM2dX] moment stages read
     uint32_t* tslot = reinterpret_cast<uint32_t*>(xempty + kM2dX);
     // MODE >= 1: per epilogue warp NB 2 KB staging buffers [16 directions][32 nodes] for the TMA stores
-    constexpr int NB = 2;
+    constexpr int NB = AS && MODE == 2 ? 1 : 2;
     float* sS = reinterpret_cast<float*>(sT + 1024);
     const size_t xbuf = (size_t)kTM * nm * 8;                           // MODE 2: one moment stage
     unsigned char* sX = sT + 1024 + (size_t)kM2dEpi * NB * 2048;         // MODE 2: [kM2dX] stages
@@ -351,7 +354,7 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             // the A buffer's last use, tile it - na
             if (it >= na) gave_up |= !bar_wait(&done[(it - na) & 1], (uint32_t)((it - na) >> 1) & 1u, err);
             if (__any_sync(0xffffffffu, gave_up)) break;
-            tc_after_sync();
+            if (!AS) tc_after_sync();
             const uint32_t at = a_lane + (na == 2 ? b : 0) * acols;
             // this half's sigma_l(j) row of the node's material (the table is padded to nmpad with zeros, and
             // raw[] is zero past the moments that exist, so no per-value bounds test is needed)
@@ -373,12 +376,23 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                 }
                 uint4 hi, mid, lo;
                 split8(v, hi, mid, lo);
-                tmem_st4(at + cl * 4, hi);
-                tmem_st4(at + NMP / 2 + cl * 4, mid);
-                tmem_st4(at + NMP + cl * 4, lo);
+                if (AS) {
+                    unsigned char* row = sA + b * 3 * aplane + (size_t)(side * (HM / 8) + cl) * kTM * 16 + (size_t)r * 16;
+                    *reinterpret_cast<uint4*>(row) = hi;
+                    *reinterpret_cast<uint4*>(row + aplane) = mid;
+                    *reinterpret_cast<uint4*>(row + 2 * aplane) = lo;
+                } else {
+                    tmem_st4(at + cl * 4, hi);
+                    tmem_st4(at + NMP / 2 + cl * 4, mid);
+                    tmem_st4(at + NMP + cl * 4, lo);
+                }
             }
-            tmem_st_wait();
-            tc_before_sync();
+            if (AS) {
+                fence_async_smem();
+            } else {
+                tmem_st_wait();
+                tc_before_sync();
+            }
             bar_arrive(&full[b]);
         }
     } else if (warp < kM2dMma) {
@@ -407,7 +421,8 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
                     // NENK and directions past NI lie outside the tensor and are not written)
                     float* st = stage + sidx * 512;
                     if (lane == 0) {
-                        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                        if (NB == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     }
                     __syncwarp();
 #pragma unroll
@@ -463,7 +478,13 @@ __global__ void __launch_bounds__(MODE == 2 ? kM2dThreadsTma : kM2dThreads, 1) m
             for (int ks = 0; ks < KT; ++ks)
                 for (int pr = 0; pr < 6; ++pr) {
                     const uint64_t db = sdesc(bBase + kProdB[pr] * (uint32_t)bplane + ks * 2 * lboB, lboB, 128);
-                    mma_bf16_ts(tmem + b * NH, a0 + kProdA[pr] * (NMP / 2) + ks * 8, db, idesc, (ks | pr) ? 1u : 0u);
+                    if (AS) {
+                        const uint64_t da = sdesc(smem_u32(sA) + (uint32_t)((3 * b + kProdA[pr]) * aplane) + ks * 2 * kTM * 16,
+                                                  kTM * 16, 128);
+                        mma_bf16_ss(tmem + b * NH, da, db, idesc, (ks | pr) ? 1u : 0u);
+                    } else {
+                        mma_bf16_ts(tmem + b * NH, a0 + kProdA[pr] * (NMP / 2) + ks * 8, db, idesc, (ks | pr) ? 1u : 0u);
+                    }
                 }
             mma_commit(&done[b]);
         }
@@ -974,10 +995,10 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-size_t m2d_tc_smem(int NH, int nmpad, int mode, int nm) {
-    const size_t b = ((3 * (size_t)NH * nmpad * 2 + 1023) / 1024) * 1024 + 1024;
+size_t m2d_tc_smem(int NH, int nmpad, int mode, int nm, bool as) {
+    const size_t b = ((3 * (size_t)NH * nmpad * 2 + 1023) / 1024) * 1024 + 1024 + (as ? 6 * (size_t)kTM * nmpad * 2 : 0);
     if (mode == 0) return b;
-    return b + (size_t)kM2dEpi * 2 * 2048 + (mode == 2 ? kM2dX * (size_t)kTM * nm * 8 : 0);
+    return b + (size_t)kM2dEpi * (as && mode == 2 ? 1 : 2) * 2048 + (mode == 2 ? kM2dX * (size_t)kTM * nm * 8 : 0);
 }
 
 size_t d2m_tc_smem(int NIpad, int nmpad) {
@@ -1031,13 +1052,20 @@ bool moments_tma_load_enabled() {
 // Returns LB_ERR_ARG when the shape does not fit the tensor-core kernels (caller falls back).
 int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a, const float* qadd, float* q) {
     if (h->NIpad > 512 || h->nmpad % 16 || h->nmpad > 64 || h->NIpad % 8) return LB_ERR_ARG;
-    // parts of the directions such that two accumulators of NH columns and an A buffer of 3 nmpad / 2 fit the 512 TMEM
-    // columns (288 directions at P5: two parts of 144; the moments are then read twice, the second time from
-    // L2), and a second A buffer where it fits
-    int nhalves = 1, NH;
+    // parts of the directions: with A in shared memory as many as two accumulators in the 512 TMEM columns ask for, with A
+    // in tensor memory as many as leave room for an A buffer of 3 nmpad / 2 columns beside them (288 directions at P5: two
+    // parts of 144 either way; the moments are then read twice, the second time from L2), and a second one where it fits
     const int acols = 3 * h->nmpad / 2;
-    while (NH = ((h->NIpad + nhalves - 1) / nhalves + 15) / 16 * 16, NH > 256 || 2 * NH + acols > 512) ++nhalves;
-    const int na = 2 * NH + 2 * acols <= 512 ? 2 : 1;
+    auto part = [&](int parts) { return ((h->NIpad + parts - 1) / parts + 15) / 16 * 16; };
+    int nhalves = h->NIpad > 256 ? 2 : 1, ntm = nhalves;
+    while (2 * part(ntm) + acols > 512) ++ntm;
+    // A goes to shared memory where tensor memory would take a part more: us at 192,000 / 1,536,000 nodes with A in shared,
+    // tensor memory for 216 and 256 directions at P5 61 / 350, 69 / 443 and 65 / 376, 71 / 455, 512 at P5 105 / 706,
+    // 110 / 747, 216 at P7 86 / 528, 90 / 590, 512 at P3 95 / 749, 97 / 768.  Up to P4 and 256 directions the two parts win
+    // where there are many nodes: 256 at P4 55 / 403, 56 / 346, 256 at P3 51 / 384, 53 / 373.
+    const bool as = nhalves < ntm && !(h->nmpad <= 32 && ntm == 2 && h->NENK >= 1 << 20);
+    if (!as) nhalves = ntm;
+    const int NH = part(nhalves), na = as || 2 * NH + 2 * acols <= 512 ? 2 : 1;
     // one CTA per SM (it holds all TMEM columns)
     int* err = h->d_tc_err;
     if (!err) return LB_ERR_STATE;
@@ -1047,7 +1075,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
     CUtensorMap xmap;
     std::memset(&xmap, 0, sizeof(xmap));
     EncodeTiledFn enc = encode_tiled();
-    bool ts = enc && !qadd && moments_tma_store_enabled() && m2d_tc_smem(NH, h->nmpad, 1, h->nm) <= 227 * 1024 &&
+    bool ts = enc && !qadd && moments_tma_store_enabled() && m2d_tc_smem(NH, h->nmpad, 1, h->nm, as) <= 227 * 1024 &&
               !((uintptr_t)q & 15) && h->NENK < (1LL << 31);
     if (ts) {
         const cuuint64_t dims[2] = {(cuuint64_t)h->NENK, (cuuint64_t)h->NI};
@@ -1062,7 +1090,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
     // null: the group sources), not when both are given
     const double* src = x ? x : a;
     bool tl = ts && src && !(x && a) && moments_tma_load_enabled() && h->nm <= 256 &&
-              m2d_tc_smem(NH, h->nmpad, 2, h->nm) <= 227 * 1024 && !((uintptr_t)src & 15);
+              m2d_tc_smem(NH, h->nmpad, 2, h->nm, as) <= 227 * 1024 && !((uintptr_t)src & 15);
     if (tl) {
         const cuuint64_t dims[2] = {(cuuint64_t)h->NENK, (cuuint64_t)h->nm};
         const cuuint64_t strides[1] = {(cuuint64_t)h->NENK * 8};
@@ -1073,32 +1101,33 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
     const int mode = tl ? 2 : ts ? 1 : 0;
-    const size_t smem = std::max<size_t>(m2d_tc_smem(NH, h->nmpad, mode, h->nm), 116 * 1024);
+    const size_t smem = std::max<size_t>(m2d_tc_smem(NH, h->nmpad, mode, h->nm, as), 116 * 1024);
     if (smem > 227 * 1024) return LB_ERR_ARG;
     static PerDevice attr;
     attr.get([&] {
-#define LB_M2DATTR(K)                                                                                      \
-    cudaFuncSetAttribute(m2d_tc_kernel<K, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);   \
-    cudaFuncSetAttribute(m2d_tc_kernel<K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);   \
-    cudaFuncSetAttribute(m2d_tc_kernel<K, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
-        LB_M2DATTR(1);
-        LB_M2DATTR(2);
-        LB_M2DATTR(3);
-        LB_M2DATTR(4);
+#define LB_M2DATTR(K, A)                                                                                      \
+    cudaFuncSetAttribute(m2d_tc_kernel<K, 0, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
+    cudaFuncSetAttribute(m2d_tc_kernel<K, 1, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
+    cudaFuncSetAttribute(m2d_tc_kernel<K, 2, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
+        LB_M2DATTR(1, false); LB_M2DATTR(2, false); LB_M2DATTR(3, false); LB_M2DATTR(4, false);
+        LB_M2DATTR(1, true); LB_M2DATTR(2, true); LB_M2DATTR(3, true); LB_M2DATTR(4, true);
 #undef LB_M2DATTR
         return 1;
     });
     const long long ntiles = (h->NENK + kTM - 1) / kTM;
     long long grid = std::min<long long>(ntiles * nhalves, (long long)h->sm_count);
     grid = std::max<long long>(nhalves, grid / nhalves * nhalves);
-#define LB_M2DTC(K, M)                                                                                              \
-    m2d_tc_kernel<K, M><<<(int)grid, M == 2 ? kM2dThreadsTma : kM2dThreads, smem, h->stream>>>(                      \
+#define LB_M2DTC(K, M, A)                                                                                              \
+    m2d_tc_kernel<K, M, A><<<(int)grid, M == 2 ? kM2dThreadsTma : kM2dThreads, smem, h->stream>>>(                      \
         map, xmap, h->d_active, x, sigl, a, qadd, h->d_mat, h->d_Ym2d, q, h->NENK, h->NI, h->NIpad, h->nm, h->nmpad, \
         NH, nhalves, na, ntiles, err)
-#define LB_M2DK(K)                           \
-    if (mode == 2) LB_M2DTC(K, 2);           \
-    else if (mode == 1) LB_M2DTC(K, 1);      \
-    else LB_M2DTC(K, 0)
+#define LB_M2DKA(K, A)                         \
+    if (mode == 2) LB_M2DTC(K, 2, A);          \
+    else if (mode == 1) LB_M2DTC(K, 1, A);     \
+    else LB_M2DTC(K, 0, A)
+#define LB_M2DK(K)                  \
+    if (as) { LB_M2DKA(K, true); }  \
+    else { LB_M2DKA(K, false); }
     switch (h->nmpad / 16) {
         case 1: LB_M2DK(1); break;
         case 2: LB_M2DK(2); break;
@@ -1106,6 +1135,7 @@ int launch_m2d_tc(Handle* h, const double* x, const float* sigl, const double* a
         default: LB_M2DK(4); break;
     }
 #undef LB_M2DK
+#undef LB_M2DKA
 #undef LB_M2DTC
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LB_OK : cuda_fail(h, e, "m2d tensor-core kernel");

@@ -33,6 +33,28 @@ SHAPES = [
 
 @pytest.mark.parametrize("n,Ng,Nc,L", SHAPES)
 def test_contractions_at_the_edges_of_their_tensor_memory_layout(n, Ng, Nc, L):
+    _check(n, Ng, Nc, L)
+
+
+# M2D with A in shared memory, where A in tensor memory would take another part of the directions: one part instead of two,
+# the most directions that one holds, two parts instead of three, and with per-thread moment loads where the ring does not fit
+SHARED_A = [
+    ((3, 2, 5), 12, 18, 5),      # 216 at P5: the fewest that take a part more
+    ((13, 14, 15), 16, 16, 5),   # 256 at P5
+    ((13, 14, 15), 12, 36, 5),   # 432 at P5 in two parts of 224, the second with fewer directions
+    ((3, 2, 5), 16, 32, 7),      # 512 at P7: the most, all of it
+    ((13, 14, 15), 12, 18, 7),   # 216 at P7
+    ((3, 2, 5), 12, 20, 4),      # 240 at P4
+    ((13, 14, 15), 16, 32, 1),   # 512 at P1
+]
+
+
+@pytest.mark.parametrize("n,Ng,Nc,L", SHARED_A)
+def test_m2d_with_its_first_operand_in_shared_memory(n, Ng, Nc, L):
+    _check(n, Ng, Nc, L)
+
+
+def _check(n, Ng, Nc, L):
     torch = pytest.importorskip("torch")
     m = M.box_mesh(*n, (0, 0, 0), (2.0, 1.5, 2.5), material=lambda c: (c[:, 2] > 1.0).astype(np.int32), Nm=2)
     k, w = P.quadrature(Ng, Nc)
