@@ -12,7 +12,7 @@
 //     captured once per group step as a CUDA graph and replayed for every Arnoldi step, on fixed
 //     per-problem ping-pong buffers;
 //   * the Gram-Schmidt dots, axpys and norms are segmented kernels: one launch for all problems.
-// The threads that take a direction are chosen from the sizes of its groups (choose_team).
+// The threads that take a direction are chosen from the sizes of its groups (choose_teams).
 #include "lb_internal.h"
 #include "gmres_host.h"
 #include <algorithm>
@@ -37,9 +37,8 @@ struct lb_batch {
     int cap = 0;
     BatchWork* d_work = nullptr;
     int work_cap = 0;
-    int nwork = 0;
     int* d_counter = nullptr;
-    int sweep_team = 0;                        // threads of a CTA that take a direction (choose_team)
+    BatchSweep sweep;                          // the sweep of the current work list
     cudaGraphExec_t gx[3] = {nullptr, nullptr, nullptr};   // residual, a->b, b->a
     cudaEvent_t ev[2] = {nullptr, nullptr};
     double last_ms = 0.0;
@@ -86,12 +85,15 @@ int prop_error(lb_batch* b, lb_handle* h, int rc, int p) {
     return bfail(b, rc, buf + (h ? h->err : std::string("error")));
 }
 
-// Work list of the batched sweep for the problems in `ids`, longest direction first.
-int build_work(lb_batch* b, const std::vector<int>& ids, int threads) {
+// Work list of the batched sweep for the problems in `ids`: directions with tile types, then the others, longest first.
+int build_work(lb_batch* b, const std::vector<int>& ids) {
     std::vector<BatchWork> w;
     std::vector<double> cost;
+    b->sweep.max_geom = 0;
     for (int p : ids) {
         lb_handle* h = b->probs[p];
+        const int threads = h->tiles_ok ? b->sweep.tile_team : b->sweep.walk_team;
+        if (!h->tiles_ok && h->nclusters > 0) b->sweep.max_geom = std::max(b->sweep.max_geom, h->ngeom);
         for (int i = 0; i < h->NI; ++i) {
             BatchWork x{};
             x.items = h->d_items + (size_t)i * h->NE;
@@ -135,7 +137,10 @@ int build_work(lb_batch* b, const std::vector<int>& ids, int threads) {
     }
     std::vector<int> ord(w.size());
     std::iota(ord.begin(), ord.end(), 0);
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return cost[a] > cost[c]; });
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) {
+        const bool ta = w[a].nxtype > 0, tc = w[c].nxtype > 0;
+        return ta != tc ? ta : cost[a] > cost[c];
+    });
     std::vector<BatchWork> ws(w.size());
     for (size_t i = 0; i < ord.size(); ++i) ws[i] = w[ord[i]];
     if ((int)ws.size() > b->work_cap) {
@@ -150,39 +155,53 @@ int build_work(lb_batch* b, const std::vector<int>& ids, int threads) {
                                     bstream(b));
     if (e == cudaSuccess) e = cudaStreamSynchronize(bstream(b));
     if (e != cudaSuccess) return bcuda(b, e, "batch work list");
-    b->nwork = (int)ws.size();
+    b->sweep.work = b->d_work;
+    b->sweep.nwork = (int)ws.size();
+    b->sweep.ntile = (int)std::count_if(ws.begin(), ws.end(), [](const BatchWork& x) { return x.nxtype > 0; });
+    b->sweep.counter = b->d_counter;
     return LB_OK;
 }
 
 int sweep_all(lb_batch* b) {
     ++b->sweep_launches;
-    int rc = launch_sweep_batch(bstream(b), b->d_work, b->nwork, b->d_counter, b->d_active, b->sweep_team,
-                                b->aux->sm_count);
+    const int rc = launch_sweep_batch(bstream(b), b->sweep, b->d_active, b->aux->sm_count);
     return rc ? bfail(b, rc, "batched sweep launch failed") : LB_OK;
 }
 
 // Threads that take a direction in the batched sweep of the problems `ids`: small teams where the groups are
 // small (a wider team's threads would idle in most passes), as long as every SM still gets a CTA of 512 / team
-// teams.  Measured: 8 problems of 8 to 20 hexes per axis (about 70 units a group) 0.655, 0.418 and 0.358 ms per
+// teams.  Measured with tile types: 8 problems of 8 to 20 hexes per axis (about 70 units a group) 0.655, 0.418 and 0.358 ms per
 // sweep with teams of 512, 256 and 128; a batch of 64 problems of 8 to 32 hexes (about 140 units a group in its
-// first group steps) 779, 703 and 715 ms per solve.
-int choose_team(lb_batch* b, const std::vector<int>& ids) {
-    double units = 0.0, groups = 0.0, dirs = 0.0;
-    for (int p : ids) {
-        const lb_handle* h = b->probs[p];
-        dirs += h->NI;
-        if (h->nclusters > 0) {
-            units += (double)h->crec_base_h[h->NI];
-            groups += (double)h->cluster_levels_total;
-        } else {
-            units += (double)h->NE * h->NI;
-            groups += (double)h->total_levels;
+// first group steps) 779, 703 and 715 ms per solve.  Without tile types, ms per solve with teams of 512, 256 and 128: 8
+// problems of 8 to 20 hexes per axis jittered (19 units a group, their blocks split on cycles) 106, 101, 107, with 8
+// materials (55 units) 30, 24.9, 25.5, with shuffled elements (48 units) 178, 134, 127; 12 of 16 to 30 hexes with 8 materials
+// (189 units) 67.7, 68.6, 72.1; 12 of the 12,741-tet mesh (18 units) 136, 98, 66.5; a single one of 78,771 tets and 80
+// directions 25.9, 30.5, 36.2.  (CTAs of 1,024 threads: 26.0 there, 1.3 to 3 times as long elsewhere.)
+void choose_teams(lb_batch* b, const std::vector<int>& ids) {
+    const char* verbose = std::getenv("LB_SWEEP_VERBOSE");
+    for (const bool tiles : {true, false}) {
+        double units = 0.0, groups = 0.0, dirs = 0.0;
+        for (int p : ids) {
+            const lb_handle* h = b->probs[p];
+            if (h->tiles_ok != tiles) continue;
+            dirs += h->NI;
+            if (h->nclusters > 0) {
+                units += (double)h->crec_base_h[h->NI];
+                groups += (double)h->cluster_levels_total;
+            } else {
+                units += (double)h->NE * h->NI;
+                groups += (double)h->total_levels;
+            }
         }
+        const double mean = units / std::max(groups, 1.0);
+        int& team = tiles ? b->sweep.tile_team : b->sweep.walk_team;
+        team = kBatchThreads;
+        for (int t : {256, 128})
+            if (mean <= t && dirs >= (double)b->aux->sm_count * kBatchThreads / t) team = t;
+        if (dirs > 0.0 && verbose && *verbose == '1')
+            std::fprintf(stderr, "batched sweep: %s, %.0f directions, %.1f units a group -> teams of %d threads\n",
+                         tiles ? "block tiles" : "block and level walk", dirs, mean, team);
     }
-    const double mean = units / std::max(groups, 1.0);
-    for (int team : {128, 256})
-        if (mean <= team && dirs >= (double)b->aux->sm_count * kBatchThreads / team) return team;
-    return kBatchThreads;
 }
 
 // y_p = A x_p for every problem in ids (direct launches).  mode 0: y = x - D T^-1 M Sigma x
@@ -516,7 +535,7 @@ int ensure_batch_buffers(lb_batch* b, int m) {
         b->cap = P;
     }
     if (!b->d_counter) {
-        cudaError_t e = cudaMalloc(&b->d_counter, sizeof(int));
+        cudaError_t e = cudaMalloc(&b->d_counter, 2 * sizeof(int));
         if (e != cudaSuccess) return bcuda(b, e, "batch counter");
     }
     b->wa.resize(P, nullptr);
@@ -649,8 +668,8 @@ int lb_batch_solve(lb_batch* b, int m, double rtol, double atol, int maxit, int*
             if (b->probs[p]->G > g) ids.push_back(p);
         for (int p : ids)
             if ((rc = mg_group_sources(b->probs[p], g))) return prop_error(b, b->probs[p], rc, p);
-        b->sweep_team = choose_team(b, ids);
-        if ((rc = build_work(b, ids, b->sweep_team))) return rc;
+        choose_teams(b, ids);
+        if ((rc = build_work(b, ids))) return rc;
         // b = D T^{-1} M src for every problem of the step, then x = b
         cudaStreamSynchronize(s);
         std::fill(b->h_active, b->h_active + P, 0);
@@ -707,7 +726,7 @@ int lb_batch_info(lb_batch* b, int* nproblems, int* max_groups, double* last_ms,
     if (nproblems) *nproblems = (int)b->probs.size();
     if (max_groups) *max_groups = Gmax;
     if (last_ms) *last_ms = b->last_ms;
-    if (sweep_threads) *sweep_threads = b->sweep_team ? kBatchThreads : 0;
+    if (sweep_threads) *sweep_threads = b->sweep.nwork ? kBatchThreads : 0;
     if (graph_launches) *graph_launches = b->graph_launches;
     if (sweep_launches) *sweep_launches = b->sweep_launches;
     return LB_OK;

@@ -326,11 +326,19 @@ struct BatchWork {
     const float4* xtab;     // [nxtype][4] the problem's tile types
     const int* xmat;        // [nxtype] material of the tile types
 };
-// Sweeps every work item whose problem has active[problem] != 0, CTAs claiming items in order from
-// *counter (reset before the launch).  team: threads of a CTA that take an item (512, 256 or 128).
+// A batched sweep: items [0, ntile) of the work list have tile types, the others [ntile, nwork) have not.  Each part
+// is claimed in order from its counter by teams of threads of a CTA.
 constexpr int kBatchThreads = 512;   // threads per CTA, two CTAs per SM
-int launch_sweep_batch(cudaStream_t s, const BatchWork* work, int nwork, int* counter, const int* active, int team,
-                       int sm_count);
+struct BatchSweep {
+    const BatchWork* work = nullptr;
+    int nwork = 0, ntile = 0;
+    int* counter = nullptr;  // [2], reset by the launch
+    int tile_team = kBatchThreads;   // 512, 256 or 128 threads take an item
+    int walk_team = kBatchThreads;   // the same without tile types
+    int max_geom = 0;        // largest type table among the items without tile types
+};
+// Sweeps every work item whose problem has active[problem] != 0.
+int launch_sweep_batch(cudaStream_t s, const BatchSweep& b, const int* active, int sm_count);
 
 // Segmented (per-problem) FP64 vector operations of a batch: one launch for all problems.
 struct SegVec {

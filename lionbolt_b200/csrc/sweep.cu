@@ -1068,52 +1068,75 @@ __global__ void __launch_bounds__(2 * HT, MINB) sweep_relay_kernel(SweepArgs a) 
 // The TEAM threads that take an item are the whole CTA, or a quarter or half of it: the block levels of a batch's
 // small meshes (8 to 20 hexes per axis: at most a few hundred blocks) leave most of 512 threads idle, and a batch
 // has far more directions than the chip has CTAs, so smaller teams keep more directions in flight per SM.
+// Directions with tile types have a kernel of their own: together with the tile walk the others' registers spill at every
+// team size, and the rows of the tiles take shared memory from their L1 (one problem of 78,771 tets and 80 directions 28.1 ms
+// per solve in one kernel, 26.0 in its own; 12 of 16 to 30 hexes per axis with 8 materials 74.4 and 68.4).
 // ---------------------------------------------------------------------------------------------
-// Shared memory of a team: tile rows (or the face vectors of up to 256 element types), tile types and their
-// tables, cross sections.
-constexpr int batch_rows(int team) { return kTileRow * team > 3 * 256 ? kTileRow * team : 3 * 256; }
-constexpr size_t batch_team_smem(int team) {
-    return 16 * ((size_t)batch_rows(team) + 4 * kMaxTileTypes + 64) + sizeof(ElemTab) * kMaxTileTypes;
+// Shared memory of a team: tile rows, tile types and their tables, cross sections.
+constexpr size_t batch_tile_smem(int team) {
+    return 16 * ((size_t)kTileRow * team + 4 * kMaxTileTypes + kMaxTileTypes / 4) + sizeof(ElemTab) * kMaxTileTypes;
+}
+// The same without tiles: cross sections and the face vectors of the element types.
+constexpr size_t batch_walk_smem(int ngeom) { return 1024 + 48 * (size_t)ngeom; }
+
+// Work item number of the calling team, claimed in order; -1: none left.
+template <int TEAM>
+__device__ __forceinline__ int claim_item(int* slot, int* counter, int nwork, int team, int tt) {
+    if (tt == 0) *slot = atomicAdd(counter, 1);
+    team_sync<kBatchThreads, TEAM>(team);
+    const int w = *slot;
+    return w < nwork ? w : -1;
 }
 
 template <int TEAM>
-__global__ void __launch_bounds__(kBatchThreads, 2) sweep_batch_kernel(const BatchWork* __restrict__ work, int nwork,
-                                                                       int* counter, const int* __restrict__ active) {
+__global__ void __launch_bounds__(kBatchThreads, 2) sweep_batch_tiles_kernel(const BatchWork* __restrict__ work, int nwork,
+                                                                             int* counter, const int* __restrict__ active) {
     constexpr int NT = kBatchThreads;
     extern __shared__ float4 s_dyn[];
     __shared__ int s_work[NT / TEAM];
     const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
-    float4* s_gt = s_dyn + team * (batch_team_smem(TEAM) / 16);   // tile rows or element types
-    float4* s_x = s_gt + batch_rows(TEAM);
+    float4* s_tile = s_dyn + team * (batch_tile_smem(TEAM) / 16);
+    float4* s_x = s_tile + kTileRow * TEAM;
     ElemTab* s_tab = reinterpret_cast<ElemTab*>(s_x + 4 * kMaxTileTypes);
-    float* s_sigt = reinterpret_cast<float*>(s_tab + kMaxTileTypes);   // [256]
-    for (;;) {
-        if (tt == 0) s_work[team] = atomicAdd(counter, 1);
-        team_sync<NT, TEAM>(team);
-        const int w = s_work[team];
-        if (w >= nwork) return;
+    float* s_sigt = reinterpret_cast<float*>(s_tab + kMaxTileTypes);
+    for (int w; (w = claim_item<TEAM>(&s_work[team], counter, nwork, team, tt)) >= 0;) {
         const BatchWork* W = work + w;
-        const int prob = __ldg(&W->problem);
-        if (active && __ldg(&active[prob]) == 0) {
+        if (active && __ldg(&active[__ldg(&W->problem)]) == 0) {
+            team_sync<NT, TEAM>(team);
+            continue;
+        }
+        // as sweep_tile_kernel
+        const int nx = __ldg(&W->nxtype);
+        for (int k = tt; k < 4 * nx; k += TEAM) s_x[k] = __ldg(&W->xtab[k]);
+        for (int k = tt; k < nx; k += TEAM) s_sigt[k] = __ldg(&W->sigt[__ldg(&W->xmat[k])]);
+        team_sync<NT, TEAM>(team);
+        const float4 d = __ldg(&W->dir);
+        build_tab<true>(s_x, s_sigt, nx, d, s_tab, tt, TEAM);
+        team_sync<NT, TEAM>(team);
+        walk_tiles<NT, TEAM>(W->crec, W->cl_start, __ldg(&W->ncl), W->psi, d, s_x, s_sigt, s_tab, s_tile, team);
+    }
+}
+
+template <int TEAM>
+__global__ void __launch_bounds__(kBatchThreads, 2) sweep_batch_kernel(const BatchWork* __restrict__ work, int nwork,
+                                                                       int* counter, const int* __restrict__ active,
+                                                                       int max_geom) {
+    constexpr int NT = kBatchThreads;
+    extern __shared__ float4 s_dyn[];
+    __shared__ int s_work[NT / TEAM];
+    const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
+    float* s_sigt = reinterpret_cast<float*>(s_dyn + team * (batch_walk_smem(max_geom) / 16));   // [256]
+    float4* s_gt = reinterpret_cast<float4*>(s_sigt + 256);   // the item's element types (face vectors)
+    for (int w; (w = claim_item<TEAM>(&s_work[team], counter, nwork, team, tt)) >= 0;) {
+        const BatchWork* W = work + w;
+        if (active && __ldg(&active[__ldg(&W->problem)]) == 0) {
             team_sync<NT, TEAM>(team);
             continue;
         }
         const int Nm = __ldg(&W->Nm);
         const float* sg = W->sigt;
         const int ngeom = __ldg(&W->ngeom);
-        const int nx = __ldg(&W->nxtype);
         const int4* crec = W->crec;
-        if (nx > 0) {
-            // block tiles, as sweep_tile_kernel
-            for (int k = tt; k < 4 * nx; k += TEAM) s_x[k] = __ldg(&W->xtab[k]);
-            for (int k = tt; k < nx; k += TEAM) s_sigt[k] = __ldg(&sg[__ldg(&W->xmat[k])]);
-            team_sync<NT, TEAM>(team);
-            const float4 d = __ldg(&W->dir);
-            build_tab<true>(s_x, s_sigt, nx, d, s_tab, tt, TEAM);
-            team_sync<NT, TEAM>(team);
-            walk_tiles<NT, TEAM>(crec, W->cl_start, __ldg(&W->ncl), W->psi, d, s_x, s_sigt, s_tab, s_gt, team);
-            continue;
-        }
         // cross sections by material, or by element type when the problem has a type table
         for (int m = tt; m < 256; m += TEAM) {
             float v = 0.f;
@@ -1634,27 +1657,43 @@ cudaError_t launch_levels_pf(const SweepArgs& a, int threads, int sm_count, cuda
 
 }  // namespace
 
-int launch_sweep_batch(cudaStream_t st, const BatchWork* work, int nwork, int* counter, const int* active, int team,
-                       int sm_count) {
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
+int launch_sweep_batch(cudaStream_t st, const BatchSweep& b, const int* active, int sm_count) {
+    cudaError_t e = cudaMemsetAsync(b.counter, 0, 2 * sizeof(int), st);
     if (e != cudaSuccess) return LB_ERR_CUDA;
-    auto run = [&](auto kernel, PerDevice& cache) {
-        const int teams = kBatchThreads / team;
-        const size_t smem = batch_team_smem(team) * teams;
-        const int per_sm = cache.get([&] {
-            int n = 0;
+    auto grid = [&](auto kernel, int n, int team, size_t smem, PerDevice& attr) {
+        attr.get([&] {
             allow_max_dynamic_smem(kernel);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBatchThreads, smem);
-            return n < 1 ? 1 : n;
+            return 1;
         });
-        kernel<<<std::min((nwork + teams - 1) / teams, sm_count * per_sm), kBatchThreads, smem, st>>>(work, nwork, counter,
-                                                                                                  active);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchThreads, smem);
+        const int teams = kBatchThreads / team;
+        return std::min((n + teams - 1) / teams, sm_count * std::max(per_sm, 1));
     };
-    static PerDevice cache[3];
-    if (team == 512) run(sweep_batch_kernel<512>, cache[0]);
-    else if (team == 256) run(sweep_batch_kernel<256>, cache[1]);
-    else if (team == 128) run(sweep_batch_kernel<128>, cache[2]);
-    else return LB_ERR_ARG;
+    auto tiles = [&](auto kernel, PerDevice& attr) {
+        const size_t smem = batch_tile_smem(b.tile_team) * (kBatchThreads / b.tile_team);
+        kernel<<<grid(kernel, b.ntile, b.tile_team, smem, attr), kBatchThreads, smem, st>>>(b.work, b.ntile, b.counter,
+                                                                                         active);
+    };
+    const int nwalk = b.nwork - b.ntile;
+    auto walk = [&](auto kernel, PerDevice& attr) {
+        const size_t smem = batch_walk_smem(b.max_geom) * (kBatchThreads / b.walk_team);
+        kernel<<<grid(kernel, nwalk, b.walk_team, smem, attr), kBatchThreads, smem, st>>>(b.work + b.ntile, nwalk,
+                                                                                       b.counter + 1, active, b.max_geom);
+    };
+    static PerDevice attr[6];
+    if (nwalk > 0) {
+        if (b.walk_team == 512) walk(sweep_batch_kernel<512>, attr[0]);
+        else if (b.walk_team == 256) walk(sweep_batch_kernel<256>, attr[1]);
+        else if (b.walk_team == 128) walk(sweep_batch_kernel<128>, attr[2]);
+        else return LB_ERR_ARG;
+    }
+    if (b.ntile > 0) {
+        if (b.tile_team == 512) tiles(sweep_batch_tiles_kernel<512>, attr[3]);
+        else if (b.tile_team == 256) tiles(sweep_batch_tiles_kernel<256>, attr[4]);
+        else if (b.tile_team == 128) tiles(sweep_batch_tiles_kernel<128>, attr[5]);
+        else return LB_ERR_ARG;
+    }
     return cudaGetLastError() == cudaSuccess ? LB_OK : LB_ERR_CUDA;
 }
 

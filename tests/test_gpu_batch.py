@@ -77,3 +77,64 @@ def test_batch_info_before_and_after_the_first_solve():
     bs.solve(m=10, rtol=1e-4)
     info = bs.info()
     assert info["sweep_threads"] > 0 and info["sweep_launches"] > 0
+
+
+def _walk_mesh(kind):
+    """Meshes without tile types, by what their directions are walked by."""
+    from helpers import jittered
+    from lionbolt_b200 import mesh as M
+    n = (6, 5, 7)
+    box = M.box_mesh(*n, (0, 0, 0), (3.0, 2.5, 3.5), material=lambda c: np.minimum(c[:, 2] / 0.4375, 7).astype(np.int32), Nm=8)
+    if kind == "type table":                 # 48 shape and material types: more than tiles have
+        return box
+    if kind == "split blocks":               # every element a shape of its own, blocks split on cycles
+        return jittered(box, 0.035)
+    if kind == "member table":               # elements in no order: blocks listed element by element
+        p = np.random.default_rng(2).permutation(box.NE)
+        node = box.node[p]
+        return M.Mesh(rg=box.rg, node=node, neighbors=M.neighbours(node), mat=box.mat[p], Nm=8)
+    node = box.node[:5]                      # fewer elements than a block has
+    return M.Mesh(rg=box.rg, node=node, neighbors=M.neighbours(node), mat=box.mat[:5], Nm=8)
+
+
+def _walk_problem(kind, seed):
+    m = _walk_mesh(kind)
+    k, w = P.quadrature(8, 10)
+    r = np.random.default_rng(seed)
+    st = r.uniform(0.2, 1.0, size=(1, 8))
+    sigs = 0.8 * st[None, :, :, None] * 0.5 ** np.arange(2)
+    return P.Problem(kind, m, k, w, 8, 10, 1, 1, st, sigs, 0.2 * st, r.uniform(size=m.NENK), np.array([0.0, 0.0, 1.0]))
+
+
+def _check_against_single(probs, which):
+    bs = BatchSolver()
+    for p in probs:
+        bs.add_problem(p)
+    bs.solve(m=20, rtol=1e-7, maxit=200)
+    for i in which:
+        mg = MultigroupSolver().set_problem(probs[i])
+        mg.solve("GMRES", m=20, rtol=1e-7, maxit=200)
+        assert rel_l2(bs.results(i)[1], mg.results()[1]) < 1e-6
+
+
+@pytest.mark.parametrize("count,team", [(2, 512), (4, 256), (8, 128)])
+@pytest.mark.parametrize("kind", ["type table", "split blocks", "member table", "no blocks"])
+def test_batched_walks_match_single_solves(kind, count, team, monkeypatch, capfd):
+    """Every walk of the batched sweep, by teams of every size (80 directions a problem, 148 SMs): reduction order inside
+    GMRES, 1e-6."""
+    monkeypatch.setenv("LB_SWEEP_VERBOSE", "1")
+    _check_against_single([_walk_problem(kind, s) for s in range(count)], (0, count - 1))
+    assert f"block and level walk, {80 * count} directions" in (err := capfd.readouterr().err)
+    assert f"teams of {team} threads" in err
+
+
+def test_batch_of_tiled_and_other_problems_matches_single_solves(monkeypatch, capfd):
+    """Two kernels share a sweep: problems with tile types and without, in turns."""
+    monkeypatch.setenv("LB_SWEEP_VERBOSE", "1")
+    probs = []
+    for s, kind in enumerate(("type table", "split blocks", "member table", "no blocks")):
+        probs += [_walk_problem(kind, s), P.multigroup_box(n=(4 + s, 4, 6), size=(2.0 + 0.5 * s, 2.0, 3.0), Ng=4, Nc=8, G=2,
+                                                           Ls=2, seed=s, slab=(0.5, 1.5))]
+    _check_against_single(probs, range(len(probs)))
+    err = capfd.readouterr().err
+    assert "block tiles, 128 directions" in err and "block and level walk, 320 directions" in err
