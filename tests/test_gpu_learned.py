@@ -201,3 +201,25 @@ def test_gradient_at_the_edges_of_its_sample_tiles(n):
     assert rel_l2(g, gref) < 2e-3
     again = op.lp_loss_grad(x, t, wt)
     assert again[0] == loss and np.array_equal(again[1], g)     # fixed summation order
+
+
+@pytest.mark.parametrize("call", ["forward", "gradient"])
+def test_a_large_batch_is_given_back(call):
+    """2,000,000 samples take 288 MB on the device while the call runs; the handle keeps no more than 256 MB, so none of it."""
+    torch = pytest.importorskip("torch")
+    op = TransportOp()
+    op.lp_set_weights(_random_weights(5))
+
+    def run(n):
+        x = np.full((n, 19), 0.5, dtype=np.float32)
+        if call == "forward":
+            return op.lp_forward(x)
+        return op.lp_loss_grad(x, np.zeros((n, 16), np.float32))[1]
+
+    first = run(20000)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    big = run(2000000)
+    assert np.all(np.isfinite(big)) and np.all(np.isfinite(first))
+    assert before - torch.cuda.mem_get_info()[0] < 32 << 20
+    assert np.all(np.isfinite(run(20000)))
