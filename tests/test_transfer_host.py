@@ -78,7 +78,7 @@ def lib(tmp_path_factory):
     (d / "fake.cpp").write_text(FAKE)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cxx = "/usr/bin/g++" if os.access("/usr/bin/g++", os.X_OK) else "g++"      # as the Makefile
-    subprocess.check_call([cxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-fopenmp", f"-I{CSRC}",
+    subprocess.check_call([cxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-fopenmp", f"-I{CSRC}",
                            f"-I{cuda}/include", str(d / "fake.cpp"), os.path.join(CSRC, "transfer.cpp"), "-o",
                            str(d / "libfake.so")])
     lib = ctypes.CDLL(str(d / "libfake.so"))
