@@ -204,6 +204,95 @@ static bool build_direction(const Handle* h, int i, int* items, std::vector<int>
     return es == NE;
 }
 
+// ---- tables of the sweep schedules that neither the rule nor the autotuner takes (LB_SWEEP_CONFIG runs them), made by their
+// first launch for a quadrature: at 768,000 tets and 288 directions they are 1.0 of 6.1 GB on the device and 0.5 of 3.7 s ----
+
+// Dataflow: chunk list, level-major across directions: every chunk's dependencies (the previous level
+// of its own direction) precede it, so claiming chunks in order can never deadlock.
+int chunk_tables(Handle* h) {
+    if (h->d_chunks && h->d_done) return LB_OK;
+    const int NI = h->NI;
+    // global level ids: gid(i, L) = sum_{i'<i} nlev[i'] + L
+    std::vector<int> gbase(NI + 1, 0);
+    for (int i = 0; i < NI; ++i) gbase[i + 1] = gbase[i] + h->nlev[i];
+    const int maxlev = *std::max_element(h->nlev.begin(), h->nlev.end());
+    std::vector<int4> chunks;
+    chunks.reserve(h->nchunks);
+    for (int L = 0; L < maxlev; ++L)
+        for (int i = 0; i < NI; ++i) {
+            if (L >= h->nlev[i]) continue;
+            const int* st = &h->lvl_start[h->lvl_base[i]];
+            int a = st[L], b = st[L + 1];
+            int prev = (L > 0) ? (st[L] - st[L - 1]) : 0;
+            for (int s = a; s < b; s += 32) {
+                int n = std::min(32, b - s);
+                chunks.push_back(make_int4(i | ((n - 1) << 24), s, gbase[i] + L, prev));
+            }
+        }
+    const int rc = dev_upload(h, &h->d_chunks, chunks.data(), chunks.size(), "upload sweep chunks");
+    return rc ? rc : dev_alloc(h, &h->d_done, (size_t)h->total_levels, "level counters");
+}
+
+// Element flags: items with every level padded to a multiple of 32 (padding = -1): a 32-element chunk of the
+// padded order never spans two levels, so its elements never depend on each other.
+int padded_tables(Handle* h) {
+    if (h->d_pitems && h->d_pbase) return LB_OK;
+    const int NI = h->NI, NE = h->NE;
+    std::vector<long long> pbase(NI + 1, 0);
+    for (int i = 0; i < NI; ++i) {
+        long long len = 0;
+        const int* st = &h->lvl_start[h->lvl_base[i]];
+        for (int L = 0; L < h->nlev[i]; ++L) len += ((st[L + 1] - st[L]) + 31) / 32 * 32;
+        pbase[i + 1] = pbase[i] + len;
+    }
+    std::vector<int> pitems((size_t)pbase[NI], -1);
+#pragma omp parallel for schedule(dynamic, 4)
+    for (int i = 0; i < NI; ++i) {
+        const int* st = &h->lvl_start[h->lvl_base[i]];
+        long long o = pbase[i];
+        for (int L = 0; L < h->nlev[i]; ++L) {
+            for (int es = st[L]; es < st[L + 1]; ++es) pitems[(size_t)o++] = h->items[(size_t)i * NE + es];
+            o = pbase[i] + (o - pbase[i] + 31) / 32 * 32;
+        }
+    }
+    const int rc = dev_upload(h, &h->d_pitems, pitems.data(), pitems.size(), "upload padded items");
+    return rc ? rc : dev_upload(h, &h->d_pbase, pbase.data(), pbase.size(), "upload padded offsets");
+}
+
+// Grouped directions: classes of directions with identical schedules (exact comparison after a hash).
+void direction_classes(Handle* h) {
+    if (!h->class_start.empty()) return;
+    const int NI = h->NI, NE = h->NE;
+    std::vector<unsigned long long> hsh(NI);
+#pragma omp parallel for schedule(static)
+    for (int i = 0; i < NI; ++i) {
+        unsigned long long x = 1469598103934665603ULL ^ (unsigned long long)h->nlev[i];
+        const int* it = &h->items[(size_t)i * NE];
+        for (int es = 0; es < NE; ++es) { x ^= (unsigned)it[es]; x *= 1099511628211ULL; }
+        hsh[i] = x;
+    }
+    std::vector<int> cls(NI, -1);   // smallest direction of the class
+    for (int i = 0; i < NI; ++i) {
+        if (cls[i] >= 0) continue;
+        cls[i] = i;
+        for (int j = i + 1; j < NI; ++j) {
+            if (cls[j] >= 0 || hsh[j] != hsh[i] || h->nlev[j] != h->nlev[i]) continue;
+            if (std::memcmp(&h->items[(size_t)i * NE], &h->items[(size_t)j * NE], sizeof(int) * (size_t)NE) == 0 &&
+                std::equal(&h->lvl_start[h->lvl_base[i]], &h->lvl_start[h->lvl_base[i]] + h->nlev[i] + 1,
+                           &h->lvl_start[h->lvl_base[j]]))
+                cls[j] = i;
+        }
+    }
+    h->class_members.clear();
+    h->class_start.assign(1, 0);
+    for (int i = 0; i < NI; ++i) {
+        if (cls[i] != i) continue;
+        for (int j = i; j < NI; ++j)
+            if (cls[j] == i) h->class_members.push_back(j);
+        h->class_start.push_back((int)h->class_members.size());
+    }
+}
+
 }  // namespace lb
 
 using namespace lb;
@@ -984,36 +1073,31 @@ int lb_set_quadrature(lb_handle* h, int NI, const double* k, const double* w) {
     h->lvl_base.assign(NI + 1, 0);
     h->lvl_start.clear();
     h->nz_upstream = 0;
-    int maxlev = 0;
     for (int i = 0; i < NI; ++i) {
         h->nlev[i] = (int)starts[i].size() - 1;
         h->lvl_base[i] = (int)h->lvl_start.size();
         h->lvl_start.insert(h->lvl_start.end(), starts[i].begin(), starts[i].end());
         h->nz_upstream += nz[i];
-        maxlev = std::max(maxlev, h->nlev[i]);
     }
     h->lvl_base[NI] = (int)h->lvl_start.size();
-    // global level ids: gid(i, L) = sum_{i'<i} nlev[i'] + L
-    std::vector<int> gbase(NI + 1, 0);
-    for (int i = 0; i < NI; ++i) gbase[i + 1] = gbase[i] + h->nlev[i];
-    h->total_levels = gbase[NI];
-    // chunk list, level-major across directions: every chunk's dependencies (the previous level
-    // of its own direction) precede it, so claiming chunks in order can never deadlock.
-    std::vector<int4> chunks;
-    chunks.reserve((size_t)NI * NE / 24 + 16);
-    for (int L = 0; L < maxlev; ++L)
-        for (int i = 0; i < NI; ++i) {
-            if (L >= h->nlev[i]) continue;
-            const int* st = &h->lvl_start[h->lvl_base[i]];
-            int a = st[L], b = st[L + 1];
-            int prev = (L > 0) ? (st[L] - st[L - 1]) : 0;
-            for (int s = a; s < b; s += 32) {
-                int n = std::min(32, b - s);
-                chunks.push_back(make_int4(i | ((n - 1) << 24), s, gbase[i] + L, prev));
-            }
-        }
-    if (chunks.size() >= (size_t)INT32_MAX) return fail(h, LB_ERR_ARG, "lb_set_quadrature: problem too large");
-    h->nchunks = (int)chunks.size();
+    h->total_levels = 0;
+    for (int i = 0; i < NI; ++i) h->total_levels += h->nlev[i];
+    // 32-element chunks of the levels (chunk_tables)
+    long long nchunks = 0;
+    for (int i = 0; i < NI; ++i) {
+        const int* st = &h->lvl_start[h->lvl_base[i]];
+        for (int L = 0; L < h->nlev[i]; ++L) nchunks += (st[L + 1] - st[L] + 31) / 32;
+    }
+    if (nchunks >= (long long)INT32_MAX) return fail(h, LB_ERR_ARG, "lb_set_quadrature: problem too large");
+    h->nchunks = (int)nchunks;
+    // tables made by the first launch that asks for them
+    for (void** p : {(void**)&h->d_chunks, (void**)&h->d_done, (void**)&h->d_pitems, (void**)&h->d_pbase}) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+    }
+    h->class_start.clear();
+    h->groups_gmax = 0;
+    h->ngroups = 0;
     // Execution order on the device: inside every level the elements are grouped by upstream-face
     // mask (ascending element id within a group).  Elements of a level are independent, so the
     // results do not change, but a warp then runs the face bodies of about 2 upstream faces instead
@@ -1036,75 +1120,12 @@ int lb_set_quadrature(lb_handle* h, int NI, const double* k, const double* w) {
     if (rc) return rc;
     rc = build_cluster_schedule(h);
     if (rc) return rc;
-    rc = dev_upload(h, &h->d_chunks, chunks.data(), chunks.size(), "upload sweep chunks");
-    if (rc) return rc;
-    rc = dev_alloc(h, &h->d_done, (size_t)h->total_levels, "level counters");
-    if (rc) return rc;
-    {
-        // items with every level padded to a multiple of 32 (padding = -1): a 32-element chunk of the
-        // padded order never spans two levels, so its elements never depend on each other
-        std::vector<long long> pbase(NI + 1, 0);
-        for (int i = 0; i < NI; ++i) {
-            long long len = 0;
-            const int* st = &h->lvl_start[h->lvl_base[i]];
-            for (int L = 0; L < h->nlev[i]; ++L) len += ((st[L + 1] - st[L]) + 31) / 32 * 32;
-            pbase[i + 1] = pbase[i] + len;
-        }
-        std::vector<int> pitems((size_t)pbase[NI], -1);
-#pragma omp parallel for schedule(dynamic, 4)
-        for (int i = 0; i < NI; ++i) {
-            const int* st = &h->lvl_start[h->lvl_base[i]];
-            long long o = pbase[i];
-            for (int L = 0; L < h->nlev[i]; ++L) {
-                for (int es = st[L]; es < st[L + 1]; ++es) pitems[(size_t)o++] = h->items[(size_t)i * NE + es];
-                o = pbase[i] + (o - pbase[i] + 31) / 32 * 32;
-            }
-        }
-        h->npitems = pbase[NI];
-        rc = dev_upload(h, &h->d_pitems, pitems.data(), pitems.size(), "upload padded items");
-        if (rc) return rc;
-        rc = dev_upload(h, &h->d_pbase, pbase.data(), pbase.size(), "upload padded offsets");
-        if (rc) return rc;
-    }
     rc = dev_upload(h, &h->d_lvl_start, h->lvl_start.data(), h->lvl_start.size(), "upload level starts");
     if (rc) return rc;
     rc = dev_upload(h, &h->d_lvl_base, h->lvl_base.data(), h->lvl_base.size(), "upload level offsets");
     if (rc) return rc;
     rc = dev_upload(h, &h->d_nlev, h->nlev.data(), h->nlev.size(), "upload level counts");
     if (rc) return rc;
-    {
-        // classes of directions with identical schedules (exact comparison after a hash)
-        std::vector<unsigned long long> hsh(NI);
-#pragma omp parallel for schedule(static)
-        for (int i = 0; i < NI; ++i) {
-            unsigned long long x = 1469598103934665603ULL ^ (unsigned long long)h->nlev[i];
-            const int* it = &h->items[(size_t)i * NE];
-            for (int es = 0; es < NE; ++es) { x ^= (unsigned)it[es]; x *= 1099511628211ULL; }
-            hsh[i] = x;
-        }
-        h->dir_class.assign(NI, -1);
-        for (int i = 0; i < NI; ++i) {
-            if (h->dir_class[i] >= 0) continue;
-            h->dir_class[i] = i;
-            for (int j = i + 1; j < NI; ++j) {
-                if (h->dir_class[j] >= 0 || hsh[j] != hsh[i] || h->nlev[j] != h->nlev[i]) continue;
-                if (std::memcmp(&h->items[(size_t)i * NE], &h->items[(size_t)j * NE], sizeof(int) * (size_t)NE) == 0 &&
-                    std::equal(&h->lvl_start[h->lvl_base[i]], &h->lvl_start[h->lvl_base[i]] + h->nlev[i] + 1,
-                               &h->lvl_start[h->lvl_base[j]]))
-                    h->dir_class[j] = i;
-            }
-        }
-        h->class_members.clear();
-        h->class_start.assign(1, 0);
-        for (int i = 0; i < NI; ++i) {
-            if (h->dir_class[i] != i) continue;
-            for (int j = i; j < NI; ++j)
-                if (h->dir_class[j] == i) h->class_members.push_back(j);
-            h->class_start.push_back((int)h->class_members.size());
-        }
-        h->groups_gmax = 0;
-        h->ngroups = 0;
-    }
     h->sweep_cfg = -1;
     h->sweep_trial = 0;
     h->sweep_trial_ms.clear();

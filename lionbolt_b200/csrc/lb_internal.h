@@ -137,20 +137,19 @@ struct Handle {
     std::vector<int4> crec_h;                        // the block records (host-only handles)
     int* d_mat = nullptr;          // [NE]
     int* d_items = nullptr;        // [NI][NE]
+    // tables of schedules that run only under LB_SWEEP_CONFIG, null until their first launch (host.cpp)
     int4* d_chunks = nullptr;      // [nchunks]
     int* d_pitems = nullptr;       // padded items: every level of every direction padded to 32 with -1
     long long* d_pbase = nullptr;  // [NI+1] start of each direction in d_pitems
-    long long npitems = 0;
+    int* d_done = nullptr;         // [total_levels]
     // directions whose schedules are bit-identical (same order, same face masks) share a walk
-    std::vector<int> dir_class;    // [NI] class representative (smallest direction id of the class)
     std::vector<int> class_members;  // directions sorted by class
-    std::vector<int> class_start;    // [nclass+1]
+    std::vector<int> class_start;    // [nclass+1] (empty until needed)
     int* d_groups = nullptr;       // per-CTA groups for the grouped sweep, built per group size
     int groups_gmax = 0, ngroups = 0;
     int* d_lvl_start = nullptr;    // concatenated level starts (copy of lvl_start)
     int* d_lvl_base = nullptr;     // [NI+1]
     int* d_nlev = nullptr;         // [NI]
-    int* d_done = nullptr;         // [total_levels]
     SweepStatus* d_status = nullptr;
     int* d_tc_err = nullptr;      // set to LB_ERR_TIMEOUT by a contraction kernel whose pipeline wait gave up (pinned
                                   // host memory, written by the device only then: reading it costs no copy)
@@ -385,6 +384,10 @@ void timers_flush(Handle* h);
 // ---- kernels (sweep.cu / moments.cu / krylov.cu) ----
 // Full transport sweep psi <- T^{-1} psi (FP32, in place, natural layout [NI][NENK]).
 int launch_sweep(Handle* h, float* psi);
+// tables made on first use (host.cpp): dataflow chunks, padded items, classes of directions
+int chunk_tables(Handle* h);
+int padded_tables(Handle* h);
+void direction_classes(Handle* h);
 // Chosen sweep launch shape (-1 while the autotuner is still timing candidates).
 int sweep_config(Handle* h, int* kind, int* threads, int* dpc, int* ilp);
 // q[i][n] = sum_j Y_j(k_i) * (sigl[mat(n)][j] * x[j][n] + a[j][n]) (+ qadd[i][n] if given).

@@ -28,7 +28,8 @@
 //    CTA barrier between levels; upstream values written by the same SM are re-read through its L1.
 //  * levels with next-level prefetch, element flags in shared memory, grouped same-schedule
 //    directions, and dataflow (warps claim 32-element chunks from a global counter and wait, with a
-//    bounded spin, on the completion counter of the previous level): candidates for other meshes.
+//    bounded spin, on the completion counter of the previous level): not tried by the autotuner any more (they came
+//    first on no mesh measured); LB_SWEEP_CONFIG runs them.
 // Meshes of hexes split along their main diagonal take the tile schedule or the resident relay; elsewhere the launch shape
 // (schedule, threads per CTA, directions or CTAs per SM, updates in flight per thread) is picked by timing the
 // first sweeps of a handle (the three fastest twice).  Every candidate computes bit-identical results.
@@ -1545,6 +1546,7 @@ cudaError_t launch_group(const SweepArgs& a, const int* groups, int ngroups, int
 // per-CTA groups of at most gmax directions with identical schedules
 int build_groups(Handle* h, int gmax) {
     if (h->groups_gmax == gmax && h->d_groups) return LB_OK;
+    direction_classes(h);
     std::vector<int> gr;
     int ng = 0;
     for (size_t c = 0; c + 1 < h->class_start.size(); ++c) {
@@ -1788,7 +1790,6 @@ Config runnable(const Handle* h, Config cfg, bool forced) {
 }  // namespace
 
 int launch_sweep(Handle* h, float* psi) {
-    const SweepArgs a = sweep_args(h, psi);
     if (h->sweep_cfg_forced < 0) {
         const char* env = std::getenv("LB_SWEEP_CONFIG");
         h->sweep_cfg_forced = (env && *env) ? std::atoi(env) : kNumConfigs;
@@ -1818,6 +1819,11 @@ int launch_sweep(Handle* h, float* psi) {
     // the element-flag schedule keeps one bit per element in shared memory
     if (cfg.kind == 3 && (size_t)((h->NE + 31) / 32) * 4 > 200 * 1024) cfg = Config{0, 1024, 1, 1};
 
+    if (cfg.kind == 1 || cfg.kind == 3) {
+        const int rc = cfg.kind == 1 ? chunk_tables(h) : padded_tables(h);
+        if (rc) return rc;
+    }
+    const SweepArgs a = sweep_args(h, psi);
     cudaError_t e = cudaSuccess;
     if (cfg.kind == 1) {
         e = cudaMemsetAsync(h->d_done, 0, sizeof(int) * (size_t)h->total_levels, h->stream);

@@ -291,3 +291,35 @@ def test_gmres_stagnation_below_the_fp32_floor_is_reported():
         mg.solve("GMRES", m=20, rtol=1e-8)
     assert ei.value.status == _lib.LB_ERR_NOCONV and "stagnated" in str(ei.value)
     assert time.perf_counter() - t0 < 20
+
+
+@pytest.mark.parametrize("cfg", range(14))
+def test_tables_of_a_forced_schedule_follow_the_quadrature(cfg, monkeypatch):
+    """The schedules that only LB_SWEEP_CONFIG runs make their tables at their first launch: again after another quadrature
+    and after another mesh."""
+    monkeypatch.setenv("LB_SWEEP_CONFIG", str(cfg))
+    m, (k, w), sigt, sigs = SWEEP_CASES["two_material"]()
+    T = TransportOp()
+    for mesh, quad in ((m, (k, w)), (m, P.quadrature(2, 6)), (M.box_mesh(3, 5, 4, (0, 0, 0), (1, 2, 1), Nm=2), P.quadrature(4, 4))):
+        o, ang, xs = _pair(mesh, *quad, sigt, sigs)
+        T.Build(mesh, ang, xs)
+        q = np.random.default_rng(cfg).uniform(0.0, 1.0, size=mesh.NENK * quad[0].shape[0])
+        for _ in range(2):
+            out = q.copy()
+            T.MatInv(out)
+            assert rel_l2(out, o.transport_inv(q)) < TOL
+
+
+def test_a_handle_holds_only_the_tables_it_sweeps_with():
+    """Per direction and element: the angular vector (16 bytes), the level order (4) and the block records (16 for six);
+    no tables of schedules that are not taken."""
+    torch = pytest.importorskip("torch")
+    torch.zeros(1, device="cuda:0")
+    box = M.box_mesh(16, 16, 20, (0, 0, 0), (1, 1, 1), Nm=1)
+    k, w = P.quadrature(12, 24)
+    warm = TransportOp().Build(M.box_mesh(2, 2, 2, (0, 0, 0), (1, 1, 1)), AngularClass(k=k, w=w), XSType(np.ones(1), np.zeros((1, 1))))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    T = TransportOp().Build(box, AngularClass(k=k, w=w), XSType(np.ones(1), np.zeros((1, 1))))
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used < 23 * box.NE * len(w) + (16 << 20)
