@@ -129,3 +129,31 @@ def test_level_relay_is_bit_identical_to_element_levels(cfg, n, amount, monkeypa
     T, v = _sweep(monkeypatch, cfg, m, k, w, sigt, q)
     assert T._h.sweep_config()["schedule"] == ("resident level relay" if cfg == 27 and m.NE <= 14000 else "level relay")
     assert np.array_equal(v, _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)[1])
+
+
+@pytest.mark.parametrize("group", [1024, 700, 0])
+def test_tile_sweep_with_several_passes_in_a_group(group, monkeypatch):
+    """Groups of more units than the CTA has threads (levels of up to some 740 here): the second pass starts without a
+    barrier, its last warps are part empty."""
+    monkeypatch.setenv("LB_CLUSTER_GROUP", str(group))
+    m = M.box_mesh(32, 32, 30, (0, 0, 0), (2.0, 1.5, 2.5), material=_two, Nm=2)
+    k, w = P.quadrature(2, 6)
+    sigt = np.array([0.3, 1.7])
+    q = np.random.default_rng(group).uniform(size=m.NENK * len(w))
+    T, v = _sweep(monkeypatch, 24, m, k, w, sigt, q)
+    assert T._h.sweep_config()["schedule"] == "block tiles"
+    assert np.array_equal(v, _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)[1])
+
+
+@pytest.mark.parametrize("cfg", [24, 25, 27])
+@pytest.mark.parametrize("n", [(5, 4, 3), (15, 14, 16)])
+def test_more_directions_than_resident_ctas(n, cfg, monkeypatch):
+    """320 directions on 148 SMs with two CTAs each: CTAs walk a second direction with the tables and rows of the first
+    still in place.  (The larger mesh does not fit the resident relay twice an SM.)"""
+    m = M.box_mesh(*n, (0, 0, 0), (2.0, 1.5, 2.5), material=_two, Nm=2)
+    k, w = P.quadrature(16, 20)
+    sigt = np.array([0.3, 1.7])
+    q = np.random.default_rng(cfg).uniform(size=m.NENK * len(w))
+    T, v = _sweep(monkeypatch, cfg, m, k, w, sigt, q)
+    assert T._h.sweep_config()["schedule"] in ("block tiles", "level relay", "resident level relay")
+    assert np.array_equal(v, _sweep(monkeypatch, LEVELS, m, k, w, sigt, q)[1])
