@@ -138,3 +138,13 @@ def test_batch_of_tiled_and_other_problems_matches_single_solves(monkeypatch, ca
     _check_against_single(probs, range(len(probs)))
     err = capfd.readouterr().err
     assert "block tiles, 128 directions" in err and "block and level walk, 320 directions" in err
+
+
+@pytest.mark.parametrize("count,team", [(2, 512), (4, 256), (8, 128)])
+def test_batched_tiles_run_the_teams_they_are_meant_to(count, team, monkeypatch, capfd):
+    monkeypatch.setenv("LB_SWEEP_VERBOSE", "1")
+    probs = [P.multigroup_box(n=(5, 4, 6), size=(2.5, 2.0, 3.0), Ng=8, Nc=10, G=1, Ls=2, seed=s, slab=(0.5, 1.5))
+             for s in range(count)]
+    _check_against_single(probs, (0, count - 1))
+    err = capfd.readouterr().err
+    assert f"block tiles, {80 * count} directions" in err and f"teams of {team} threads" in err
