@@ -234,7 +234,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
 // and read by six products 110 KB, B 83 KB, the output staged 147 KB): 3,500 of its 5,400 clocks at 288 directions and
 // P5.  A in tensor memory leaves 300 KB.  At 3,072,000 nodes a first call fell from 1.00 to 0.96 ms; repeated without
 // a pause the chip's power limit holds the clock down and it is 1.029 ms against 1.051.  168 directions at P7 (192,000
-// nodes): 67 us against 81, since one part of the directions now holds them all; 288 at P7: 100 against 128.
+// nodes): 67 us against 79; 288 at P7: 99 against 126.
 // ---------------------------------------------------------------------------------------------
 constexpr int kM2dEpi = 12;                          // epilogue warps (three per TMEM lane quarter)
 constexpr int kM2dMma = 8 + kM2dEpi;                 // the MMA warp
@@ -736,7 +736,8 @@ __global__ void __launch_bounds__(kD2mThreads, 1) d2m_tc_kernel(const int* __res
 // 288 directions at the SM's 128 bytes per clock; without the A planes it is half.  The A stages use what the two tile
 // accumulators (3 nmpad columns each) leave of the 512 TMEM columns, 48 columns a stage.
 // Measured there: a first call 0.87 ms against 0.93, repeated without a pause (the chip's power limit then holds the
-// clock down) 0.992 against 1.049; 192,000 nodes, 288 directions, P5: 71 us against 75.
+// clock down) 0.992 against 1.049; 192,000 nodes, 288 directions, P5: 71 us against 75.  The vote of a converter warp on its
+// waits (below) costs 1 % of a first call there, 2 % at 168 directions and P3 (0.276 ms at 1,536,000 nodes against 0.270).
 // Every wait is bounded (error flag), as in the other kernels.  No cluster, no multicast.
 // ---------------------------------------------------------------------------------------------
 constexpr int kKT = 32;        // directions per K chunk

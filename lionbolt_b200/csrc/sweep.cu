@@ -1946,7 +1946,8 @@ int sweep_config(Handle* h, int* kind, int* threads, int* dpc, int* ilp) {
 //  needs completion counters and took 4.5 ms against 0.30 ms at 57,456 tets and 288 directions.)
 //
 //  The call is synchronous on the handle's stream, and writes to psi issued on other streams must be complete
-//  before it.  Schedules of more than kNoAllocMaxLevels (direction, level) pairs are refused.
+//  before it.  Schedules of more than kNoAllocMaxLevels (direction, level) pairs are refused: as many as the counters
+//  of the dataflow form held; nothing is held per level now, but what the call refuses stays as it is.
 // =============================================================================================
 namespace lb {
 namespace {
