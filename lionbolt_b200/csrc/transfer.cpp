@@ -6,10 +6,11 @@
 // pinned buffer while the other one is on the bus, so the bus carries the device's own type and nothing is
 // allocated per call.  An operator application on a 132 MB angular vector took 82 ms with pageable copies.
 // Transfers up to 4 MB use a pair of 95 KB buffers that come with the handle; larger ones a pair of 512 KB that is allocated
-// when first needed, and one of 4 MB once the handle has moved 512 MB through it.  Pinning costs 0.5 ms per MB, paid by the
+// when first needed, and one of 4 MB once the handle has moved 128 MB through it.  Pinning costs 0.5 ms per MB, paid by the
 // call that needs it, and so has to be small against that call: the first sweep of a handle on a vector of 31 MB (7.7 MB)
 // took 11.4 (3.9) ms with pageable copies, 23 (10) with a pair of 8 MB, 6.2 (3.1) with 1 MB and 3.4 (1.6) with 512 KB.
-// Later ones take 65.8 MB there and back in 7.0 ms with 512 KB and 5.2 with 4 MB, which is worth its 4.4 ms from then on.
+// Later ones take 65.8 MB there and back in 7.0 ms with 512 KB and 5.2 with 4 MB (24.6 MB of results in 1.94 and 1.6).  The 4.4 ms
+// that these cost come when the first 128 MB have saved as much against pageable copies (3.0 ms for the 24.6 MB).
 // All go with the handle.  Only chunks of 256 KB up use several threads: waking them costs a small one more than it
 // saves, and they are half the host's (at most 8), so that threads still spinning after a transfer leave the
 // caller its core.
@@ -25,7 +26,7 @@ namespace {
 
 constexpr size_t kPipeLarge = (size_t)1 << 19;    // bytes of a large buffer at first
 constexpr size_t kPipeMax = (size_t)4 << 20;      // and after kGrowAfter bytes
-constexpr size_t kGrowAfter = (size_t)1 << 29;
+constexpr size_t kGrowAfter = (size_t)1 << 27;
 constexpr size_t kLarge = (size_t)4 << 20;        // transfers above take the large buffers (and smaller ones once they exist)
 constexpr size_t kHoldMax = (size_t)256 << 20;     // bytes of a vector on its way that a handle keeps the place of
 constexpr size_t kThreaded = (size_t)1 << 18;     // bytes of a chunk from which several threads do the work

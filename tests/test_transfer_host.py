@@ -146,7 +146,7 @@ def test_a_first_large_transfer_pins_little(lib, handle):
 @pytest.mark.parametrize("refused", [False, True])
 def test_a_handle_that_moves_much_gets_larger_buffers(lib, handle, refused):
     before = lib.t_pinned()
-    src, dev = np.ones(64 * MB, np.uint8), np.zeros(64 * MB, np.uint8)
+    src, dev = np.ones(16 * MB, np.uint8), np.zeros(16 * MB, np.uint8)
     for k in range(9):
         if k == 8 and refused:
             lib.t_pin_limit(lib.t_pinned())
